@@ -243,6 +243,77 @@ def run(s):
     return {"y": y, "coords": level.coords, "src": level.src, "nbr": level.nb.nbr, "gray": level.nb.gray}
 
 
+# ------------------------------------------------------------------------------------------ the same in 64 bits
+def _map64(coords):
+    """int64 [n, 27]: row of each neighbour, -1 where there is none."""
+    key = lambda q: ((q[..., 0] * 4100 + q[..., 1] + 1) * 4100 + q[..., 2] + 1) * 4100 + q[..., 3] + 1
+    q = coords.long()
+    have, order = key(q).sort()
+    o = torch.tensor([-1, 0, 1], device=q.device)
+    taps = torch.cat([torch.zeros(27, 1, dtype=torch.int64, device=q.device), torch.cartesian_prod(o, o, o)], 1)
+    out = []
+    for part in q.split(1 << 20):
+        k = key(part[:, None] + taps[None])
+        at = torch.searchsorted(have, k).clamp(max=have.numel() - 1)
+        out.append(torch.where(have[at] == k, order[at], -1))
+    return torch.cat(out)
+
+
+def _conv64(x, w, b, nbr, rows=None, slot=None):
+    """Rows of the map (all, or the listed ones with the weight set of their slot) times x and w in 64 bits, the bias added."""
+    rows = torch.arange(nbr.shape[0], device=x.device) if rows is None else rows
+    co = w.shape[0] if slot is None else w.shape[0] // 8
+    y = torch.zeros((rows.numel(), co), dtype=torch.float64, device=x.device)
+    for s in range(1 if slot is None else 8):
+        mine = torch.arange(rows.numel(), device=x.device) if slot is None else (slot == s).nonzero()[:, 0]
+        ws = w[s * co:(s + 1) * co].double()
+        for at in mine.split(1 << 19):
+            part = torch.zeros((at.numel(), co), dtype=torch.float64, device=x.device)
+            for v in range(27):
+                r = nbr[rows[at], v]
+                have = (r >= 0).nonzero()[:, 0]
+                part[have] += x[r[have]].double() @ ws[:, v].T
+            y[at] = part if b is None else part + b[s * co:(s + 1) * co].double()
+    return y
+
+
+def _norm64(x, ln):
+    gamma, beta, eps = ln
+    y = torch.nn.functional.layer_norm(x, x.shape[-1:], eps=eps)
+    return y if gamma is None else y * gamma.double() + beta.double()
+
+
+def exact(case, seed):
+    kind, s = case["kind"], prepare(case, seed)
+    if kind == "maps":
+        return None
+    s = {k: v.cuda() if isinstance(v, torch.Tensor) else v for k, v in s.items()}
+    x, nbr, f = s["x"], _map64(s["coords"]), torch.nn.functional
+    if kind == "layers":
+        y = x
+        for w in s["ws"]:
+            y = _conv64(y, w, None, nbr)
+        return y
+    if kind == "up":
+        kept = (s["logits"] > 0).nonzero()
+        parent, slot = kept[:, 0], kept[:, 1]
+        coords = torch.cat([s["coords"][parent, :1], 2 * s["coords"][parent, 1:] + torch.stack([slot & 1, (slot >> 1) & 1, slot >> 2], 1)], 1)
+        h = f.silu(_norm64(x.double(), s["ln"]))
+        h = f.silu(_norm64(_conv64(h, s["w"], s["b"], nbr, parent, slot), (None, None, 1e-6)))
+        cs, co = case["ci"] // 8, case["co"]
+        skip = x.view(-1, 8, cs)[parent, slot].double().repeat_interleave(co // cs, 1)
+        return {"y": _conv64(h, s["w2"], s["b2"], _map64(coords)) + skip, "coords": None, "src": None, "nbr": None, "gray": None}
+    y = _conv64(x, s["w"], s["b"], nbr)
+    if kind == "step":
+        return {"y": y, "nbr": None, "gray": None}
+    if kind == "host":
+        return y
+    if kind == "resblock":
+        return _conv64(f.gelu(_norm64(y, s["ln"])), s["w2"], s["b2"], nbr) + x.double()
+    y = f.silu(_norm64(y, s["ln"]) @ s["w_in"].double().T + s["b_in"].double())
+    return y @ s["w_out"].double().T + s["b_out"].double() + x.double()
+
+
 # ------------------------------------------------------------------------------------------ cost and precision
 MAP_ROW = 27 * 4 + 4          # bytes of a row of the neighbour map and its mask
 
