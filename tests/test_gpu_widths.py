@@ -1,0 +1,73 @@
+"""Channel widths and row counts at which the conv kernels change form: rows that end in a half chunk of 32 channels, and accumulator
+widths that are no power of two.
+
+Bounds.  Inputs are rounded to the storage type, the oracle sums in fp32 (tap by tap, channel by channel).  A result of K = 27 Ci
+products with |y| about 1 carries at most half a rounding step of the storage type from its own rounding and as much from
+the oracle's, plus K * 2^-24 * sum|x w| from either order of summation (fp32 legs: that alone)."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from trellis2_cuda_b200 import scenes
+
+pytestmark = pytest.mark.gpu
+TD = {"f32": torch.float32, "f16": torch.float16, "bf16": torch.bfloat16}
+STEP = {"f16": 2.0 ** -10, "bf16": 2.0 ** -7, "f32": 2.0 ** -23}
+
+
+@pytest.fixture(scope="module")
+def sp():
+    import trellis2_cuda_b200 as m
+    m.context()
+    return m
+
+
+def scene(n, Ci, Co, dt, seed=0, slots=1):
+    rng = np.random.default_rng([n, Ci, Co, seed])
+    res = max(4, int(round((n / 0.3) ** (1 / 3))))
+    cells = rng.choice(res ** 3, size=n, replace=False)
+    c = np.stack([np.zeros_like(cells), cells // (res * res), cells // res % res, cells % res], 1).astype(np.int32)
+    x = oracle.round_to(rng.standard_normal((n, Ci), dtype=np.float32), dt)
+    w = oracle.round_to(scenes.kaiming_uniform_weight(slots * Co, Ci, seed), dt)
+    b = oracle.round_to(0.1 * rng.standard_normal(slots * Co).astype(np.float32), dt)
+    return c, x, w, b
+
+
+def check(y, want, Ci, dt, what, steps=1.0, bias=None):
+    """`bias` [columns]: the sum was rounded once before the bias went in, at a size of up to |want| + |bias|."""
+    got, want = y.float().cpu().numpy().astype(np.float64), np.asarray(want, np.float64)
+    most = np.maximum(np.abs(want), np.abs(got)) + (0 if bias is None else np.abs(bias))
+    size = 2.0 ** np.floor(np.log2(np.maximum(most, 2.0 ** -6)))
+    order = 27 * Ci * 2.0 ** -24 * 8.0                 # sum |x w| stays below 8 for Kaiming weights and unit features
+    allow = order + (0 if dt == "f32" else steps * STEP[dt] * size)
+    bad = np.abs(got - want) > allow
+    assert np.isfinite(got).all() and not bad.any(), f"{what}: {bad.sum()} of {bad.size}, worst {np.abs(got - want).max():.3e}"
+
+
+@pytest.mark.parametrize("dt,n,Ci,Co", [("bf16", 700, 32, 32), ("f16", 129, 96, 160), ("bf16", 1000, 160, 96), ("f16", 385, 224, 224), ("bf16", 640, 32, 256),
+                                        ("bf16", 300, 64, 192), ("f16", 257, 288, 320)])
+def test_half_chunks_and_accumulator_widths(sp, dt, n, Ci, Co):
+    c, x, w, b = scene(n, Ci, Co, dt)
+    nbr, _, _, _ = oracle.build_neighbors(c)
+    want = oracle.conv_block(x, w, b, nbr, dt)
+    xd, wd, bd = (torch.from_numpy(t).cuda().to(TD[dt]) for t in (x, w, b))
+    for tile_rows in (128, 256):
+        cache = sp.build_neighbors(torch.from_numpy(c).cuda(), tile_rows=tile_rows)
+        y = sp.subm_conv(xd, wd, bd, cache)
+        sp.context().device_status()
+        check(y, want, Ci, dt, f"{dt} {n} {Ci}->{Co} tile {tile_rows}", steps=2.0, bias=b)     # conv and bias are rounded one after the other
+
+
+def test_subdivision_conv_with_half_chunks(sp):
+    """8 weight sets, rows of 96 channels."""
+    Ci, Cc, dt = 96, 96, "bf16"
+    c, x, w, b = scene(400, Ci, Cc, dt, slots=8)
+    sub = np.random.default_rng(3).standard_normal((400, 8)).astype(np.float16)
+    parent = sp.build_neighbors(torch.from_numpy(c).cuda())
+    level = sp.subdivide(parent, torch.from_numpy(sub).cuda())
+    y = sp.subdiv_conv(*(torch.from_numpy(t).cuda().to(TD[dt]) for t in (x, w, b)), level)
+    nbr, _, _, _ = oracle.build_neighbors(c)
+    full = oracle.conv_block(x, w, b, nbr, dt).reshape(400 * 8, Cc)
+    src = level.src.cpu().numpy()
+    check(y, full[src], Ci, dt, "subdivision", steps=2.0, bias=b.reshape(8, Cc)[src % 8])

@@ -53,15 +53,16 @@ using namespace umma;
 // Only the peer-memory form, whose map arrives with the call, still has two index warps that build the table from map
 // rows (4-byte cp.async, one 108-byte row per warp instruction), mark absent / out-of-range entries and flag the taps
 // that read a peer.
-template <int BN, int MH, int G, int U, bool PEERS, class T>
+template <int BN, int MH, int G, int U, bool PEERS, bool TAIL, class T>
 __global__ void __launch_bounds__(num_threads(MH, G), 1) k_conv_umma(const __grid_constant__ CUtensorMap tmw, const ConvArgs a) {
+  static_assert(!TAIL || (MH == 1 && !PEERS), "half chunks run on 128-row tiles of local rows");
   static_assert(G == 1 || (G == 2 && MH == 1), "a second gather group only fits beside 128-row tiles");
   constexpr int UNIT = stage_bytes(BN, MH);          // MH gathered A halves + one weight slab
   constexpr int STAGE = U * UNIT;
   constexpr int S = num_stages(BN, MH, U);
   constexpr int B_BYTES = BN * 128;
   constexpr int NB = num_acc_bufs(BN, MH);            // accumulator buffers, each MH halves of BN columns
-  constexpr int TMEM_COLS = NB * MH * BN < 32 ? 32 : NB * MH * BN;
+  constexpr int TMEM_COLS = tmem_cols(NB * MH * BN);
   constexpr int ROWS = MH * TILE_M;
   constexpr int PITCH = PEERS ? tab_pitch(MH) : ROWS;  // the index warps write a map row per instruction: an odd pitch keeps that conflict-free
   constexpr int TABW = 27 * PITCH;
@@ -85,7 +86,10 @@ __global__ void __launch_bounds__(num_threads(MH, G), 1) k_conv_umma(const __gri
   const uint32_t bar_full = smem_u32(bars), bar_empty = bar_full + 8 * S, bar_accf = bar_empty + 8 * S, bar_acce = bar_accf + 16,
                  bar_tready = bar_acce + 16, bar_tfree = bar_tready + 8 * NTAB;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nchunk = a.Ci / KCH;
+  // TAIL: rows of an odd multiple of 32 channels end in a chunk of 32: half of the gather threads copy nothing for it, the
+  // weight box reads zeros past the row's end and the chunk takes two MMAs instead of four.  A form of its own, because
+  // asking at run time in these role loops cost every other width 6 to 12 % (217,821 x 256: conv 380 -> 426 us).
+  const int nchunk = TAIL ? (a.Ci + KCH - 1) / KCH : a.Ci / KCH;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; s++) { mbar_init(bar_full + 8 * s, NUM_PROD_THREADS + 1); mbar_init(bar_empty + 8 * s, 1); }
@@ -206,7 +210,7 @@ __global__ void __launch_bounds__(num_threads(MH, G), 1) k_conv_umma(const __gri
           }
           // After a wait was given up this thread loads and signals nothing more: the table may hold anything, and an
           // arrival on a barrier whose phase is still waiting for bytes in flight would overrun its count.
-          if (alive && !diag(a, 1)) {
+          if (alive && !diag(a, 1) && (!TAIL || c16 < 4 || c + 1 < nchunk)) {
             const uint32_t dst = smem_base + st * STAGE + k * UNIT + dst_thread;
             const T* xs = x + c * KCH + c16 * 8;
             if (PEERS && __builtin_expect(remote, 0)) {          // one branch per unit, not per copy: a P2P load when the owner is a peer
@@ -391,6 +395,7 @@ __global__ void __launch_bounds__(num_threads(MH, G), 1) k_conv_umma(const __gri
         const uint32_t d_tmem = tmem_base + buf * (MH * BN);
         const int halves = tile.rows > TILE_M ? MH : 1;
         const int nunits = __popc(tile.mask) * nchunk;
+        [[maybe_unused]] int c = 0;
         for (int u0 = 0; u0 < nunits; u0 += U, it++) {
           const int nu = nunits - u0 < U ? nunits - u0 : U;
           const uint32_t s = it % S, ph = (it / S) & 1;
@@ -407,6 +412,13 @@ __global__ void __launch_bounds__(num_threads(MH, G), 1) k_conv_umma(const __gri
 #pragma unroll
             for (int k = 0; k < U; k++) {
               if (k >= nu) break;
+              if constexpr (TAIL) {
+                if (++c == nchunk) {
+                  c = 0;
+                  tc_mma_k32(d_tmem, ds + ((k * UNIT) >> 4), ds + ((k * UNIT + MH * A_BYTES) >> 4), idesc, u0 + k > 0 ? 1u : 0u);
+                  continue;
+                }
+              }
 #pragma unroll
               for (int h = 0; h < MH; h++) {
                 if (h < halves)
@@ -493,29 +505,37 @@ static EncodeTiledFn encode_fn() {
   return fn;
 }
 
-template <int BN, int MH, int G, int U, bool PEERS, class T>
+template <int BN, int MH, int G, int U, bool PEERS, class T, bool TAIL = false>
 int launch_p(t2sc_ctx* ctx, const CUtensorMap& tm, const ConvArgs& args, i64 max_items) {
   constexpr int smem = num_stages(BN, MH, U) * U * stage_bytes(BN, MH) + aux_bytes(MH) + 1024;
   static_assert(smem <= SMEM_BUDGET && num_stages(BN, MH, U) >= 2, "shared memory budget");
   static bool attr_set[16] = {};
   if (!attr_set[ctx->device & 15]) {
-    T2_CUDA(ctx, cudaFuncSetAttribute(k_conv_umma<BN, MH, G, U, PEERS, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    T2_CUDA(ctx, cudaFuncSetAttribute(k_conv_umma<BN, MH, G, U, PEERS, TAIL, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     attr_set[ctx->device & 15] = true;
   }
   int grid = (int)(max_items < ctx->num_sms ? max_items : ctx->num_sms);
-  k_conv_umma<BN, MH, G, U, PEERS, T><<<grid, num_threads(MH, G), smem, ctx->stream>>>(tm, args);
+  k_conv_umma<BN, MH, G, U, PEERS, TAIL, T><<<grid, num_threads(MH, G), smem, ctx->stream>>>(tm, args);
   T2_LAUNCHED(ctx);
   return T2SC_OK;
 }
 
 // Which form runs.  128-row tiles with Co <= 128 (accumulator tiles of 32..128 columns): two gather groups and two units
 // per stage (measured 5-12 % faster than one unit per stage at 64 and 128 channels; four units per stage are no better
-// than two).  Co % 256 == 0: one unit per stage (a stage is 48 KB there), the second gather group only for Ci = 64.
+// than two).  Wider tiles: one unit per stage (a stage is 36 to 48 KB there), the second gather group only for Ci = 64.
 // 256-row tiles and the peer-memory form: one group, one unit per stage.  The diagnostic build can force one unit per
 // stage (T2SC_UNITS=1) to compare the forms.
 template <int BN, int MH, class T>
 int launch_bn(t2sc_ctx* ctx, const CUtensorMap& tm, const ConvArgs& args, i64 max_items) {
-  if (args.npeers > 0) return launch_p<BN, MH, 1, 1, true, T>(ctx, tm, args, max_items);
+  if constexpr ((BN & (BN - 1)) == 0) {
+    if (args.npeers > 0) return launch_p<BN, MH, 1, 1, true, T>(ctx, tm, args, max_items);
+  }
+  if constexpr (MH == 1) {
+    if (args.Ci % KCH != 0) {
+      if constexpr (BN <= 128) return launch_p<BN, MH, 2, 2, false, T, true>(ctx, tm, args, max_items);
+      else return launch_p<BN, MH, 1, 1, false, T, true>(ctx, tm, args, max_items);
+    }
+  }
   if constexpr (MH == 1 && BN <= 128) {
 #ifdef T2SC_DIAG
     static const int force_u = [] { const char* e = getenv("T2SC_UNITS"); return e ? atoi(e) : 0; }();
@@ -532,6 +552,15 @@ int launch_bn(t2sc_ctx* ctx, const CUtensorMap& tm, const ConvArgs& args, i64 ma
 
 template <int MH, class T>
 int launch_t(t2sc_ctx* ctx, int BN, const CUtensorMap& tm, const ConvArgs& args, i64 max_items) {
+  if constexpr (MH == 1) {
+    switch (BN) {
+      case 224: return launch_bn<224, MH, T>(ctx, tm, args, max_items);
+      case 192: return launch_bn<192, MH, T>(ctx, tm, args, max_items);
+      case 160: return launch_bn<160, MH, T>(ctx, tm, args, max_items);
+      case 96: return launch_bn<96, MH, T>(ctx, tm, args, max_items);
+      default: break;
+    }
+  }
   switch (BN) {
     case 256: return launch_bn<256, MH, T>(ctx, tm, args, max_items);
     case 128: return launch_bn<128, MH, T>(ctx, tm, args, max_items);
@@ -540,25 +569,27 @@ int launch_t(t2sc_ctx* ctx, int BN, const CUtensorMap& tm, const ConvArgs& args,
   }
 }
 
-int pick_bn(int Co) {
-  for (int bn : {256, 128, 64, 32}) if (Co % bn == 0) return bn;
+// Columns of an accumulator: the widest multiple of 32 up to 256 that divides Co, because every column slab gathers the
+// tile's rows again.  The peer-memory form and 256-row tiles are built for the powers of two only (`pow2`).
+int pick_bn(int Co, bool pow2 = false) {
+  for (int bn : {256, 224, 192, 160, 128, 96, 64, 32})
+    if (Co % bn == 0 && (!pow2 || (bn & (bn - 1)) == 0)) return bn;
   return 0;
 }
 
 }  // namespace
 
-bool conv_umma_supported(int dtype, int Ci, int Co, const EpiDev& ep) {
-  (void)ep;
-  return (dtype == T2SC_F16 || dtype == T2SC_BF16) && Ci % KCH == 0 && Co % 32 == 0;
+bool conv_umma_supported(int dtype, int Ci, int Co, int tile_rows) {
+  return (dtype == T2SC_F16 || dtype == T2SC_BF16) && Ci % (tile_rows == TILE_M ? KCH / 2 : KCH) == 0 && Co % 32 == 0;
 }
 
-bool conv_umma_fuses_ln(int Co) { return pick_bn(Co) == Co; }
+bool conv_umma_fuses_ln(int Co, bool pow2) { return pick_bn(Co, pow2) == Co; }
 
 int conv_umma_launch(t2sc_ctx* ctx, const t2sc_plan* plan, const void* x, const void* w, i64 w_rows, const EpiDev& ep, void* y,
                      int dtype, i64 n_in, int Ci, int Co, int part, const void* const* x_peers, const int64_t* rows_peers, int n_peers,
                      int self_rank, const uint32_t* peer_nbr) {
   T2_CUDA(ctx, cudaSetDevice(ctx->device));
-  const int BN = pick_bn(Co);
+  const int BN = pick_bn(Co, n_peers > 0 || plan->tile_rows != TILE_M);
   T2_REQ(ctx, BN > 0, "Co=%d", Co);
   T2_REQ(ctx, !ep.ln || Co == BN, "fused LayerNorm needs the whole row in one tile (Co=%d)", Co);
   EncodeTiledFn enc = encode_fn();

@@ -53,6 +53,8 @@ __host__ __device__ constexpr int num_stages(int BN, int MH, int U = 1) {
   return s > 8 ? 8 : s;
 }
 __host__ __device__ constexpr int num_acc_bufs(int BN, int MH) { return 2 * MH * BN <= 512 ? 2 : 1; }
+// TMEM is allocated in powers of two from 32 columns up
+__host__ __device__ constexpr int tmem_cols(int used) { int c = 32; while (c < used) c *= 2; return c; }
 
 struct ConvArgs {
   const void* x; void* y; const uint32_t* nbr; const int* order; const int* src;
@@ -197,6 +199,11 @@ __device__ __forceinline__ void tc_mma_k64(uint32_t d_tmem, uint64_t adesc, uint
                "add.u32 x, al, 6;\n\tmov.b64 a, {x, ah};\n\tadd.u32 x, bl, 6;\n\tmov.b64 b, {x, bh};\n\t"
                "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, t;\n\t}"
                ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+// The same for a unit of 32 channels (the last chunk of a row whose length is an odd multiple of 32): two MMAs.
+__device__ __forceinline__ void tc_mma_k32(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  tc_mma(d_tmem, adesc, bdesc, idesc, accumulate);
+  tc_mma(d_tmem, adesc + 2, bdesc + 2, idesc, 1u);
 }
 __device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t* r) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"

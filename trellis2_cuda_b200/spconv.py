@@ -371,11 +371,12 @@ class Level:
     parent: Optional[SpConvCache] = None
     _up_plans: Optional[dict] = None
 
-    def up_plan_for(self, Cc: int) -> _Plan:
+    def up_plan_for(self, Cc: int, Ci: int = 64) -> _Plan:
         """Schedule of the subdivision conv into Cc child channels: 256-row tiles, two 128-row accumulators per weight slab
         (the 8 child slots have 8 weight sets, so a slab is reused by fewer rows than in a submanifold conv; measured on
-        886,752 parents -> 3,288,465 children, 128 -> 64: 2.35 ms against 2.80 ms with 128-row tiles)."""
-        tr = 256
+        886,752 parents -> 3,288,465 children, 128 -> 64: 2.35 ms against 2.80 ms with 128-row tiles).  128-row tiles for input
+        rows that end in half a chunk, which have that form only."""
+        tr = 256 if Ci % 64 == 0 else 128
         if self._up_plans is None:
             self._up_plans = {}
         if tr not in self._up_plans:
@@ -416,7 +417,7 @@ def subdiv_conv(x: torch.Tensor, w: torch.Tensor, b: Optional[torch.Tensor], lev
         raise T2scError(-1, "subdivision conv needs 8*Cc weight rows")
     if x.shape[0] != level.parent.N:
         raise T2scError(-1, f"spconv shapes: x has {x.shape[0]} rows, parent cache has {level.parent.N}")
-    return _conv(level.parent.ctx, level.up_plan_for(w.shape[0] // 8), x, w, b, w.shape[0] // 8, ln, act, None, None, variant, out)
+    return _conv(level.parent.ctx, level.up_plan_for(w.shape[0] // 8, w.shape[-1]), x, w, b, w.shape[0] // 8, ln, act, None, None, variant, out)
 
 
 def gather_rows(x: torch.Tensor, src: torch.Tensor, C: int, out: Optional[torch.Tensor] = None) -> torch.Tensor:
