@@ -71,3 +71,19 @@ def test_subdivision_conv_with_half_chunks(sp):
     full = oracle.conv_block(x, w, b, nbr, dt).reshape(400 * 8, Cc)
     src = level.src.cpu().numpy()
     check(y, full[src], Ci, dt, "subdivision", steps=2.0, bias=b.reshape(8, Cc)[src % 8])
+
+
+@pytest.mark.parametrize("n,Ci,Co", [(1, 32, 64), (63, 32, 64), (64, 64, 10), (65, 64, 64), (300, 32, 130), (2500, 64, 64), (9000, 32, 64), (29000, 32, 32)])
+def test_fp32_splits(sp, n, Ci, Co):
+    """The fp32 kernel splits a tile's taps over clusters of 1, 2, 4 and 8 CTAs by the number of tiles."""
+    c, x, w, b = scene(n, Ci, Co, "f32")
+    nbr, _, _, _ = oracle.build_neighbors(c)
+    res = np.random.default_rng(1).standard_normal((n, Co), dtype=np.float32)
+    want = oracle.conv_block(x, w, b, nbr, "f32", act_kind="silu", residual=res)
+    for tile_rows in (128, 256):
+        cache = sp.build_neighbors(torch.from_numpy(c).cuda(), tile_rows=tile_rows)
+        args = [torch.from_numpy(t).cuda() for t in (x, w, b)]
+        y = sp.subm_conv(*args, cache, act="silu", residual=torch.from_numpy(res).cuda())
+        sp.context().device_status()
+        check(y, want, Ci, "f32", f"f32 {n} {Ci}->{Co} tile {tile_rows}")
+        assert torch.equal(y, sp.subm_conv(*args, cache, act="silu", residual=torch.from_numpy(res).cuda()))     # ranks add in a fixed order

@@ -155,6 +155,8 @@ static inline TilePart tile_part(const t2sc_plan* p, int part) {
 }
 int conv_simt_launch(t2sc_ctx* ctx, const t2sc_plan* plan, const void* x, const void* w, const EpiDev& ep, void* y,
                      int dtype, i64 n_in, int Ci, int Co, int part = T2SC_PART_ALL);
+int conv_f32_launch(t2sc_ctx* ctx, const t2sc_plan* plan, const float* x, const float* w, const EpiDev& ep, float* y, i64 n_in, int Ci, int Co,
+                    int part);
 bool conv_umma_supported(int dtype, int Ci, int Co, int tile_rows);
 // can the tcgen05 path hold a whole output row in one accumulator (fused LayerNorm)?  pow2: its forms of 32, 64, 128 and 256 columns alone
 bool conv_umma_fuses_ln(int Co, bool pow2 = false);

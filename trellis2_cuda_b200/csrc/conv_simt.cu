@@ -1,7 +1,7 @@
-// CUDA-core variant of the masked implicit-GEMM sparse conv: fp32 math on fp32 / fp16 / bf16 storage.
+// CUDA-core variant of the masked implicit-GEMM sparse conv for fp16 / bf16 storage (fp32 math), and the row pass.
 //
-// This is the path for fp32 features (the tensor cores would drop them to tf32) and for shapes the
-// tcgen05 kernel does not take (Ci not a multiple of 64, Co not a multiple of 32).  It computes the
+// This is the path for output widths the tcgen05 kernel does not take (Co not a multiple of 32); fp32 features
+// have a kernel of their own (conv_f32.cu).  It computes the
 // operator of src/spconv.cu:91-150 (trellis2-cuda): y[i,co] = sum over the tile's taps, ascending, of
 // x[nbr[i,v],:] . w[co,v,:], fp32 accumulation, absent neighbours contributing zeros.
 // One CTA = 128 rows of a plan tile x 64 output channels; 256 threads, 8x4 outputs each; K in chunks of 16.
@@ -281,14 +281,13 @@ void row_epilogue_pick(cudaStream_t st, const void* x, const EpiDev& ep, void* y
 
 int conv_simt_launch(t2sc_ctx* ctx, const t2sc_plan* plan, const void* x, const void* w, const EpiDev& ep, void* y,
                      int dtype, i64 n_in, int Ci, int Co, int part) {
+  if (dtype == T2SC_F32) return conv_f32_launch(ctx, plan, (const float*)x, (const float*)w, ep, (float*)y, n_in, Ci, Co, part);
   T2_REQ(ctx, Ci % BK == 0, "Ci=%d", Ci);
   const TilePart tp = tile_part(plan, part);
   T2_CUDA(ctx, cudaSetDevice(ctx->device));
   const int subs = plan->tile_rows / BM;
   dim3 grid((unsigned)(plan->max_tiles * subs), (unsigned)cdiv_i(Co, BN));
-  if (dtype == T2SC_F32)
-    k_conv_simt<float><<<grid, 256, 0, ctx->stream>>>((const float*)x, (const float*)w, plan->nbr, plan->order, plan->src, plan->tiles, tp.lo, tp.hi, ep, (float*)y, Ci, Co, subs, (uint32_t)n_in, ctx->status);
-  else if (dtype == T2SC_F16)
+  if (dtype == T2SC_F16)
     k_conv_simt<__half><<<grid, 256, 0, ctx->stream>>>((const __half*)x, (const __half*)w, plan->nbr, plan->order, plan->src, plan->tiles, tp.lo, tp.hi, ep, (__half*)y, Ci, Co, subs, (uint32_t)n_in, ctx->status);
   else
     k_conv_simt<__nv_bfloat16><<<grid, 256, 0, ctx->stream>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)w, plan->nbr, plan->order, plan->src, plan->tiles, tp.lo, tp.hi, ep, (__nv_bfloat16*)y, Ci, Co, subs, (uint32_t)n_in, ctx->status);
