@@ -87,3 +87,21 @@ def test_fp32_splits(sp, n, Ci, Co):
         sp.context().device_status()
         check(y, want, Ci, "f32", f"f32 {n} {Ci}->{Co} tile {tile_rows}")
         assert torch.equal(y, sp.subm_conv(*args, cache, act="silu", residual=torch.from_numpy(res).cuda()))     # ranks add in a fixed order
+
+
+@pytest.mark.parametrize("dt", ["f16", "bf16", "f32"])
+@pytest.mark.parametrize("n,C", [(1, 8), (10007, 32), (19001, 40), (10007, 64), (33, 72), (10007, 128), (777, 136), (5003, 256), (1000, 264), (601, 1024), (301, 1032)])
+def test_row_pass_over_its_lane_groups(sp, dt, n, C):
+    """Rows of 4, 8, 16 and 32 lanes, partly filled ones, and more rows than one sweep of the grid.  Against 64 bits with the pass's
+    rounding points: LayerNorm, activation and residual each round once, a flipped rounding of one moves the next by as
+    much again; fp32 adds the sums over C."""
+    g = torch.Generator(device="cuda").manual_seed(n + C)
+    x, r = (torch.randn((n, C), generator=g, device="cuda").to(TD[dt]) for _ in range(2))
+    gamma, beta = torch.rand(C, generator=g, device="cuda") + 0.5, torch.randn(C, generator=g, device="cuda")
+    y = sp.row_epilogue(x, ln=(gamma, beta, 1e-6), act="silu", residual=r)
+    v = torch.nn.functional.layer_norm(x.double(), (C,), eps=1e-6) * gamma.double()
+    h = torch.nn.functional.silu((v + beta.double()).to(TD[dt]).double()).to(TD[dt]).double()
+    want = h + r.double()
+    size = v.abs() + beta.double().abs() + want.abs() + r.double().abs()        # the terms of every sum along the way
+    assert ((y.double() - want).abs() <= (4 if dt != "f32" else 16) * STEP[dt] * (size + 2.0 ** -6)).all()
+    assert torch.equal(sp.row_epilogue(x, ln=(gamma, beta, 1e-6), act="silu", residual=r, out=x), y)        # in place

@@ -159,6 +159,21 @@ __global__ void __launch_bounds__(256) k_row_epilogue(const T* x, EpiDev ep, T* 
   }
 }
 
+// 8 values as they lie in memory, so that a load can be in flight while nothing waits for its conversion
+template <class T> struct Raw8 {
+  uint4 r;
+  __device__ __forceinline__ void load(const T* p) { r = *(const uint4*)p; }
+  __device__ __forceinline__ void unpack(float* o) const {
+    const T* h = (const T*)&r;
+#pragma unroll
+    for (int i = 0; i < 8; i++) o[i] = to_f<T>(h[i]);
+  }
+};
+template <> struct Raw8<float> {
+  float4 a, b;
+  __device__ __forceinline__ void load(const float* p) { a = *(const float4*)p; b = *((const float4*)p + 1); }
+  __device__ __forceinline__ void unpack(float* o) const { o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w; o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w; }
+};
 template <class T> __device__ __forceinline__ void store8(T* p, const float* v);
 template <> __device__ __forceinline__ void store8<float>(float* p, const float* v) {
   *(float4*)p = make_float4(v[0], v[1], v[2], v[3]); *((float4*)p + 1) = make_float4(v[4], v[5], v[6], v[7]);
@@ -176,104 +191,149 @@ template <> __device__ __forceinline__ void store8<__nv_bfloat16>(__nv_bfloat16*
   *(uint4*)p = o;
 }
 
-// The same pass for rows of up to NV * 256 channels, C % 8 == 0: one warp per row, the row read ONCE in pieces of 8
-// channels (16-byte loads for the 16-bit types) and held in registers through the statistics and the transform.
-template <class T, int NV>
-__global__ void __launch_bounds__(256) k_row_epilogue_vec(const T* x, EpiDev ep, T* y, i64 n, int C) {   // y may alias x
-  const i64 row = (blockIdx.x * (i64)blockDim.x + threadIdx.x) >> 5; const int lane = threadIdx.x & 31;
-  if (row >= n) return;
-  const T* xr = x + row * C; T* yr = y + row * C;
+// SiLU of the 16-bit storage types: ex2.approx and rcp.approx, as the tcgen05 kernel's epilogue takes it (about 2^-21 relative,
+// against 2^-11 of the rounding that follows)
+template <class T> __device__ __forceinline__ float act_row(float v, int act) {
+  if constexpr (sizeof(T) == 2) { if (act == T2SC_ACT_SILU) return __fdividef(v, 1.f + __expf(-v)); }
+  return act_apply(v, act);
+}
+
+// The same pass for rows of up to NV * 256 channels, C % 8 == 0: LPR lanes per row (32, or 16 / 8 / 4 for rows of at most 128 /
+// 64 / 32 channels), the row read ONCE in pieces of 8 channels (16-byte loads for the 16-bit types) and held in registers
+// through the statistics and the transform.  Bound by HBM when the instructions allow it: 886,752 x 128 fp16 with LayerNorm
+// and SiLU move 454 MB (69 us at 6.55 TB/s).  With a whole warp per row, half of its lanes idle, gamma and beta fetched again
+// for every row (64 bytes for 16 of x) and IEEE divisions that pass took 387 us; so the lanes fit the row, a thread keeps its
+// piece of gamma and beta over the rows of a grid-stride loop (NV <= 2; wider rows read them from the L1), and the next row
+// is in flight while one is worked on.
+template <class T, int NV, int LPR>
+__global__ void __launch_bounds__(256, NV == 1 ? 4 : NV <= 4 ? 2 : 1) k_row_epilogue_vec(const T* x, EpiDev ep, T* y, i64 n, int C) {   // y may alias x
+  static_assert(NV == 1 || LPR == 32, "several pieces per lane only for whole warps");
+  constexpr int RPB = 256 / LPR;
+  constexpr bool KEEP = NV <= 2;          // gamma and beta in registers
+  const int lane = threadIdx.x % LPR;
+  const unsigned group = LPR == 32 ? 0xffffffffu : ((1u << (LPR & 31)) - 1) << ((threadIdx.x & 31) / LPR * LPR);
   const T* bias = (const T*)ep.bias; const T* res = (const T*)ep.residual; const T* skx = (const T*)ep.skip_x;
   const int nvec = C >> 3;
-  float h[NV][8];
+  auto sum = [&](float v) {
 #pragma unroll
-  for (int k = 0; k < NV; k++) {
-    const int vi = lane + 32 * k;
-    if (vi < nvec) {
-      load8<T>(xr + vi * 8, h[k]);
-      if (bias) {
-        float b[8]; load8<T>(bias + vi * 8, b);
+    for (int o = LPR / 2; o; o >>= 1) v += __shfl_xor_sync(group, v, o);
+    return v;
+  };
+  auto affine = [&](int vi, float* g, float* be) {
 #pragma unroll
-        for (int i = 0; i < 8; i++) h[k][i] = rnd<T>(h[k][i] + b[i]);
-      }
+    for (int i = 0; i < 8; i++) { g[i] = 1.f; be[i] = 0.f; }
+    if (ep.gamma) load8<float>(ep.gamma + vi * 8, g);
+    if (ep.beta) load8<float>(ep.beta + vi * 8, be);
+  };
+  float kg[KEEP ? NV : 1][8], kb[KEEP ? NV : 1][8];
+  if constexpr (KEEP) {
+    if (ep.ln) {
+#pragma unroll
+      for (int k = 0; k < NV; k++) if (lane + LPR * k < nvec) affine(lane + LPR * k, kg[k], kb[k]);
     }
   }
-  if (ep.ln) {
-    float s = 0.f;
+  i64 row = blockIdx.x * (i64)RPB + threadIdx.x / LPR;
+  const i64 step = gridDim.x * (i64)RPB;
+  Raw8<T> next[NV];
+  auto fetch = [&](i64 r) {
 #pragma unroll
-    for (int k = 0; k < NV; k++)
-      if (lane + 32 * k < nvec) {
+    for (int k = 0; k < NV; k++) if (lane + LPR * k < nvec) next[k].load(x + r * C + (lane + LPR * k) * 8);
+  };
+  if (row < n) fetch(row);
+  for (; row < n; row += step) {
+    float h[NV][8];
 #pragma unroll
-        for (int i = 0; i < 8; i++) s += h[k][i];
-      }
+    for (int k = 0; k < NV; k++) if (lane + LPR * k < nvec) next[k].unpack(h[k]);
+    if (row + step < n) fetch(row + step);
+    if (bias) {
 #pragma unroll
-    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    const float mean = s / (float)C;
-    float q = 0.f;
+      for (int k = 0; k < NV; k++) {
+        const int vi = lane + LPR * k;
+        if (vi < nvec) {
+          float b[8]; load8<T>(bias + vi * 8, b);
 #pragma unroll
-    for (int k = 0; k < NV; k++)
-      if (lane + 32 * k < nvec) {
-#pragma unroll
-        for (int i = 0; i < 8; i++) { const float d = h[k][i] - mean; q += d * d; }
-      }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
-    const float rstd = rsqrtf(q / (float)C + ep.eps);
-#pragma unroll
-    for (int k = 0; k < NV; k++) {
-      const int vi = lane + 32 * k;
-      if (vi < nvec) {
-        float g[8], be[8];
-        if (ep.gamma) { const float4 a = __ldg((const float4*)(ep.gamma + vi * 8)), b = __ldg((const float4*)(ep.gamma + vi * 8) + 1);
-                        g[0] = a.x; g[1] = a.y; g[2] = a.z; g[3] = a.w; g[4] = b.x; g[5] = b.y; g[6] = b.z; g[7] = b.w; }
-        if (ep.beta) { const float4 a = __ldg((const float4*)(ep.beta + vi * 8)), b = __ldg((const float4*)(ep.beta + vi * 8) + 1);
-                       be[0] = a.x; be[1] = a.y; be[2] = a.z; be[3] = a.w; be[4] = b.x; be[5] = b.y; be[6] = b.z; be[7] = b.w; }
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-          float v = rstd * (h[k][i] - mean);
-          if (ep.gamma) v = g[i] * v;
-          if (ep.beta) v = v + be[i];
-          h[k][i] = rnd<T>(v);
+          for (int i = 0; i < 8; i++) h[k][i] = rnd<T>(h[k][i] + b[i]);
         }
       }
     }
-  }
-  int sp = 0, ss = 0;
-  if (skx) { const int sv = ep.skip_src[row]; sp = sv >> 3; ss = sv & 7; }
+    if (ep.ln) {
+      float s = 0.f;
 #pragma unroll
-  for (int k = 0; k < NV; k++) {
-    const int vi = lane + 32 * k;
-    if (vi >= nvec) continue;
-    if (ep.act) {
+      for (int k = 0; k < NV; k++)
+        if (lane + LPR * k < nvec) {
 #pragma unroll
-      for (int i = 0; i < 8; i++) h[k][i] = rnd<T>(act_apply(h[k][i], ep.act));
+          for (int i = 0; i < 8; i++) s += h[k][i];
+        }
+      const float mean = sum(s) / (float)C;
+      float q = 0.f;
+#pragma unroll
+      for (int k = 0; k < NV; k++)
+        if (lane + LPR * k < nvec) {
+#pragma unroll
+          for (int i = 0; i < 8; i++) { const float d = h[k][i] - mean; q += d * d; }
+        }
+      const float rstd = rsqrtf(sum(q) / (float)C + ep.eps);
+#pragma unroll
+      for (int k = 0; k < NV; k++) {
+        const int vi = lane + LPR * k;
+        if (vi < nvec) {
+          float tg[8], tb[8];
+          if constexpr (!KEEP) affine(vi, tg, tb);
+          const float* g = KEEP ? kg[KEEP ? k : 0] : tg; const float* be = KEEP ? kb[KEEP ? k : 0] : tb;
+#pragma unroll
+          for (int i = 0; i < 8; i++) {
+            float v = rstd * (h[k][i] - mean);
+            if (ep.gamma) v = g[i] * v;
+            if (ep.beta) v = v + be[i];
+            h[k][i] = rnd<T>(v);
+          }
+        }
+      }
     }
-    if (res) {
-      float r[8]; load8<T>(res + row * C + vi * 8, r);
+    int sp = 0, ss = 0;
+    if (skx) { const int sv = ep.skip_src[row]; sp = sv >> 3; ss = sv & 7; }
 #pragma unroll
-      for (int i = 0; i < 8; i++) h[k][i] = rnd<T>(h[k][i] + r[i]);
-    }
-    if (skx) {
-      const T* sx = skx + (i64)sp * ep.skip_cin + ss * (ep.skip_cin / 8);
+    for (int k = 0; k < NV; k++) {
+      const int vi = lane + LPR * k;
+      if (vi >= nvec) continue;
+      if (ep.act) {
 #pragma unroll
-      for (int i = 0; i < 8; i++) h[k][i] = rnd<T>(h[k][i] + to_f<T>(sx[(vi * 8 + i) / ep.skip_rep]));
+        for (int i = 0; i < 8; i++) h[k][i] = rnd<T>(act_row<T>(h[k][i], ep.act));
+      }
+      if (res) {
+        float r[8]; load8<T>(res + row * C + vi * 8, r);
+#pragma unroll
+        for (int i = 0; i < 8; i++) h[k][i] = rnd<T>(h[k][i] + r[i]);
+      }
+      if (skx) {
+        const T* sx = skx + (i64)sp * ep.skip_cin + ss * (ep.skip_cin / 8);
+#pragma unroll
+        for (int i = 0; i < 8; i++) h[k][i] = rnd<T>(h[k][i] + to_f<T>(sx[(vi * 8 + i) / ep.skip_rep]));
+      }
+      store8<T>(y + row * C + vi * 8, h[k]);
     }
-    store8<T>(yr + vi * 8, h[k]);
   }
 }
 
 template <class T>
-void row_epilogue_pick(cudaStream_t st, const void* x, const EpiDev& ep, void* y, i64 n, int C) {
-  const int grid = cdiv_i(n * 32, 256);
+void row_epilogue_pick(t2sc_ctx* ctx, const void* x, const EpiDev& ep, void* y, i64 n, int C) {
   const bool aligned = (uintptr_t)x % 16 == 0 && (uintptr_t)y % 16 == 0 && (!ep.residual || (uintptr_t)ep.residual % 16 == 0) &&
                        (!ep.bias || (uintptr_t)ep.bias % 16 == 0) && (!ep.gamma || (uintptr_t)ep.gamma % 16 == 0) && (!ep.beta || (uintptr_t)ep.beta % 16 == 0);
   if (C % 8 == 0 && aligned && C <= 2048) {
-    if (C <= 256) k_row_epilogue_vec<T, 1><<<grid, 256, 0, st>>>((const T*)x, ep, (T*)y, n, C);
-    else if (C <= 512) k_row_epilogue_vec<T, 2><<<grid, 256, 0, st>>>((const T*)x, ep, (T*)y, n, C);
-    else if (C <= 1024) k_row_epilogue_vec<T, 4><<<grid, 256, 0, st>>>((const T*)x, ep, (T*)y, n, C);
-    else k_row_epilogue_vec<T, 8><<<grid, 256, 0, st>>>((const T*)x, ep, (T*)y, n, C);
+    const int lanes = C <= 32 ? 4 : C <= 64 ? 8 : C <= 128 ? 16 : 32;
+    const i64 blocks = (n * lanes + 255) / 256, most = (C <= 256 ? 4ll : C <= 1024 ? 2ll : 1ll) * ctx->num_sms;       // as many as are resident
+    const int grid = (int)(blocks < most ? blocks : most);
+#define T2_ROWS(NV, LPR) k_row_epilogue_vec<T, NV, LPR><<<grid, 256, 0, ctx->stream>>>((const T*)x, ep, (T*)y, n, C)
+    if (C <= 32) T2_ROWS(1, 4);
+    else if (C <= 64) T2_ROWS(1, 8);
+    else if (C <= 128) T2_ROWS(1, 16);
+    else if (C <= 256) T2_ROWS(1, 32);
+    else if (C <= 512) T2_ROWS(2, 32);
+    else if (C <= 1024) T2_ROWS(4, 32);
+    else T2_ROWS(8, 32);
+#undef T2_ROWS
   } else {
-    k_row_epilogue<T><<<grid, 256, 0, st>>>((const T*)x, ep, (T*)y, n, C);
+    k_row_epilogue<T><<<cdiv_i(n * 32, 256), 256, 0, ctx->stream>>>((const T*)x, ep, (T*)y, n, C);
   }
 }
 
@@ -297,9 +357,9 @@ int conv_simt_launch(t2sc_ctx* ctx, const t2sc_plan* plan, const void* x, const 
 
 int row_epilogue_launch(t2sc_ctx* ctx, const void* x, const EpiDev& ep, void* y, i64 n, int C, int dtype) {
   T2_CUDA(ctx, cudaSetDevice(ctx->device));
-  if (dtype == T2SC_F32) row_epilogue_pick<float>(ctx->stream, x, ep, y, n, C);
-  else if (dtype == T2SC_F16) row_epilogue_pick<__half>(ctx->stream, x, ep, y, n, C);
-  else row_epilogue_pick<__nv_bfloat16>(ctx->stream, x, ep, y, n, C);
+  if (dtype == T2SC_F32) row_epilogue_pick<float>(ctx, x, ep, y, n, C);
+  else if (dtype == T2SC_F16) row_epilogue_pick<__half>(ctx, x, ep, y, n, C);
+  else row_epilogue_pick<__nv_bfloat16>(ctx, x, ep, y, n, C);
   T2_LAUNCHED(ctx);
   return T2SC_OK;
 }
