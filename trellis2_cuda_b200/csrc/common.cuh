@@ -48,7 +48,7 @@ struct t2sc_plan {
   int* bounds = nullptr;        // = meta + 8, device [3]: {0, first boundary tile, realised tile count}; parts are [b0,b1) and [b1,b2)
   int* ntiles = nullptr;        // = bounds + 2: realised tile count (<= max_tiles)
   bool split = false;           // made by t2sc_plan_create_split: interior tiles first, boundary tiles last
-  unsigned long long* stats = nullptr;  // device [2]: computed taps, active taps
+  unsigned long long* stats = nullptr;  // device: pairs of computed taps, active taps, to be added up
   i64 max_tiles = 0;
   int tile_rows = 256;           // 128 or 256
 };

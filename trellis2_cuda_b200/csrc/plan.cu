@@ -20,7 +20,7 @@ namespace {
 // surface shell lead: the 8 corner taps, then the 12 edge taps, then the 6 face taps, then the centre.  Rows
 // that differ only in common taps then end up adjacent, which shrinks the union mask of a tile (measured on a
 // 218k-voxel shell: active/computed taps 0.833 -> 0.855 for 128-row tiles).
-__constant__ uint8_t TAP_RANK[27] = {0, 8, 1, 9, 20, 10, 2, 11, 3, 12, 21, 13, 22, 26, 23, 14, 24, 15, 4, 16, 5, 17, 25, 18, 6, 19, 7};
+__device__ constexpr uint8_t TAP_RANK[27] = {0, 8, 1, 9, 20, 10, 2, 11, 3, 12, 21, 13, 22, 26, 23, 14, 24, 15, 4, 16, 5, 17, 25, 18, 6, 19, 7};
 __device__ __forceinline__ uint32_t mask_key(uint32_t g) {
   uint32_t k = 0;
 #pragma unroll
@@ -35,7 +35,7 @@ __device__ __forceinline__ uint32_t mask_key(uint32_t g) {
 // halo_from > 0 (split plan, no src): group 1 = rows with a map entry >= halo_from (a row of a peer), group 0 = the rest
 template <class K>
 __global__ void k_plan_keys(const int* __restrict__ gray, const int* __restrict__ src, const uint32_t* __restrict__ nbr, uint32_t halo_from,
-                            i64 m, i64 block_rows, int block_bits, int drop,
+                            i64 m, uint32_t block_rows, int block_bits, int drop,
                             K* __restrict__ keys, int* __restrict__ iota, int* __restrict__ group_cnt) {
   // group sizes: counted per CTA in shared memory first (millions of rows on eight counters in global memory were the
   // whole time of this kernel)
@@ -52,7 +52,7 @@ __global__ void k_plan_keys(const int* __restrict__ gray, const int* __restrict_
 #pragma unroll 9
       for (int v = 0; v < 27; v++) { const uint32_t r = __ldg(e + v); grp |= (r != NBR_EMPTY && r >= halo_from) ? 1 : 0; }
     }
-    unsigned long long blk = (unsigned long long)(i / block_rows);
+    const unsigned long long blk = (uint32_t)i / block_rows;          // rows are below 2^30: no 64-bit division
     const unsigned long long k = ((unsigned long long)grp << (27 + block_bits)) | (blk << 27) | mask_key((uint32_t)gray[nrow]);
     keys[i] = (K)(k >> drop);
     iota[i] = (int)i;
@@ -72,6 +72,7 @@ __global__ void k_plan_keys(const int* __restrict__ gray, const int* __restrict_
 // the interior part of a split plan is tiles [bounds[0], bounds[1]), its boundary part [bounds[1], bounds[2]); any other
 // plan is all interior.  Without HEADER the descriptors are read back (rebuild of the table alone).
 constexpr uint32_t TABLE_ABSENT = 0x80000000u;
+constexpr int META_SLOTS = 32, META_MAX = 32, META_STATS = META_MAX + META_SLOTS, META_INTS = META_STATS + 4 * META_SLOTS;
 template <int TILE, bool HEADER>
 __global__ void __launch_bounds__(256) k_plan_tiles_table(const uint32_t* __restrict__ nbr, const int* __restrict__ gray, const int* __restrict__ src,
                                                           const int* __restrict__ order, const int* __restrict__ group_cnt, int ngroups, int split,
@@ -81,7 +82,7 @@ __global__ void __launch_bounds__(256) k_plan_tiles_table(const uint32_t* __rest
   const int t = blockIdx.x;
   __shared__ int s_row[TILE];
   __shared__ uint32_t s_e[27 * (TILE + 1)];
-  __shared__ uint32_t s_or;
+  __shared__ uint32_t s_or, s_big;
   __shared__ int s_act, s_part;
   PlanTile tile;
   if constexpr (HEADER) {
@@ -106,6 +107,7 @@ __global__ void __launch_bounds__(256) k_plan_tiles_table(const uint32_t* __rest
     if (t >= bounds[2]) return;
     tile = tiles[t];
   }
+  if (threadIdx.x == 0) s_big = 0;
   __syncthreads();
   uint32_t o = 0; int act = 0;
   for (int j = threadIdx.x; j < TILE; j += 256) {
@@ -127,33 +129,37 @@ __global__ void __launch_bounds__(256) k_plan_tiles_table(const uint32_t* __rest
       if (mask == 0) mask = 1u << 13;       // no row of the tile has any neighbour: one tap of zero-filled rows still initialises the accumulators
       tile.mask = mask;
       tiles[t] = tile;
-      atomicAdd(&stats[0], (unsigned long long)tile.rows * __popc(mask));
-      atomicAdd(&stats[1], (unsigned long long)s_act);
+      atomicAdd(&stats[2 * (t % META_SLOTS)], (unsigned long long)tile.rows * __popc(mask));
+      atomicAdd(&stats[2 * (t % META_SLOTS) + 1], (unsigned long long)s_act);
       if (hist) atomicAdd(&hist[s_part + __popc(mask)], 1);       // tiles of this part with this many taps (k_plan_perm)
     }
   }
   uint32_t big = 0;         // the largest present entry: lets the bounds check skip its scan when every entry is in range
-  // all of a thread's loads are issued before the first of them is used: one load latency per tile, not one per entry
-  constexpr int PER = (TILE * 27 + 255) / 256;
-  uint32_t val[PER];
+  // A warp copies one row of the map per instruction (lane = tap), sixteen rows in flight: no index arithmetic per entry, and
+  // the odd pitch keeps the transposing stores free of bank conflicts.  (With 27 entries spread over 32 lanes and a division
+  // per entry it was no faster, because what held this kernel up were its atomics, see below.)
+  constexpr int BATCH = 16;
+  const int lane = threadIdx.x & 31, tap = lane < 27 ? lane : 26;
+#pragma unroll 1
+  for (int j0 = (threadIdx.x >> 5) * BATCH; j0 < TILE; j0 += 8 * BATCH) {
+    uint32_t val[BATCH];
 #pragma unroll
-  for (int k = 0; k < PER; k++) {
-    const int e = threadIdx.x + 256 * k;
-    val[k] = NBR_EMPTY;
-    if (e < TILE * 27) { const int j = e / 27, v = e - j * 27, nr = s_row[j]; if (nr >= 0) val[k] = __ldg(nbr + (i64)nr * 27 + v); }
-  }
+    for (int k = 0; k < BATCH; k++) {
+      const int nr = s_row[j0 + k];
+      val[k] = nr >= 0 ? __ldg(nbr + (i64)nr * 27 + tap) : NBR_EMPTY;
+    }
 #pragma unroll
-  for (int k = 0; k < PER; k++) {
-    const int e = threadIdx.x + 256 * k;
-    if (e < TILE * 27) {
-      const int j = e / 27, v = e - j * 27;
+    for (int k = 0; k < BATCH; k++) {
       if (val[k] == NBR_EMPTY) val[k] = TABLE_ABSENT; else big = max(big, val[k]);
-      s_e[v * (TILE + 1) + j] = val[k];
+      if (lane < 27) s_e[tap * (TILE + 1) + j0 + k] = val[k];
     }
   }
   big = __reduce_max_sync(0xffffffffu, big);
-  if ((threadIdx.x & 31) == 0 && big > *(volatile uint32_t*)max_entry) atomicMax(max_entry, big);
+  if ((threadIdx.x & 31) == 0) atomicMax(&s_big, big);
   __syncthreads();
+  // One atomic per tile, spread over META_SLOTS words as the statistics are.  (An atomic per warp on one word, which grows from tile
+  // to tile on a scene in order, was most of this kernel: 353 -> 129 us on 3,288,465 rows, whose 710 MB take 108; 24.7 -> 12.5 us on 217,821.)
+  if (threadIdx.x == 0) atomicMax(max_entry + t % META_SLOTS, s_big);
   uint32_t* out = table + (i64)t * 27 * TILE;
   for (int e = threadIdx.x; e < TILE * 27; e += 256) {
     const int v = e / TILE, j = e - v * TILE;
@@ -181,7 +187,7 @@ __global__ void k_plan_perm(const PlanTile* __restrict__ tiles, const int* __res
 // entries at or above n_in (the rows of the feature array) become absent and are reported (status bit 8)
 __global__ void k_plan_table_check(uint32_t* __restrict__ table, const int* __restrict__ ntiles, int per_tile, uint32_t n_in, int* status,
                                    const uint32_t* __restrict__ max_entry) {
-  if (*max_entry < n_in) return;          // the usual case: nothing to blank, nothing to scan
+  if (__reduce_max_sync(0xffffffffu, max_entry[threadIdx.x % META_SLOTS]) < n_in) return;          // the usual case: nothing to blank, nothing to scan
   const i64 n = (i64)*ntiles * per_tile;
   bool bad = false;
   for (i64 i = blockIdx.x * (i64)blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
@@ -196,10 +202,10 @@ int plan_tiles_table(t2sc_ctx* ctx, t2sc_plan* p, const int32_t* gray, const int
   if (p->n_out == 0) return T2SC_OK;
   if (p->tile_rows == 128)
     k_plan_tiles_table<128, HEADER><<<(unsigned)p->max_tiles, 256, 0, ctx->stream>>>(p->nbr, gray, p->src, p->order, gcnt, ngroups, p->split ? 1 : 0, p->n_out,
-                                                                                       p->tiles, p->bounds, p->stats, p->tnbr, (uint32_t*)(p->meta + 11), hist, win);
+                                                                                       p->tiles, p->bounds, p->stats, p->tnbr, (uint32_t*)(p->meta + META_MAX), hist, win);
   else
     k_plan_tiles_table<256, HEADER><<<(unsigned)p->max_tiles, 256, 0, ctx->stream>>>(p->nbr, gray, p->src, p->order, gcnt, ngroups, p->split ? 1 : 0, p->n_out,
-                                                                                       p->tiles, p->bounds, p->stats, p->tnbr, (uint32_t*)(p->meta + 11), hist, win);
+                                                                                       p->tiles, p->bounds, p->stats, p->tnbr, (uint32_t*)(p->meta + META_MAX), hist, win);
   T2_LAUNCHED(ctx);
   if (HEADER && hist) {
     const i64 bins = (cdiv_i(p->max_tiles, win) + 1) * 64;
@@ -217,7 +223,7 @@ int plan_tiles_table(t2sc_ctx* ctx, t2sc_plan* p, const int32_t* gray, const int
 int plan_table_prepare(t2sc_ctx* ctx, t2sc_plan* p, i64 n_in) {
   if (p->table_n_in == n_in || p->n_out == 0) return T2SC_OK;
   if (p->table_n_in >= 0) { int rc = plan_tiles_table<false>(ctx, p, nullptr, nullptr, 0); if (rc != T2SC_OK) return rc; }
-  k_plan_table_check<<<2 * ctx->num_sms, 256, 0, ctx->stream>>>(p->tnbr, p->ntiles, 27 * p->tile_rows, (uint32_t)n_in, ctx->status, (const uint32_t*)(p->meta + 11));
+  k_plan_table_check<<<2 * ctx->num_sms, 256, 0, ctx->stream>>>(p->tnbr, p->ntiles, 27 * p->tile_rows, (uint32_t)n_in, ctx->status, (const uint32_t*)(p->meta + META_MAX));
   T2_LAUNCHED(ctx);
   p->table_n_in = n_in;
   return T2SC_OK;
@@ -260,10 +266,11 @@ static int plan_create(t2sc_ctx* ctx, const uint32_t* nbr, const int32_t* gray, 
   PL(t2_alloc(ctx, &p->tiles, (size_t)p->max_tiles));
   PL(t2_alloc(ctx, &p->perm, (size_t)p->max_tiles));
   PL(t2_alloc(ctx, &p->tnbr, (size_t)p->max_tiles * 27 * tile_rows));
-  // one small block, one memset: group counts [0..8), part bounds [8..11), largest map entry [11], tap statistics (two u64) from int 12
-  PL(t2_alloc(ctx, &p->meta, 16));
-  p->bounds = p->meta + 8; p->ntiles = p->bounds + 2; p->stats = (unsigned long long*)(p->meta + 12);
-  PL(cudaMemsetAsync(p->meta, 0, 16 * sizeof(int), ctx->stream));
+  // one small block, one memset: group counts [0..8), part bounds [8..11), largest map entry and
+  // tap statistics in META_SLOTS words each
+  PL(t2_alloc(ctx, &p->meta, META_INTS));
+  p->bounds = p->meta + 8; p->ntiles = p->bounds + 2; p->stats = (unsigned long long*)(p->meta + META_STATS);
+  PL(cudaMemsetAsync(p->meta, 0, META_INTS * sizeof(int), ctx->stream));
   if (m > 0) {
     int block_bits = 0;
     while (((m + block_rows - 1) / block_rows) > (1ll << block_bits)) block_bits++;
@@ -281,14 +288,14 @@ static int plan_create(t2sc_ctx* ctx, const uint32_t* nbr, const int32_t* gray, 
     int* iota = (int*)(buf + 2 * koff);
     if (narrow) {
       uint32_t *keys = (uint32_t*)buf, *keys2 = (uint32_t*)(buf + koff);
-      k_plan_keys<uint32_t><<<cdiv_i(m, 256), 256, 0, ctx->stream>>>(gray, src, nbr, (uint32_t)halo_from, m, block_rows, block_bits, drop, keys, iota, p->meta);
+      k_plan_keys<uint32_t><<<cdiv_i(m, 256), 256, 0, ctx->stream>>>(gray, src, nbr, (uint32_t)halo_from, m, (uint32_t)(block_rows < m ? block_rows : m), block_bits, drop, keys, iota, p->meta);
       ctx->launches++; PL(cudaGetLastError());
       PL(cub::DeviceRadixSort::SortPairs(nullptr, tb, keys, keys2, iota, p->order, (int)m, 0, key_bits, ctx->stream));
       PL(scratch.get(&tmp, tb));
       PL(cub::DeviceRadixSort::SortPairs(tmp, tb, keys, keys2, iota, p->order, (int)m, 0, key_bits, ctx->stream));
     } else {
       unsigned long long *keys = (unsigned long long*)buf, *keys2 = (unsigned long long*)(buf + koff);
-      k_plan_keys<unsigned long long><<<cdiv_i(m, 256), 256, 0, ctx->stream>>>(gray, src, nbr, (uint32_t)halo_from, m, block_rows, block_bits, drop, keys, iota, p->meta);
+      k_plan_keys<unsigned long long><<<cdiv_i(m, 256), 256, 0, ctx->stream>>>(gray, src, nbr, (uint32_t)halo_from, m, (uint32_t)(block_rows < m ? block_rows : m), block_bits, drop, keys, iota, p->meta);
       ctx->launches++; PL(cudaGetLastError());
       PL(cub::DeviceRadixSort::SortPairs(nullptr, tb, keys, keys2, iota, p->order, (int)m, 0, key_bits, ctx->stream));
       PL(scratch.get(&tmp, tb));
@@ -351,10 +358,11 @@ extern "C" int t2sc_plan_destroy(t2sc_ctx* ctx, t2sc_plan* p) {
 
 extern "C" int t2sc_plan_stats(t2sc_ctx* ctx, t2sc_plan* p, int64_t* tiles, int64_t* computed_taps, int64_t* active_taps) {
   T2_REQ(ctx, ctx && p, "null context or plan");
-  int nt = 0; unsigned long long st[2] = {0, 0};
+  int nt = 0; unsigned long long st[2 * META_SLOTS] = {0};
   T2_CUDA(ctx, cudaMemcpyAsync(&nt, p->ntiles, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   T2_CUDA(ctx, cudaMemcpyAsync(st, p->stats, sizeof(st), cudaMemcpyDeviceToHost, ctx->stream));
   T2_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  for (int q = 1; q < META_SLOTS; q++) { st[0] += st[2 * q]; st[1] += st[2 * q + 1]; }
   if (tiles) *tiles = nt;
   if (computed_taps) *computed_taps = (int64_t)st[0];
   if (active_taps) *active_taps = (int64_t)st[1];
