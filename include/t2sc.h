@@ -102,6 +102,19 @@ int t2sc_subdivide_count(t2sc_ctx* ctx, const void* sub, int sub_dtype, int64_t 
 int t2sc_subdivide_emit(t2sc_ctx* ctx, const void* sub, int sub_dtype, const int32_t* coords, const int32_t* off,
                         int64_t n, int32_t* child_coords, int32_t* src);
 
+/* The same two steps for a level whose children's neighbour map is to be read off the parents' map instead of being hashed.
+ * nbr [n,27] is the map t2sc_build_neighbors made for `coords` in a grid of W x H x D.  count_info also fills info [n] (pairs
+ * {row of the first child, 8-bit set of children}; emit_info writes the first, count_info the second) and tells whether
+ * the parents' map says everything about the children (*whole_host = 1): it does not when two parents share a place or a
+ * parent lies outside the grid.  subdivide_neighbors then gives the map and masks that t2sc_build_neighbors gives for
+ * the children in a grid of 2W x 2H x 2D. */
+int t2sc_subdivide_count_info(t2sc_ctx* ctx, const void* sub, int sub_dtype, const int32_t* coords, const uint32_t* nbr, int W, int H, int D,
+                              int64_t n, int32_t* off, uint32_t* info, int64_t* m_host, int* whole_host);
+int t2sc_subdivide_emit_info(t2sc_ctx* ctx, const void* sub, int sub_dtype, const int32_t* coords, const int32_t* off,
+                             int64_t n, int32_t* child_coords, int32_t* src, uint32_t* info);
+int t2sc_subdivide_neighbors(t2sc_ctx* ctx, const uint32_t* parent_nbr, const uint32_t* info, const int32_t* src, int64_t m,
+                             uint32_t* nbr, int32_t* gray);
+
 /* Replaces k_gather_rows (src/sdec.cu:34-37): y[r,:] = x.view(-1,C)[src[r],:]. */
 int t2sc_gather_rows(t2sc_ctx* ctx, const void* x, const int32_t* src, int64_t m, int C, int dtype, void* y);
 /* Replaces k_add_skip (src/sdec.cu:39-43): h[r,c] += x[src[r]>>3, (src[r]&7)*(Cin/8) + c/rep]. */

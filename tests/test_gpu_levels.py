@@ -1,0 +1,56 @@
+"""A subdivided level's map read off its parents' against the hashed one, bit for bit."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from trellis2_cuda_b200 import scenes
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def sp():
+    import trellis2_cuda_b200 as m
+    m.context()
+    return m
+
+
+def cube(n, res, seed, origin=0, batches=2):
+    rng = np.random.default_rng([n, res, seed])
+    cells = rng.choice(batches * res ** 3, size=n, replace=False)
+    b, r = np.divmod(cells, res ** 3)
+    return np.stack([b, r // (res * res) + origin, r // res % res + origin, r % res + origin], 1).astype(np.int32)
+
+
+@pytest.mark.parametrize("name,coords,extent,derived", [
+    ("one parent", cube(1, 1, 0), 4096, True), ("33 parents", cube(33, 4, 1), 4096, True), ("dense", cube(900, 8, 2), 8, True),
+    ("odd grid", cube(700, 9, 3), 9, True), ("at the end of the grid", cube(500, 8, 4, origin=2040), 4096, True),
+    ("children outside the grid", cube(500, 8, 5, origin=2044), 4096, False), ("parents outside their map's grid", cube(500, 8, 6), 7, False),
+    ("two parents at one place", np.concatenate([cube(300, 8, 7), cube(300, 8, 7)[5:9]]), 4096, False)])
+def test_child_map_from_the_parents(sp, name, coords, extent, derived):
+    n = len(coords)
+    sub = np.random.default_rng(n).standard_normal((n, 8)).astype(np.float16)
+    sub[n // 2] = -1
+    sub[0] = 1
+    d = torch.from_numpy(coords).cuda()
+    lv = sp.subdivide(sp.build_neighbors(d, extent, extent, extent), torch.from_numpy(sub).cuda())
+    cc, src = oracle.subdivide(coords, sub.astype(np.float32) > 0)
+    assert np.array_equal(lv.coords.cpu().numpy(), cc) and np.array_equal(lv.src.cpu().numpy(), src), name
+    want = sp.build_neighbors(lv.coords, want_sorted=False)
+    assert torch.equal(lv.nb.nbr, want.nbr) and torch.equal(lv.nb.gray, want.gray), name
+    if derived:
+        nbr, gray, _, _ = oracle.build_neighbors(cc)
+        assert np.array_equal(lv.nb.nbr.cpu().numpy().view(np.uint32), nbr) and np.array_equal(lv.nb.gray.cpu().numpy(), gray), name
+
+
+def test_child_map_follows_what_the_caller_changed(sp):
+    c = torch.from_numpy(cube(400, 8, 9)).cuda()
+    sub = torch.ones((400, 8), dtype=torch.uint8, device="cuda")
+    parent = sp.build_neighbors(c)
+    parent.nbr.fill_(-1)                      # the map is not what it was built as: the children's comes from their coordinates
+    lv = sp.subdivide(parent, sub)
+    assert torch.equal(lv.nb.nbr, sp.build_neighbors(lv.coords).nbr)
+    with torch.inference_mode():
+        lv = sp.subdivide(sp.build_neighbors(c), sub)
+        assert torch.equal(lv.nb.nbr, sp.build_neighbors(lv.coords).nbr)

@@ -43,7 +43,9 @@ extern "C" int t2sc_ctx_create(int device, void* stream, t2sc_ctx** out) {
   if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess) {
     uint64_t thr = UINT64_MAX; cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr);
   }
-  if ((e = cudaMalloc(&c->status, sizeof(int))) != cudaSuccess || (e = cudaMemset(c->status, 0, sizeof(int))) != cudaSuccess) {
+  if ((e = cudaMalloc(&c->status, sizeof(int))) != cudaSuccess || (e = cudaMemset(c->status, 0, sizeof(int))) != cudaSuccess ||
+      (e = cudaMallocHost(&c->pinned, 64)) != cudaSuccess) {
+    cudaFree(c->status);
     if (c->own_stream) cudaStreamDestroy(c->stream);
     delete c; return t2sc_fail(nullptr, T2SC_ERR_CUDA, "t2sc_ctx_create: %s", cudaGetErrorString(e));
   }
@@ -70,6 +72,7 @@ extern "C" int t2sc_ctx_destroy(t2sc_ctx* ctx) {
   if (ctx->arena) cudaFreeAsync(ctx->arena, ctx->stream);
   cudaStreamSynchronize(ctx->stream);
   cudaFree(ctx->status);
+  cudaFreeHost(ctx->pinned);
   if (ctx->done) cudaEventDestroy(ctx->done);
   if (ctx->own_stream) cudaStreamDestroy(ctx->stream);
   delete ctx;

@@ -94,7 +94,7 @@ __global__ void k_brick_insert(const int4* __restrict__ coords, int n, int Wb, i
   }
 }
 
-// Where a voxel's 8 bricks come from: the hash table.
+// Where a voxel's 8 bricks come from: the hash table, or (a subdivided level) the parent level, whose voxels ARE the bricks.
 struct HashBricks {
   const int4* coords; int W, H, D, Wb, Hb, Db; const unsigned long long* keys; const BrickVals* vals; uint32_t mask;
   // parity of the voxel in its brick, and the 8 rows of brick t = (sx, sy, sz) of its 2x2x2 neighbourhood of bricks: along one
@@ -119,6 +119,25 @@ struct HashBricks {
       if (2 * bz + 1 >= D) v[4] = v[5] = v[6] = v[7] = NBR_EMPTY;
     }
     return (q.y & 1) | ((q.z & 1) << 1) | ((q.w & 1) << 2);
+  }
+};
+
+// A child's brick t is its parent or one of the parent's neighbours; info[q] = {row of q's first child, 8-bit set of its
+// children}, and a parent's children lie in slot order one behind the other.
+struct ParentBricks {
+  const int* src; const uint32_t* nbr; const uint2* info;
+  __device__ __forceinline__ int load(i64 row, int t, uint32_t* v) const {
+    const int sv = __ldg(src + row), p = sv >> 3, slot = sv & 7;
+    // offset of the brick from the parent along an axis: slot bit 0 -> {-1, 0}, 1 -> {0, +1}
+    const int ox = (t & 1) + (slot & 1), oy = ((t >> 1) & 1) + ((slot >> 1) & 1), oz = (t >> 2) + (slot >> 2);
+    const uint32_t q = __ldg(nbr + (i64)p * 27 + ox * 9 + oy * 3 + oz);
+    if (q != NBR_EMPTY) {
+      const uint2 f = __ldg(info + q);
+#pragma unroll
+      for (int e = 0; e < 8; e++)
+        if (f.y >> e & 1) v[e] = f.x + __popc(f.y & ((1u << e) - 1));
+    }
+    return slot;
   }
 };
 
@@ -215,19 +234,30 @@ template <> __device__ __forceinline__ bool sub_keep<__half>(const __half* s, i6
 template <> __device__ __forceinline__ bool sub_keep<__nv_bfloat16>(const __nv_bfloat16* s, i64 e) { return __bfloat162float(s[e]) > 0.f; }
 template <> __device__ __forceinline__ bool sub_keep<uint8_t>(const uint8_t* s, i64 e) { return s[e] != 0; }
 
-template <class T> __global__ void k_c2s_count(const T* __restrict__ sub, int n, int* __restrict__ cnt) {
+// With info: the parent's set of children as bits (k_c2s_emit adds the first child's row), and *partial is set when the
+// children's map cannot be read off the parents' (t2sc_subdivide_neighbors): a parent outside the grid the parents' map was
+// built in, one whose children would leave the children's grid, or one of several parents at one place, of which the
+// parents' map names the first only.
+template <class T> __global__ void k_c2s_count(const T* __restrict__ sub, int n, int* __restrict__ cnt, const int4* __restrict__ co,
+                                               const uint32_t* __restrict__ nbr, int W, int H, int D, uint2* __restrict__ info, int* __restrict__ partial) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  int c = 0;
+  uint32_t bits = 0;
 #pragma unroll
-  for (int s = 0; s < 8; s++) c += sub_keep<T>(sub, (i64)i * 8 + s);
-  cnt[i] = c;
+  for (int s = 0; s < 8; s++) bits |= (sub_keep<T>(sub, (i64)i * 8 + s) ? 1u : 0u) << s;
+  cnt[i] = __popc(bits);
+  if (info) {
+    info[i].y = bits;
+    const int4 q = co[i];
+    if (q.x < 0 || (unsigned)q.y >= (unsigned)W || (unsigned)q.z >= (unsigned)H || (unsigned)q.w >= (unsigned)D || nbr[(i64)i * 27 + 13] != (uint32_t)i) atomicOr(partial, 1);
+  }
 }
 template <class T> __global__ void k_c2s_emit(const T* __restrict__ sub, const int4* __restrict__ co, const int* __restrict__ off,
-                                              int n, int4* __restrict__ nco, int* __restrict__ src) {
+                                              int n, int4* __restrict__ nco, int* __restrict__ src, uint2* __restrict__ info) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   int r = off[i]; int4 q = co[i];
+  if (info) info[i].x = (uint32_t)r;
 #pragma unroll
   for (int s = 0; s < 8; s++)
     if (sub_keep<T>(sub, (i64)i * 8 + s)) {
@@ -345,7 +375,8 @@ extern "C" int t2sc_valid_taps(t2sc_ctx* ctx, const int32_t* gray, const int32_t
   return T2SC_OK;
 }
 
-extern "C" int t2sc_subdivide_count(t2sc_ctx* ctx, const void* sub, int sub_dtype, int64_t n, int32_t* off, int64_t* m_host) {
+static int subdivide_count(t2sc_ctx* ctx, const void* sub, int sub_dtype, int64_t n, int32_t* off, int64_t* m_host,
+                           const int32_t* coords, const uint32_t* nbr, int W, int H, int D, uint32_t* info, int* whole_host) {
   T2_REQ(ctx, ctx != nullptr, "null context");
   T2_REQ(ctx, n >= 0 && n < (1ll << 28), "n=%lld", (long long)n);
   T2_REQ(ctx, sub_dtype == T2SC_F16 || sub_dtype == T2SC_BF16 || sub_dtype == T2SC_U8, "sub dtype %d", sub_dtype);
@@ -356,41 +387,80 @@ extern "C" int t2sc_subdivide_count(t2sc_ctx* ctx, const void* sub, int sub_dtyp
   if (n == 0) return T2SC_OK;
   T2_REQ(ctx, sub != nullptr, "null sub");
   Scratch scratch(ctx);
-  int* cnt = nullptr; char* tmp = nullptr; size_t tb = 0;
+  int *cnt = nullptr, *partial = nullptr; char* tmp = nullptr; size_t tb = 0;
   T2_CUDA(ctx, scratch.get(&cnt, (size_t)n));
+  if (info) {
+    T2_CUDA(ctx, scratch.get(&partial, 1));
+    T2_CUDA(ctx, cudaMemsetAsync(partial, 0, sizeof(int), ctx->stream));
+  }
   int g = cdiv_i(n, 256);
-  if (sub_dtype == T2SC_F16) k_c2s_count<__half><<<g, 256, 0, ctx->stream>>>((const __half*)sub, (int)n, cnt);
-  else if (sub_dtype == T2SC_BF16) k_c2s_count<__nv_bfloat16><<<g, 256, 0, ctx->stream>>>((const __nv_bfloat16*)sub, (int)n, cnt);
-  else k_c2s_count<uint8_t><<<g, 256, 0, ctx->stream>>>((const uint8_t*)sub, (int)n, cnt);
+  const int4* co = (const int4*)coords; uint2* inf = (uint2*)info;
+  if (sub_dtype == T2SC_F16) k_c2s_count<__half><<<g, 256, 0, ctx->stream>>>((const __half*)sub, (int)n, cnt, co, nbr, W, H, D, inf, partial);
+  else if (sub_dtype == T2SC_BF16) k_c2s_count<__nv_bfloat16><<<g, 256, 0, ctx->stream>>>((const __nv_bfloat16*)sub, (int)n, cnt, co, nbr, W, H, D, inf, partial);
+  else k_c2s_count<uint8_t><<<g, 256, 0, ctx->stream>>>((const uint8_t*)sub, (int)n, cnt, co, nbr, W, H, D, inf, partial);
   T2_LAUNCHED(ctx);
   T2_CUDA(ctx, cub::DeviceScan::InclusiveSum(nullptr, tb, cnt, off + 1, (int)n, ctx->stream));
   T2_CUDA(ctx, scratch.get(&tmp, tb));
   T2_CUDA(ctx, cub::DeviceScan::InclusiveSum(tmp, tb, cnt, off + 1, (int)n, ctx->stream));
   if (m_host) {
-    int m = 0;
-    T2_CUDA(ctx, cudaMemcpyAsync(&m, off + n, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    // both words land in the context's pinned block, so one wait covers them
+    T2_CUDA(ctx, cudaMemcpyAsync(ctx->pinned, off + n, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    if (partial) T2_CUDA(ctx, cudaMemcpyAsync(ctx->pinned + 1, partial, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     T2_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    *m_host = m;
+    *m_host = ctx->pinned[0];
+    if (whole_host) *whole_host = ctx->pinned[1] == 0;
   }
   return T2SC_OK;
 }
 
+extern "C" int t2sc_subdivide_count(t2sc_ctx* ctx, const void* sub, int sub_dtype, int64_t n, int32_t* off, int64_t* m_host) {
+  return subdivide_count(ctx, sub, sub_dtype, n, off, m_host, nullptr, nullptr, 0, 0, 0, nullptr, nullptr);
+}
+
+extern "C" int t2sc_subdivide_count_info(t2sc_ctx* ctx, const void* sub, int sub_dtype, const int32_t* coords, const uint32_t* nbr, int W, int H, int D,
+                                         int64_t n, int32_t* off, uint32_t* info, int64_t* m_host, int* whole_host) {
+  T2_REQ(ctx, ctx != nullptr, "null context");
+  T2_REQ(ctx, m_host && whole_host && W > 0 && H > 0 && D > 0, "null result or grid extent %d %d %d", W, H, D);
+  *whole_host = 1;
+  T2_REQ(ctx, n <= 0 || (coords && nbr && info), "null tensor");
+  T2_REQ(ctx, (uintptr_t)coords % 16 == 0 && (uintptr_t)info % 8 == 0, "coords must be 16-byte aligned, info 8-byte");
+  return subdivide_count(ctx, sub, sub_dtype, n, off, m_host, coords, nbr, W, H, D, info, whole_host);
+}
+
 extern "C" int t2sc_subdivide_emit(t2sc_ctx* ctx, const void* sub, int sub_dtype, const int32_t* coords, const int32_t* off,
                                    int64_t n, int32_t* child_coords, int32_t* src) {
+  return t2sc_subdivide_emit_info(ctx, sub, sub_dtype, coords, off, n, child_coords, src, nullptr);
+}
+
+extern "C" int t2sc_subdivide_emit_info(t2sc_ctx* ctx, const void* sub, int sub_dtype, const int32_t* coords, const int32_t* off,
+                                        int64_t n, int32_t* child_coords, int32_t* src, uint32_t* info) {
   T2_REQ(ctx, ctx != nullptr, "null context");
   T2_REQ(ctx, n >= 0 && n < (1ll << 28), "n=%lld", (long long)n);
   T2_REQ(ctx, sub_dtype == T2SC_F16 || sub_dtype == T2SC_BF16 || sub_dtype == T2SC_U8, "sub dtype %d", sub_dtype);
   if (n == 0) return T2SC_OK;
   T2_REQ(ctx, sub && coords && off && child_coords && src, "null tensor");
-  T2_REQ(ctx, (uintptr_t)coords % 16 == 0 && (uintptr_t)child_coords % 16 == 0, "coords must be 16-byte aligned");
+  T2_REQ(ctx, (uintptr_t)coords % 16 == 0 && (uintptr_t)child_coords % 16 == 0 && (uintptr_t)info % 8 == 0, "coords must be 16-byte aligned, info 8-byte");
   T2_CUDA(ctx, cudaSetDevice(ctx->device));
   int g = cdiv_i(n, 256);
-  if (sub_dtype == T2SC_F16)
-    k_c2s_emit<__half><<<g, 256, 0, ctx->stream>>>((const __half*)sub, (const int4*)coords, off, (int)n, (int4*)child_coords, src);
-  else if (sub_dtype == T2SC_BF16)
-    k_c2s_emit<__nv_bfloat16><<<g, 256, 0, ctx->stream>>>((const __nv_bfloat16*)sub, (const int4*)coords, off, (int)n, (int4*)child_coords, src);
-  else
-    k_c2s_emit<uint8_t><<<g, 256, 0, ctx->stream>>>((const uint8_t*)sub, (const int4*)coords, off, (int)n, (int4*)child_coords, src);
+  const int4* co = (const int4*)coords; int4* nco = (int4*)child_coords; uint2* inf = (uint2*)info;
+  if (sub_dtype == T2SC_F16) k_c2s_emit<__half><<<g, 256, 0, ctx->stream>>>((const __half*)sub, co, off, (int)n, nco, src, inf);
+  else if (sub_dtype == T2SC_BF16) k_c2s_emit<__nv_bfloat16><<<g, 256, 0, ctx->stream>>>((const __nv_bfloat16*)sub, co, off, (int)n, nco, src, inf);
+  else k_c2s_emit<uint8_t><<<g, 256, 0, ctx->stream>>>((const uint8_t*)sub, co, off, (int)n, nco, src, inf);
+  T2_LAUNCHED(ctx);
+  return T2SC_OK;
+}
+
+// The children's neighbour map without a hash table: every neighbour of a child is a child of its parent or of one of the
+// parent's 26 neighbours.  (On 3,288,465 children the table took a memset of 335 MB, an atomic insertion per row and eight
+// probes per row.)
+extern "C" int t2sc_subdivide_neighbors(t2sc_ctx* ctx, const uint32_t* parent_nbr, const uint32_t* info, const int32_t* src, int64_t m,
+                                        uint32_t* nbr, int32_t* gray) {
+  T2_REQ(ctx, ctx != nullptr, "null context");
+  T2_REQ(ctx, m >= 0 && m < (1ll << 30), "m=%lld", (long long)m);
+  if (m == 0) return T2SC_OK;
+  T2_REQ(ctx, parent_nbr && info && src && nbr && gray && (uintptr_t)info % 8 == 0, "null or unaligned tensor");
+  T2_CUDA(ctx, cudaSetDevice(ctx->device));
+  k_brick_neighbors<<<cdiv_i(m, 32), 256, 0, ctx->stream>>>(ParentBricks{src, parent_nbr, (const uint2*)info}, (int)m, nbr, gray, nullptr, nullptr);
   T2_LAUNCHED(ctx);
   return T2SC_OK;
 }

@@ -78,6 +78,11 @@ def _chk(t: torch.Tensor, name: str, dtype=None, ndim=None):
         raise T2scError(-1, f"{name} must have {ndim} dims, got {tuple(t.shape)}")
 
 
+def _version(t: torch.Tensor) -> Optional[int]:
+    """How often the tensor was written in place, or None for one made under inference_mode, which does not count that."""
+    return None if t.is_inference() else t._version
+
+
 @dataclasses.dataclass
 class SpConvCfg:
     """Tile configuration, as the reference's ``SpConvCfg{B1,BK,S}`` (src/spconv.h:13)."""
@@ -151,6 +156,21 @@ class SpConvCache:
         self.vk: dict = {}
         self._plan = None
         self._block_rows, self._tile_rows = block_rows, tile_rows
+        self._extent = None       # set by build_neighbors: the grid, and what its map and coordinates were then
+
+    def _built(self, extent) -> "SpConvCache":
+        cv, nv = _version(self.coords), _version(self.nbr)
+        if cv is not None and nv is not None:
+            self._extent = (extent, self.coords, cv, self.nbr, nv)
+        return self
+
+    def _map_extent(self):
+        """The grid this cache's map was built in, or None if the map or the coordinates may have changed since."""
+        if self._extent is None:
+            return None
+        extent, coords, cv, nbr, nv = self._extent
+        same = self.coords is coords and self.nbr is nbr and _version(coords) == cv and _version(nbr) == nv
+        return extent if same else None
 
     def valid(self, B1: int):
         if B1 not in self.vk:
@@ -208,7 +228,7 @@ def build_neighbors(coords: torch.Tensor, W: int = 4096, H: int = 4096, D: int =
     gray = torch.empty(n, dtype=torch.int32, device=coords.device)
     srt = torch.empty(n, dtype=torch.int32, device=coords.device) if want_sorted else None
     ctx.check(ctx.lib.t2sc_build_neighbors(ctx.h, _ptr(coords), n, W, H, D, _ptr(nbr), _ptr(gray), _ptr(srt)))
-    return SpConvCache(ctx, coords, nbr, gray, srt, block_rows, tile_rows)
+    return SpConvCache(ctx, coords, nbr, gray, srt, block_rows, tile_rows)._built((W, H, D))
 
 
 def build_neighbors_range(coords: torch.Tensor, row_lo: int, row_hi: int, W: int = 4096, H: int = 4096, D: int = 4096):
@@ -399,13 +419,25 @@ def subdivide(parent: SpConvCache, sub: torch.Tensor, want_sorted: bool = False)
     ctx = parent.ctx
     off = torch.empty(n + 1, dtype=torch.int32, device=sub.device)
     m = ctypes.c_int64(0)
-    ctx.check(ctx.lib.t2sc_subdivide_count(ctx.h, _ptr(sub), _DT[sub.dtype], n, _ptr(off), ctypes.byref(m)))
+    extent = None if want_sorted else parent._map_extent()
+    whole, info = ctypes.c_int(0), None
+    if extent is not None:        # the children's grid is 4096^3, so a parent past 2047 has children outside it
+        info = torch.empty((n, 2), dtype=torch.int32, device=sub.device)
+        ctx.check(ctx.lib.t2sc_subdivide_count_info(ctx.h, _ptr(sub), _DT[sub.dtype], _ptr(parent.coords), _ptr(parent.nbr),
+                                                    *(min(e, 2048) for e in extent), n, _ptr(off), _ptr(info), ctypes.byref(m), ctypes.byref(whole)))
+    else:
+        ctx.check(ctx.lib.t2sc_subdivide_count(ctx.h, _ptr(sub), _DT[sub.dtype], n, _ptr(off), ctypes.byref(m)))
     coords = torch.empty((m.value, 4), dtype=torch.int32, device=sub.device)
     src = torch.empty(m.value, dtype=torch.int32, device=sub.device)
     if m.value:
-        ctx.check(ctx.lib.t2sc_subdivide_emit(ctx.h, _ptr(sub), _DT[sub.dtype], _ptr(parent.coords), _ptr(off), n, _ptr(coords), _ptr(src)))
-    nb = build_neighbors(coords, 4096, 4096, 4096, want_sorted=want_sorted)
-    return Level(coords, src, nb, parent)
+        ctx.check(ctx.lib.t2sc_subdivide_emit_info(ctx.h, _ptr(sub), _DT[sub.dtype], _ptr(parent.coords), _ptr(off), n, _ptr(coords), _ptr(src), _ptr(info)))
+    if not (whole.value and m.value):
+        return Level(coords, src, build_neighbors(coords, 4096, 4096, 4096, want_sorted=want_sorted), parent)
+    # every parent is in the grid and alone at its place: the children's map follows from the parents'
+    nbr = torch.empty((m.value, 27), dtype=torch.int32, device=sub.device)
+    gray = torch.empty(m.value, dtype=torch.int32, device=sub.device)
+    ctx.check(ctx.lib.t2sc_subdivide_neighbors(ctx.h, _ptr(parent.nbr), _ptr(info), _ptr(src), m.value, _ptr(nbr), _ptr(gray)))
+    return Level(coords, src, SpConvCache(ctx, coords, nbr, gray, None)._built((4096, 4096, 4096)), parent)
 
 
 def subdiv_conv(x: torch.Tensor, w: torch.Tensor, b: Optional[torch.Tensor], level: Level, *, ln=None, act=None,
