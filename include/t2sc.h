@@ -183,6 +183,13 @@ typedef struct {
 int t2sc_subm_conv(t2sc_ctx* ctx, t2sc_plan* plan, const void* x, const void* w, const t2sc_epilogue* ep,
                    void* y, int dtype, int64_t n_in, int Ci, int Co, int variant);
 
+/* The conv1 -> k_gather_rows pair from the PARENTS' submanifold plan (128-row tiles, no src): every parent row is multiplied with
+ * all 8 weight sets and only kept children are stored.  y [m,Cc] in child order, w [8*Cc,27,Ci], bias [8*Cc]; info as left by
+ * t2sc_subdivide_emit_info; Cc = 64, fp16 / bf16, Ci % 64 == 0, no skip.  The bits are those of t2sc_subm_conv with a
+ * subdivision plan. */
+int t2sc_subdiv_conv_parents(t2sc_ctx* ctx, t2sc_plan* parent_plan, const void* x, const void* w, const t2sc_epilogue* ep, void* y,
+                             int dtype, int64_t n_in, int Ci, int Cc, const uint32_t* info);
+
 /* t2sc_subm_conv over one part of a plan (T2SC_PART_*): the rows of the other part are left untouched in y.  n_in is the
  * index space of the plan's map as for t2sc_subm_conv; T2SC_PART_INTERIOR of a split plan reads rows below n_own only, so
  * x may end there (a rank whose boundary tiles gather the halo rows from peer memory never copies them). */

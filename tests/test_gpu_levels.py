@@ -54,3 +54,26 @@ def test_child_map_follows_what_the_caller_changed(sp):
     with torch.inference_mode():
         lv = sp.subdivide(sp.build_neighbors(c), sub)
         assert torch.equal(lv.nb.nbr, sp.build_neighbors(lv.coords).nbr)
+
+
+@pytest.mark.parametrize("n,Ci,dt", [(1, 64, torch.float16), (129, 128, torch.bfloat16), (1500, 192, torch.float16)])
+def test_subdivision_conv_over_the_parents_tiles(sp, n, Ci, dt):
+    """Every slot of every parent, kept children stored, against the children's own tiles: the same products in the same order."""
+    g = torch.Generator(device="cuda").manual_seed(n)
+    coords = torch.from_numpy(cube(n, max(2, round((n / 1.2) ** (1 / 3))), 1)).cuda()
+    sub = (torch.rand((n, 8), generator=g, device="cuda") < 0.6).to(torch.uint8)
+    sub[0] = 1
+    if n > 8:
+        sub[5] = 0
+    x = torch.randn((n, Ci), generator=g, device="cuda").to(dt)
+    w = (torch.randn((8 * 64, 27, Ci), generator=g, device="cuda") * 0.03).to(dt)
+    b = torch.randn(8 * 64, generator=g, device="cuda").to(dt)
+    gamma, beta = torch.rand(64, generator=g, device="cuda") + 0.5, torch.randn(64, generator=g, device="cuda")
+    level = sp.subdivide(sp.build_neighbors(coords), sub)
+    assert level._from_parents(x, 64)
+    for kw in (dict(), dict(ln=(None, None, 1e-6), act="silu"), dict(ln=(gamma, beta, 1e-6), act="gelu")):
+        for bias in (b, None):
+            assert torch.equal(sp.subdiv_conv(x, w, bias, level, **kw), sp.subdiv_conv(x, w, bias, level, variant="umma", **kw)), kw
+    sp.context().device_status()
+    level.src = level.src.clone()             # no longer the list its parents' children were counted for
+    assert not level._from_parents(x, 64)

@@ -149,6 +149,21 @@ extern "C" int t2sc_subm_conv_part(t2sc_ctx* ctx, t2sc_plan* plan, const void* x
   return row_epilogue_launch(ctx, y, rest, y, plan->n_out, Co, dtype);
 }
 
+extern "C" int t2sc_subdiv_conv_parents(t2sc_ctx* ctx, t2sc_plan* plan, const void* x, const void* w, const t2sc_epilogue* ep, void* y,
+                                        int dtype, int64_t n_in, int Ci, int Cc, const uint32_t* info) {
+  T2_REQ(ctx, ctx && plan, "null context or plan");
+  T2_REQ(ctx, n_in == plan->n_in, "spconv shapes: x has %lld rows, the plan's neighbour map is over %lld", (long long)n_in, (long long)plan->n_in);
+  EpiDev e = epi_dev(ep);
+  if ((dtype != T2SC_F16 && dtype != T2SC_BF16) || Ci <= 0 || Ci % 64 || Cc != CONV_CHILD_CO || plan->src || plan->tile_rows != 128 || plan->split || e.skip_x)
+    return t2sc_fail(ctx, T2SC_ERR_UNSUPPORTED, "subdivision conv from the parents' plan needs fp16/bf16, Ci %% 64 == 0, Cc == %d, a submanifold plan with 128-row tiles, no skip (Ci=%d Cc=%d dtype=%d)",
+                     CONV_CHILD_CO, Ci, Cc, dtype);
+  if (plan->n_out == 0) return T2SC_OK;
+  T2_REQ(ctx, x && w && y && info, "null tensor");
+  T2_REQ(ctx, (uintptr_t)x % 16 == 0 && (uintptr_t)w % 16 == 0 && (uintptr_t)y % 16 == 0 && (uintptr_t)info % 8 == 0, "x, w, y must be 16-byte aligned, info 8-byte");
+  T2_REQ(ctx, (uintptr_t)e.bias % 16 == 0 && (uintptr_t)e.residual % 16 == 0, "epilogue bias and residual must be 16-byte aligned");
+  return conv_umma_launch(ctx, plan, x, w, 8ll * Cc, e, y, dtype, n_in, Ci, Cc, T2SC_PART_ALL, nullptr, nullptr, 0, 0, nullptr, info);
+}
+
 extern "C" int t2sc_subm_conv_peers(t2sc_ctx* ctx, t2sc_plan* plan, const void* const* x_peers, const int64_t* rows_peers, int n_peers,
                                     int self_rank, const void* w, const t2sc_epilogue* ep, void* y, int dtype, int Ci, int Co) {
   return t2sc_subm_conv_peers_part(ctx, plan, nullptr, x_peers, rows_peers, n_peers, self_rank, w, ep, y, dtype, Ci, Co, T2SC_PART_ALL);

@@ -53,7 +53,10 @@ using namespace umma;
 // Only the peer-memory form, whose map arrives with the call, still has two index warps that build the table from map
 // rows (4-byte cp.async, one 108-byte row per warp instruction), mark absent / out-of-range entries and flag the taps
 // that read a peer.
-template <int BN, int MH, int G, int U, bool PEERS, bool TAIL, class T>
+//
+// CHILD > 0 (subdivision conv from the parents' tiles): the BN columns are BN / CHILD child slots of CHILD channels; the epilogue
+// treats each as a row of its own, of the child that sits there, and skips slots that are not kept.
+template <int BN, int MH, int G, int U, bool PEERS, bool TAIL, int CHILD, class T>
 __global__ void __launch_bounds__(num_threads(MH, G), 1) k_conv_umma(const __grid_constant__ CUtensorMap tmw, const ConvArgs a) {
   static_assert(!TAIL || (MH == 1 && !PEERS), "half chunks run on 128-row tiles of local rows");
   static_assert(G == 1 || (G == 2 && MH == 1), "a second gather group only fits beside 128-row tiles");
@@ -102,7 +105,7 @@ __global__ void __launch_bounds__(num_threads(MH, G), 1) k_conv_umma(const __gri
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   if (a.ep.ln) {        // the whole row is one accumulator (n_cot == 1): column = index
-    for (int i = threadIdx.x; i < BN; i += blockDim.x) { gamma_s[i] = a.ep.gamma ? a.ep.gamma[i] : 1.f; beta_s[i] = a.ep.beta ? a.ep.beta[i] : 0.f; }
+    for (int i = threadIdx.x; i < (CHILD ? CHILD : BN); i += blockDim.x) { gamma_s[i] = a.ep.gamma ? a.ep.gamma[i] : 1.f; beta_s[i] = a.ep.beta ? a.ep.beta[i] : 0.f; }
   }
   if (warp == WARP_MMA) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");
@@ -455,6 +458,8 @@ __global__ void __launch_bounds__(num_threads(MH, G), 1) k_conv_umma(const __gri
       const uint32_t buf = acc_it % NB, aph = (acc_it / NB) & 1;
       const int orow = j < tile.rows ? (dense ? tile.start + j : a.order[tile.start + j]) : -1;
       const int wcol0 = tile.wbase * a.Co + cot * BN;      // bias index of this item's first column
+      uint2 kids = make_uint2(0u, 0u);
+      if constexpr (CHILD > 0) { if (orow >= 0) kids = __ldg(a.child_info + orow); }
       int sp = 0, ss = 0;
       if (has_skip && orow >= 0) { int sv = a.ep.skip_src[orow]; sp = sv >> 3; ss = sv & 7; }
       // this warp's copy of the item's bias values, in flight while it waits for the accumulator
@@ -470,7 +475,17 @@ __global__ void __launch_bounds__(num_threads(MH, G), 1) k_conv_umma(const __gri
       if (warp == WARP_EPI0 && lane == 0) trace(a, 4, 1, acc_it);
       tc_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + buf * (MH * BN) + half * BN;
-      if (!diag(a, 64)) epilogue_row<BN, T>(a, taddr, orow, cot, a.ep.bias ? bias_w : nullptr, gamma_s, beta_s, sp, ss);
+      if constexpr (CHILD > 0) {
+#pragma unroll 1
+        for (int s = 0; s < BN / CHILD; s++) {
+          const int slot = cot * (BN / CHILD) + s;
+          const int crow = kids.y >> slot & 1 ? (int)kids.x + __popc(kids.y & ((1u << slot) - 1)) : -1;
+          if (__any_sync(0xffffffffu, crow >= 0))
+            epilogue_row<CHILD, T>(a, taddr + s * CHILD, crow, 0, a.ep.bias ? bias_w + s * CHILD : nullptr, gamma_s, beta_s, 0, 0);
+        }
+      } else {
+        if (!diag(a, 64)) epilogue_row<BN, T>(a, taddr, orow, cot, a.ep.bias ? bias_w : nullptr, gamma_s, beta_s, sp, ss);
+      }
       tc_fence_before();
       mbar_arrive(bar_acce + 8 * buf);
       if (warp == WARP_EPI0 && lane == 0) trace(a, 4, 2, acc_it);
@@ -505,17 +520,17 @@ static EncodeTiledFn encode_fn() {
   return fn;
 }
 
-template <int BN, int MH, int G, int U, bool PEERS, class T, bool TAIL = false>
+template <int BN, int MH, int G, int U, bool PEERS, class T, bool TAIL = false, int CHILD = 0>
 int launch_p(t2sc_ctx* ctx, const CUtensorMap& tm, const ConvArgs& args, i64 max_items) {
   constexpr int smem = num_stages(BN, MH, U) * U * stage_bytes(BN, MH) + aux_bytes(MH) + 1024;
   static_assert(smem <= SMEM_BUDGET && num_stages(BN, MH, U) >= 2, "shared memory budget");
   static bool attr_set[16] = {};
   if (!attr_set[ctx->device & 15]) {
-    T2_CUDA(ctx, cudaFuncSetAttribute(k_conv_umma<BN, MH, G, U, PEERS, TAIL, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    T2_CUDA(ctx, cudaFuncSetAttribute(k_conv_umma<BN, MH, G, U, PEERS, TAIL, CHILD, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     attr_set[ctx->device & 15] = true;
   }
   int grid = (int)(max_items < ctx->num_sms ? max_items : ctx->num_sms);
-  k_conv_umma<BN, MH, G, U, PEERS, TAIL, T><<<grid, num_threads(MH, G), smem, ctx->stream>>>(tm, args);
+  k_conv_umma<BN, MH, G, U, PEERS, TAIL, CHILD, T><<<grid, num_threads(MH, G), smem, ctx->stream>>>(tm, args);
   T2_LAUNCHED(ctx);
   return T2SC_OK;
 }
@@ -587,11 +602,11 @@ bool conv_umma_fuses_ln(int Co, bool pow2) { return pick_bn(Co, pow2) == Co; }
 
 int conv_umma_launch(t2sc_ctx* ctx, const t2sc_plan* plan, const void* x, const void* w, i64 w_rows, const EpiDev& ep, void* y,
                      int dtype, i64 n_in, int Ci, int Co, int part, const void* const* x_peers, const int64_t* rows_peers, int n_peers,
-                     int self_rank, const uint32_t* peer_nbr) {
+                     int self_rank, const uint32_t* peer_nbr, const uint32_t* child_info) {
   T2_CUDA(ctx, cudaSetDevice(ctx->device));
-  const int BN = pick_bn(Co, n_peers > 0 || plan->tile_rows != TILE_M);
+  const int BN = child_info ? 256 : pick_bn(Co, n_peers > 0 || plan->tile_rows != TILE_M);
   T2_REQ(ctx, BN > 0, "Co=%d", Co);
-  T2_REQ(ctx, !ep.ln || Co == BN, "fused LayerNorm needs the whole row in one tile (Co=%d)", Co);
+  T2_REQ(ctx, !ep.ln || Co == BN || child_info, "fused LayerNorm needs the whole row in one tile (Co=%d)", Co);
   EncodeTiledFn enc = encode_fn();
   if (!enc) return t2sc_fail(ctx, T2SC_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
   // weights [w_rows, 27, Ci] as a 3-D tensor (innermost first): Ci, 27, w_rows; box = 64 channels x 1 tap x BN rows
@@ -623,10 +638,14 @@ int conv_umma_launch(t2sc_ctx* ctx, const t2sc_plan* plan, const void* x, const 
   args.perm = plan->balanced ? plan->perm : nullptr;
   args.x = x; args.y = y; args.nbr = peer_nbr ? peer_nbr : plan->nbr; args.order = plan->order; args.src = plan->src;
   args.tiles = plan->tiles; args.tile_lo = tile_part(plan, part).lo; args.tile_hi = tile_part(plan, part).hi; args.status = ctx->status;
-  args.Ci = Ci; args.Co = Co; args.n_cot = Co / BN; args.is_bf16 = dtype == T2SC_BF16; args.ep = ep;
+  args.Ci = Ci; args.Co = Co; args.n_cot = (child_info ? 8 * Co : Co) / BN; args.is_bf16 = dtype == T2SC_BF16; args.ep = ep;
+  args.child_info = (const uint2*)child_info;
   i64 max_items = plan->max_tiles * args.n_cot;
   int rc;
-  if (plan->tile_rows == 2 * TILE_M)
+  if (child_info)
+    rc = dtype == T2SC_BF16 ? launch_p<256, 1, 1, 1, false, __nv_bfloat16, false, CONV_CHILD_CO>(ctx, tm, args, max_items)
+                            : launch_p<256, 1, 1, 1, false, __half, false, CONV_CHILD_CO>(ctx, tm, args, max_items);
+  else if (plan->tile_rows == 2 * TILE_M)
     rc = dtype == T2SC_BF16 ? launch_t<2, __nv_bfloat16>(ctx, BN, tm, args, max_items) : launch_t<2, __half>(ctx, BN, tm, args, max_items);
   else
     rc = dtype == T2SC_BF16 ? launch_t<1, __nv_bfloat16>(ctx, BN, tm, args, max_items) : launch_t<1, __half>(ctx, BN, tm, args, max_items);

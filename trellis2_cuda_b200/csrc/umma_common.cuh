@@ -68,6 +68,7 @@ struct ConvArgs {
   uint32_t xp_rows[8];      // PEERS: rows of every peer's array
   int dense_rows;           // > 0: no neighbour map at all - a plain row-major GEMM over this many rows (t2sc_linear): tile t is rows
                             // [t * tile rows, ...), its one "tap" reads input row = output row, weights are [Co, 1, Ci]
+  const uint2* child_info;  // CHILD form: {row of the first child, set of children} per parent row
   long long* trace;         // diagnostic build only (T2SC_TRACE=file): per-tile timestamps of CTA 0's roles, [role][event][tile < 64]
   int wait_limit;           // bounded waits give up after this many cycles >> WAIT_LIMIT_SHIFT
   int dbg_skip;             // diagnostic build only (T2SC_DEBUG_SKIP), always 0 in the shipped library: 1 = no A gather, 2 = no B load,
@@ -89,6 +90,7 @@ static inline void diag_args(ConvArgs& args) {
   args.trace = nullptr;
   args.dense_rows = 0;
   args.perm = nullptr;
+  args.child_info = nullptr;
   args.wait_limit = (int)(WAIT_LIMIT_CYCLES >> WAIT_LIMIT_SHIFT);
 #ifdef T2SC_DIAG
   static const int dbg_skip = [] { const char* e = getenv("T2SC_DEBUG_SKIP"); return e ? atoi(e) : 0; }();

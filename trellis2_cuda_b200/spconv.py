@@ -370,6 +370,21 @@ def _conv(ctx, plan, x, w, b, Co, ln, act, residual, skip, variant, out):
     return y
 
 
+def _conv_parents(level, x, w, b, ln, act, out):
+    _chk(x, "x", None, 2); _chk(w, "w", x.dtype, 3)
+    Ci, Cc = x.shape[1], w.shape[0] // 8
+    if w.shape[1] != 27 or w.shape[2] != Ci:
+        raise T2scError(-1, f"spconv shapes: w {tuple(w.shape)} does not match x {tuple(x.shape)}")
+    ctx, plan = level.parent.ctx, level.parent.plan_for(256, Ci)
+    y = out if out is not None else torch.empty((level.src.shape[0], Cc), dtype=x.dtype, device=x.device)
+    e, keep = _epilogue(Cc, x.dtype, b, ln, act, None, None)
+    plan.set_input_rows(x.shape[0])
+    info = level._info[0]
+    plan.keep = keep + [info]             # as in _conv
+    ctx.check(ctx.lib.t2sc_subdiv_conv_parents(ctx.h, plan.h, _ptr(x), _ptr(w), ctypes.byref(e), _ptr(y), _DT[x.dtype], x.shape[0], Ci, Cc, _ptr(info)))
+    return y
+
+
 def subm_conv(x: torch.Tensor, w: torch.Tensor, b: Optional[torch.Tensor], c: SpConvCache, *, ln=None, act=None,
               residual=None, skip=None, variant: str = "auto", out=None) -> torch.Tensor:
     """y = subm_conv3d(x, w, b) (src/spconv.cu:160-175): x [N,Ci], w [Co,27,Ci], b [Co] or None -> [N,Co] in
@@ -390,6 +405,16 @@ class Level:
     nb: SpConvCache
     parent: Optional[SpConvCache] = None
     _up_plans: Optional[dict] = None
+    _info: Optional[tuple] = None      # (int32 [n,2]: first child and set of children of every parent, the src it belongs to, its version)
+
+    def _from_parents(self, x: torch.Tensor, Cc: int) -> bool:
+        """Whether the subdivision conv runs over the parents' tiles with all 8 slots (t2sc_subdiv_conv_parents) or over the
+        children's.  At 64 child channels a tile of children takes as long to gather as a tile of parents does, and
+        computes a quarter of what the 256-column tile of four slots computes: all 8 slots cost what about 2.7 cost
+        one by one, and the children need no schedule of their own."""
+        return (self._info is not None and self.src is self._info[1] and _version(self.src) == self._info[2] and Cc == 64
+                and x.dtype in (torch.float16, torch.bfloat16) and x.shape[1] % 64 == 0
+                and self.parent._tile_rows_for(256, x.shape[1]) == 128 and self.src.shape[0] > 2.7 * self.parent.N)
 
     def up_plan_for(self, Cc: int, Ci: int = 64) -> _Plan:
         """Schedule of the subdivision conv into Cc child channels: 256-row tiles, two 128-row accumulators per weight slab
@@ -419,7 +444,7 @@ def subdivide(parent: SpConvCache, sub: torch.Tensor, want_sorted: bool = False)
     ctx = parent.ctx
     off = torch.empty(n + 1, dtype=torch.int32, device=sub.device)
     m = ctypes.c_int64(0)
-    extent = None if want_sorted else parent._map_extent()
+    extent = parent._map_extent()
     whole, info = ctypes.c_int(0), None
     if extent is not None:        # the children's grid is 4096^3, so a parent past 2047 has children outside it
         info = torch.empty((n, 2), dtype=torch.int32, device=sub.device)
@@ -431,13 +456,14 @@ def subdivide(parent: SpConvCache, sub: torch.Tensor, want_sorted: bool = False)
     src = torch.empty(m.value, dtype=torch.int32, device=sub.device)
     if m.value:
         ctx.check(ctx.lib.t2sc_subdivide_emit_info(ctx.h, _ptr(sub), _DT[sub.dtype], _ptr(parent.coords), _ptr(off), n, _ptr(coords), _ptr(src), _ptr(info)))
-    if not (whole.value and m.value):
-        return Level(coords, src, build_neighbors(coords, 4096, 4096, 4096, want_sorted=want_sorted), parent)
+    known = (info, src, _version(src)) if info is not None and m.value and _version(src) is not None else None
+    if not (whole.value and m.value) or want_sorted:
+        return Level(coords, src, build_neighbors(coords, 4096, 4096, 4096, want_sorted=want_sorted), parent, None, known)
     # every parent is in the grid and alone at its place: the children's map follows from the parents'
     nbr = torch.empty((m.value, 27), dtype=torch.int32, device=sub.device)
     gray = torch.empty(m.value, dtype=torch.int32, device=sub.device)
     ctx.check(ctx.lib.t2sc_subdivide_neighbors(ctx.h, _ptr(parent.nbr), _ptr(info), _ptr(src), m.value, _ptr(nbr), _ptr(gray)))
-    return Level(coords, src, SpConvCache(ctx, coords, nbr, gray, None)._built((4096, 4096, 4096)), parent)
+    return Level(coords, src, SpConvCache(ctx, coords, nbr, gray, None)._built((4096, 4096, 4096)), parent, None, known)
 
 
 def subdiv_conv(x: torch.Tensor, w: torch.Tensor, b: Optional[torch.Tensor], level: Level, *, ln=None, act=None,
@@ -449,6 +475,8 @@ def subdiv_conv(x: torch.Tensor, w: torch.Tensor, b: Optional[torch.Tensor], lev
         raise T2scError(-1, "subdivision conv needs 8*Cc weight rows")
     if x.shape[0] != level.parent.N:
         raise T2scError(-1, f"spconv shapes: x has {x.shape[0]} rows, parent cache has {level.parent.N}")
+    if variant == "auto" and level._from_parents(x, w.shape[0] // 8):
+        return _conv_parents(level, x, w, b, ln, act, out)
     return _conv(level.parent.ctx, level.up_plan_for(w.shape[0] // 8, w.shape[-1]), x, w, b, w.shape[0] // 8, ln, act, None, None, variant, out)
 
 
