@@ -74,6 +74,9 @@ extern "C" int t2sc_ctx_destroy(t2sc_ctx* ctx) {
   cudaFree(ctx->status);
   cudaFreeHost(ctx->pinned);
   if (ctx->done) cudaEventDestroy(ctx->done);
+  for (cudaEvent_t v : ctx->ev) if (v) cudaEventDestroy(v);
+  if (ctx->copy_in) cudaStreamDestroy(ctx->copy_in);
+  if (ctx->copy_out) cudaStreamDestroy(ctx->copy_out);
   if (ctx->own_stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
   return T2SC_OK;
@@ -109,6 +112,11 @@ extern "C" int t2sc_subm_conv_part(t2sc_ctx* ctx, t2sc_plan* plan, const void* x
                                    void* y, int dtype, int64_t n_in, int Ci, int Co, int variant, int part) {
   T2_REQ(ctx, ctx && plan, "null context or plan");
   T2_REQ(ctx, part == T2SC_PART_ALL || part == T2SC_PART_INTERIOR || part == T2SC_PART_BOUNDARY, "part=%d", part);
+  return conv_dispatch(ctx, plan, x, w, ep, y, dtype, n_in, Ci, Co, variant, part);
+}
+
+int conv_dispatch(t2sc_ctx* ctx, t2sc_plan* plan, const void* x, const void* w, const t2sc_epilogue* ep, void* y, int dtype, int64_t n_in,
+                  int Ci, int Co, int variant, int part) {
   T2_REQ(ctx, dtype == T2SC_F32 || dtype == T2SC_F16 || dtype == T2SC_BF16, "dtype %d", dtype);
   T2_REQ(ctx, Ci > 0 && Co > 0 && Ci % 32 == 0, "spconv shapes Ci=%d Co=%d (Ci must be a multiple of 32)", Ci, Co);
   // the reference requires N == c.N (src/spconv.cu:162); a plan whose map indexes a longer array says so (t2sc_plan_set_input_rows)
@@ -257,6 +265,56 @@ extern "C" int t2sc_row_epilogue(t2sc_ctx* ctx, const void* x, const t2sc_epilog
 }
 
 // ------------------------------------------------------------------------------------------ host-buffer operator
+namespace {
+// rows list[0..count) of y [n, vecs] to the same rows of out (pinned host memory): a warp per row, whole lines
+__global__ void k_rows_out(const uint4* __restrict__ y, const int* __restrict__ list, int count, int vecs, uint4* __restrict__ out) {
+  const i64 row = (blockIdx.x * (i64)blockDim.x + threadIdx.x) >> 5;
+  if (row >= count) return;
+  const i64 at = (i64)list[row] * vecs;
+  for (int c = threadIdx.x & 31; c < vecs; c += 32) out[at + c] = __ldg(y + at + c);
+}
+
+// device address of a pinned host buffer, or null for pageable memory
+void* pinned_address(const void* p) {
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) { (void)cudaGetLastError(); return nullptr; }
+  return at.type == cudaMemoryTypeHost ? at.devicePointer : nullptr;
+}
+
+// The call's device buffers and plan, returned when it ends; copies on the side streams end first.
+struct HostCall {
+  t2sc_ctx* ctx;
+  int32_t *coords = nullptr, *gray = nullptr; uint32_t* nbr = nullptr;
+  char *x = nullptr, *w = nullptr, *b = nullptr, *y = nullptr;
+  int* late = nullptr;
+  t2sc_plan* plan = nullptr;
+  bool side = false;            // work may be in flight on the side streams
+  explicit HostCall(t2sc_ctx* c) : ctx(c) {}
+  ~HostCall() {
+    if (side) { cudaStreamSynchronize(ctx->copy_in); cudaStreamSynchronize(ctx->copy_out); }
+    if (plan) t2sc_plan_destroy(ctx, plan);
+    t2_free(ctx, coords); t2_free(ctx, nbr); t2_free(ctx, gray); t2_free(ctx, x); t2_free(ctx, w); t2_free(ctx, b); t2_free(ctx, y); t2_free(ctx, late);
+  }
+};
+
+cudaError_t side_streams(t2sc_ctx* ctx) {
+  cudaError_t e = cudaSuccess;
+  for (cudaStream_t* s : {&ctx->copy_in, &ctx->copy_out})
+    if (!*s && (e = cudaStreamCreateWithFlags(s, cudaStreamNonBlocking)) != cudaSuccess) return e;
+  for (cudaEvent_t& v : ctx->ev)
+    if (!v && (e = cudaEventCreateWithFlags(&v, cudaEventDisableTiming)) != cudaSuccess) return e;
+  return e;
+}
+}  // namespace
+
+// Bound by the link: features in and results out are about 2 ms each way on 218 k rows of 256 channels (PCIe, 55 GB/s), the
+// kernels 0.5 ms.  Copying in, computing and copying out one after the other left each direction of the link idle half
+// of the time.  With pinned buffers the features go in as up to 8 chunks of rows on a stream of their own while the map and
+// the plan are made from the coordinates, which went first; the plan groups the rows by the last chunk they read, each
+// group's tiles run when that chunk has arrived, and then the chunk of results with the same number goes out on a third
+// stream.  The rows of it that still wait for a later chunk (a few per cent of a scene in Morton order) are written to the
+// host buffer by k_rows_out at the end.  Where they are more than an eighth of all rows (a scene in random order), everything
+// goes out at the end in one copy.  A chunk is at least 4 MB, 70 us of link time: less than that is not worth its launches.
 extern "C" int t2sc_subm_conv_host(t2sc_ctx* ctx, const int32_t* coords_host, int64_t n, int W, int H, int D,
                                    const void* x_host, const void* w_host, const void* bias_host, void* y_host,
                                    int dtype, int Ci, int Co) {
@@ -265,38 +323,85 @@ extern "C" int t2sc_subm_conv_host(t2sc_ctx* ctx, const int32_t* coords_host, in
   if (n == 0) return T2SC_OK;
   T2_REQ(ctx, coords_host && x_host && w_host && y_host, "null host buffer");
   T2_REQ(ctx, dtype == T2SC_F32 || dtype == T2SC_F16 || dtype == T2SC_BF16, "dtype %d", dtype);
-  size_t es = dtype_size(dtype);
-  int32_t* coords = nullptr; uint32_t* nbr = nullptr; int32_t* gray = nullptr;
-  char *x = nullptr, *w = nullptr, *b = nullptr, *y = nullptr;
-  t2sc_plan* plan = nullptr;
-  int rc = T2SC_OK;
-  auto cleanup = [&]() {
-    if (plan) t2sc_plan_destroy(ctx, plan);
-    t2_free(ctx, coords); t2_free(ctx, nbr); t2_free(ctx, gray); t2_free(ctx, x); t2_free(ctx, w); t2_free(ctx, b); t2_free(ctx, y);
-  };
-#define HOST_TRY(call) do { cudaError_t e_ = (call); if (e_ != cudaSuccess) { cleanup(); return t2sc_fail(ctx, T2SC_ERR_CUDA, "CUDA %s: %s", #call, cudaGetErrorString(e_)); } } while (0)
-  HOST_TRY(cudaSetDevice(ctx->device));
-  HOST_TRY(t2_alloc(ctx, &coords, (size_t)n * 4));
-  HOST_TRY(t2_alloc(ctx, &nbr, (size_t)n * 27));
-  HOST_TRY(t2_alloc(ctx, &gray, (size_t)n));
-  HOST_TRY(t2_alloc(ctx, &x, (size_t)n * Ci * es));
-  HOST_TRY(t2_alloc(ctx, &w, (size_t)Co * 27 * Ci * es));
-  HOST_TRY(t2_alloc(ctx, &y, (size_t)n * Co * es));
-  HOST_TRY(cudaMemcpyAsync(coords, coords_host, (size_t)n * 16, cudaMemcpyHostToDevice, ctx->stream));
-  HOST_TRY(cudaMemcpyAsync(x, x_host, (size_t)n * Ci * es, cudaMemcpyHostToDevice, ctx->stream));
-  HOST_TRY(cudaMemcpyAsync(w, w_host, (size_t)Co * 27 * Ci * es, cudaMemcpyHostToDevice, ctx->stream));
-  if (bias_host) {
-    HOST_TRY(t2_alloc(ctx, &b, (size_t)Co * es));
-    HOST_TRY(cudaMemcpyAsync(b, bias_host, (size_t)Co * es, cudaMemcpyHostToDevice, ctx->stream));
+  T2_REQ(ctx, Ci > 0 && Co > 0, "spconv shapes Ci=%d Co=%d", Ci, Co);
+  const size_t es = dtype_size(dtype), xrow = (size_t)Ci * es, yrow = (size_t)Co * es, wbytes = (size_t)Co * 27 * xrow;
+  T2_CUDA(ctx, cudaSetDevice(ctx->device));
+  constexpr size_t CHUNK = 4u << 20;
+  const size_t lesser = (size_t)n * (xrow < yrow ? xrow : yrow);
+  int chunks = (int)(lesser / CHUNK < 8 ? lesser / CHUNK : 8);
+  void* y_mapped = nullptr;
+  if (chunks < 2 || yrow % 16 || !pinned_address(x_host) || !(y_mapped = pinned_address(y_host)) || (uintptr_t)y_mapped % 16) chunks = 1;
+  const i64 chunk_rows = (n + chunks - 1) / chunks;
+  chunks = (int)((n + chunk_rows - 1) / chunk_rows);
+  HostCall c(ctx);
+  T2_CUDA(ctx, t2_alloc(ctx, &c.coords, (size_t)n * 4));
+  T2_CUDA(ctx, t2_alloc(ctx, &c.nbr, (size_t)n * 27));
+  T2_CUDA(ctx, t2_alloc(ctx, &c.gray, (size_t)n));
+  T2_CUDA(ctx, t2_alloc(ctx, &c.x, (size_t)n * xrow));
+  T2_CUDA(ctx, t2_alloc(ctx, &c.w, wbytes));
+  T2_CUDA(ctx, t2_alloc(ctx, &c.y, (size_t)n * yrow));
+  if (bias_host) T2_CUDA(ctx, t2_alloc(ctx, &c.b, yrow));
+  t2sc_epilogue ep; memset(&ep, 0, sizeof(ep)); ep.bias = c.b;
+  int rc;
+  if (chunks < 2) {
+    T2_CUDA(ctx, cudaMemcpyAsync(c.coords, coords_host, (size_t)n * 16, cudaMemcpyHostToDevice, ctx->stream));
+    T2_CUDA(ctx, cudaMemcpyAsync(c.x, x_host, (size_t)n * xrow, cudaMemcpyHostToDevice, ctx->stream));
+    T2_CUDA(ctx, cudaMemcpyAsync(c.w, w_host, wbytes, cudaMemcpyHostToDevice, ctx->stream));
+    if (bias_host) T2_CUDA(ctx, cudaMemcpyAsync(c.b, bias_host, yrow, cudaMemcpyHostToDevice, ctx->stream));
+    if ((rc = t2sc_build_neighbors(ctx, c.coords, n, W, H, D, c.nbr, c.gray, nullptr)) != T2SC_OK) return rc;
+    if ((rc = t2sc_plan_create(ctx, c.nbr, c.gray, n, nullptr, n, 0, 0, &c.plan)) != T2SC_OK) return rc;
+    if ((rc = t2sc_subm_conv(ctx, c.plan, c.x, c.w, &ep, c.y, dtype, n, Ci, Co, T2SC_VARIANT_AUTO)) != T2SC_OK) return rc;
+    T2_CUDA(ctx, cudaMemcpyAsync(y_host, c.y, (size_t)n * yrow, cudaMemcpyDeviceToHost, ctx->stream));
+  } else {
+    T2_CUDA(ctx, side_streams(ctx));
+    T2_CUDA(ctx, t2_alloc(ctx, &c.late, (size_t)n + 1));           // [n] is their number
+    cudaEvent_t *in = ctx->ev, *out = ctx->ev + 8, ev_coords = ctx->ev[16], ev_weights = ctx->ev[17], ev_start = ctx->ev[18], ev_end = ctx->ev[19];
+    T2_CUDA(ctx, cudaMemsetAsync(c.late + n, 0, sizeof(int), ctx->stream));
+    T2_CUDA(ctx, cudaEventRecord(ev_start, ctx->stream));          // the buffers exist from here on
+    c.side = true;
+    T2_CUDA(ctx, cudaStreamWaitEvent(ctx->copy_in, ev_start, 0));
+    T2_CUDA(ctx, cudaMemcpyAsync(c.coords, coords_host, (size_t)n * 16, cudaMemcpyHostToDevice, ctx->copy_in));
+    T2_CUDA(ctx, cudaEventRecord(ev_coords, ctx->copy_in));
+    T2_CUDA(ctx, cudaMemcpyAsync(c.w, w_host, wbytes, cudaMemcpyHostToDevice, ctx->copy_in));
+    if (bias_host) T2_CUDA(ctx, cudaMemcpyAsync(c.b, bias_host, yrow, cudaMemcpyHostToDevice, ctx->copy_in));
+    T2_CUDA(ctx, cudaEventRecord(ev_weights, ctx->copy_in));
+    for (int q = 0; q < chunks; q++) {
+      const i64 lo = q * chunk_rows, hi = lo + chunk_rows < n ? lo + chunk_rows : n;
+      T2_CUDA(ctx, cudaMemcpyAsync(c.x + lo * xrow, (const char*)x_host + lo * xrow, (size_t)(hi - lo) * xrow, cudaMemcpyHostToDevice, ctx->copy_in));
+      T2_CUDA(ctx, cudaEventRecord(in[q], ctx->copy_in));
+    }
+    T2_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ev_coords, 0));
+    if ((rc = t2sc_build_neighbors(ctx, c.coords, n, W, H, D, c.nbr, c.gray, nullptr)) != T2SC_OK) return rc;
+    if ((rc = plan_create_chunked(ctx, c.nbr, c.gray, n, chunk_rows, c.late, c.late + n, &c.plan)) != T2SC_OK) return rc;
+    // how many rows come late, while the features are still on their way
+    T2_CUDA(ctx, cudaMemcpyAsync(ctx->pinned, c.late + n, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    T2_CUDA(ctx, ctx_wait(ctx));
+    const int n_late = ctx->pinned[0];
+    const bool stream_out = n_late <= n / 8;
+    T2_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ev_weights, 0));
+    for (int q = 0; q < chunks; q++) {
+      const i64 lo = q * chunk_rows, hi = lo + chunk_rows < n ? lo + chunk_rows : n;
+      T2_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, in[q], 0));
+      if ((rc = conv_dispatch(ctx, c.plan, c.x, c.w, &ep, c.y, dtype, n, Ci, Co, T2SC_VARIANT_AUTO, PART_GROUP0 + q)) != T2SC_OK) return rc;
+      if (!stream_out) continue;
+      T2_CUDA(ctx, cudaEventRecord(out[q], ctx->stream));
+      T2_CUDA(ctx, cudaStreamWaitEvent(ctx->copy_out, out[q], 0));
+      T2_CUDA(ctx, cudaMemcpyAsync((char*)y_host + lo * yrow, c.y + lo * yrow, (size_t)(hi - lo) * yrow, cudaMemcpyDeviceToHost, ctx->copy_out));
+    }
+    if (!stream_out) {
+      T2_CUDA(ctx, cudaMemcpyAsync(y_host, c.y, (size_t)n * yrow, cudaMemcpyDeviceToHost, ctx->stream));
+    } else {
+      if (n_late) {
+        k_rows_out<<<cdiv_i((i64)n_late * 32, 256), 256, 0, ctx->copy_out>>>((const uint4*)c.y, c.late, n_late, (int)(yrow / 16), (uint4*)y_mapped);
+        T2_LAUNCHED(ctx);
+      }
+      T2_CUDA(ctx, cudaEventRecord(ev_end, ctx->copy_out));
+      T2_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ev_end, 0));
+    }
   }
-  if ((rc = t2sc_build_neighbors(ctx, coords, n, W, H, D, nbr, gray, nullptr)) != T2SC_OK) { cleanup(); return rc; }
-  if ((rc = t2sc_plan_create(ctx, nbr, gray, n, nullptr, n, 0, 0, &plan)) != T2SC_OK) { cleanup(); return rc; }
-  t2sc_epilogue ep; memset(&ep, 0, sizeof(ep)); ep.bias = b;
-  if ((rc = t2sc_subm_conv(ctx, plan, x, w, &ep, y, dtype, n, Ci, Co, T2SC_VARIANT_AUTO)) != T2SC_OK) { cleanup(); return rc; }
-  HOST_TRY(cudaMemcpyAsync(y_host, y, (size_t)n * Co * es, cudaMemcpyDeviceToHost, ctx->stream));
-  HOST_TRY(ctx_wait(ctx));
-#undef HOST_TRY
-  cleanup();
+  T2_CUDA(ctx, cudaMemcpyAsync(ctx->pinned + 2, ctx->status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+  T2_CUDA(ctx, ctx_wait(ctx));
+  if (!ctx->pinned[2]) return T2SC_OK;
   int st = 0;
   return t2sc_device_status(ctx, &st);
 }

@@ -23,6 +23,8 @@ struct t2sc_ctx {
   size_t arena_bytes = 0, arena_want = 0;
   int* status = nullptr;        // device word; kernels OR an error code into it when a bounded wait gives up
   int* pinned = nullptr;        // 64 bytes of pinned host memory: where small results are read back to
+  cudaStream_t copy_in = nullptr, copy_out = nullptr;   // of the host-buffer call, made on its first large use
+  cudaEvent_t ev[20] = {nullptr};                       // its events: 8 chunks in, 8 groups done, coords, weights, start, end
   cudaEvent_t done = nullptr;   // event the host polls when it waits for the stream (see ctx_wait in api.cu)
   char err[1024] = {0};
 };
@@ -45,9 +47,10 @@ struct t2sc_plan {
   int* perm = nullptr;          // [max_tiles]: positions -> tile numbers, each part's tiles by falling tap count: the order the
                                 // tcgen05 kernel's CTAs take them in, so that every SM gets long and short tiles alike
   bool balanced = false;        // perm is filled (maps sorted as one block); large maps keep plan order for L2 locality
-  int* meta = nullptr;          // device [16]: group counts, bounds, stats (one allocation, one memset)
+  int* meta = nullptr;          // device: group counts, bounds, stats, group bounds (one allocation, one memset)
   int* bounds = nullptr;        // = meta + 8, device [3]: {0, first boundary tile, realised tile count}; parts are [b0,b1) and [b1,b2)
   int* ntiles = nullptr;        // = bounds + 2: realised tile count (<= max_tiles)
+  int* group_tiles = nullptr;   // = meta + 16, device [9]: first tile of every group and the tile count (chunked plans)
   bool split = false;           // made by t2sc_plan_create_split: interior tiles first, boundary tiles last
   unsigned long long* stats = nullptr;  // device: pairs of computed taps, active taps, to be added up
   i64 max_tiles = 0;
@@ -149,11 +152,20 @@ int plan_table_prepare(t2sc_ctx* ctx, t2sc_plan* plan, i64 n_in);      // plan.c
 // implemented in the kernel files
 // which tiles of a plan a launch covers: pointers to the first tile index and to the index one past the last
 struct TilePart { const int* lo; const int* hi; };
+constexpr int PART_GROUP0 = 16;
 static inline TilePart tile_part(const t2sc_plan* p, int part) {
   if (part == T2SC_PART_INTERIOR) return TilePart{p->bounds, p->bounds + 1};
   if (part == T2SC_PART_BOUNDARY) return TilePart{p->bounds + 1, p->bounds + 2};
+  if (part >= PART_GROUP0) return TilePart{p->group_tiles + (part - PART_GROUP0), p->group_tiles + (part - PART_GROUP0) + 1};
   return TilePart{p->bounds, p->bounds + 2};
 }
+// A plan whose rows are grouped by the last chunk of `chunk_rows` feature rows that any of their taps reads (at most 8 chunks): group
+// q's tiles (part PART_GROUP0 + q) can run once chunks 0..q have arrived.  late[] (room for n) receives the rows whose group
+// lies behind their own chunk, *n_late their number (zeroed by the caller).
+int plan_create_chunked(t2sc_ctx* ctx, const uint32_t* nbr, const int32_t* gray, i64 n, i64 chunk_rows, int* late, int* n_late, t2sc_plan** out);
+// t2sc_subm_conv_part for any part, PART_GROUP0 + q included
+int conv_dispatch(t2sc_ctx* ctx, t2sc_plan* plan, const void* x, const void* w, const t2sc_epilogue* ep, void* y, int dtype, int64_t n_in,
+                  int Ci, int Co, int variant, int part);
 int conv_simt_launch(t2sc_ctx* ctx, const t2sc_plan* plan, const void* x, const void* w, const EpiDev& ep, void* y,
                      int dtype, i64 n_in, int Ci, int Co, int part = T2SC_PART_ALL);
 int conv_f32_launch(t2sc_ctx* ctx, const t2sc_plan* plan, const float* x, const float* w, const EpiDev& ep, float* y, i64 n_in, int Ci, int Co,

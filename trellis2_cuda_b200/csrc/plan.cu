@@ -33,14 +33,15 @@ __device__ __forceinline__ uint32_t mask_key(uint32_t g) {
 // key = group | block (block_bits wide) | mask key (27 bits), most significant first, with the `drop` least significant
 // mask-key bits left out; K is uint32_t when that fits in 32 bits (half the sort traffic), else unsigned long long.
 // halo_from > 0 (split plan, no src): group 1 = rows with a map entry >= halo_from (a row of a peer), group 0 = the rest
+// chunk_rows > 0 (no src): group = chunk of the largest map entry; rows whose group lies behind their own chunk go to late[]
 template <class K>
 __global__ void k_plan_keys(const int* __restrict__ gray, const int* __restrict__ src, const uint32_t* __restrict__ nbr, uint32_t halo_from,
-                            i64 m, uint32_t block_rows, int block_bits, int drop,
+                            uint32_t chunk_rows, int* __restrict__ late, int* __restrict__ n_late, i64 m, uint32_t block_rows, int block_bits, int drop,
                             K* __restrict__ keys, int* __restrict__ iota, int* __restrict__ group_cnt) {
   // group sizes: counted per CTA in shared memory first (millions of rows on eight counters in global memory were the
   // whole time of this kernel)
   __shared__ int s_cnt[8];
-  const bool grouped = src || halo_from;
+  const bool grouped = src || halo_from || chunk_rows;
   if (grouped && threadIdx.x < 8) s_cnt[threadIdx.x] = 0;
   if (grouped) __syncthreads();
   i64 i = blockIdx.x * (i64)blockDim.x + threadIdx.x;
@@ -51,6 +52,14 @@ __global__ void k_plan_keys(const int* __restrict__ gray, const int* __restrict_
       const uint32_t* e = nbr + i * 27;
 #pragma unroll 9
       for (int v = 0; v < 27; v++) { const uint32_t r = __ldg(e + v); grp |= (r != NBR_EMPTY && r >= halo_from) ? 1 : 0; }
+    }
+    else if (chunk_rows) {
+      const uint32_t* e = nbr + i * 27;
+      uint32_t last = 0;
+#pragma unroll 9
+      for (int v = 0; v < 27; v++) { const uint32_t r = __ldg(e + v); if (r != NBR_EMPTY) last = max(last, r); }
+      grp = (int)(min(last, (uint32_t)(m - 1)) / chunk_rows);
+      if (grp > (int)((uint32_t)i / chunk_rows)) late[atomicAdd(n_late, 1)] = (int)i;
     }
     const unsigned long long blk = (uint32_t)i / block_rows;          // rows are below 2^30: no 64-bit division
     const unsigned long long k = ((unsigned long long)grp << (27 + block_bits)) | (blk << 27) | mask_key((uint32_t)gray[nrow]);
@@ -76,7 +85,7 @@ constexpr int META_SLOTS = 32, META_MAX = 32, META_STATS = META_MAX + META_SLOTS
 template <int TILE, bool HEADER>
 __global__ void __launch_bounds__(256) k_plan_tiles_table(const uint32_t* __restrict__ nbr, const int* __restrict__ gray, const int* __restrict__ src,
                                                           const int* __restrict__ order, const int* __restrict__ group_cnt, int ngroups, int split,
-                                                          i64 m, PlanTile* __restrict__ tiles, int* __restrict__ bounds,
+                                                          i64 m, PlanTile* __restrict__ tiles, int* __restrict__ bounds, int* __restrict__ group_tiles, bool slots,
                                                           unsigned long long* __restrict__ stats, uint32_t* __restrict__ table,
                                                           uint32_t* __restrict__ max_entry, int* __restrict__ hist, int win) {
   const int t = blockIdx.x;
@@ -93,16 +102,17 @@ __global__ void __launch_bounds__(256) k_plan_tiles_table(const uint32_t* __rest
       const int c = ngroups == 1 ? (int)m : group_cnt[q];
       const int nt = (c + TILE - 1) / TILE;
       if (q == 1) first_boundary = tl;
+      if (t == 0 && threadIdx.x == 0) group_tiles[q] = tl;
       if (!mine && t < tl + nt) { mine = true; g = q; start = row + (t - tl) * TILE; rows = min(TILE, row + c - start); }
       row += c; tl += nt;
     }
-    if (t == 0 && threadIdx.x == 0) { bounds[0] = 0; bounds[1] = split ? first_boundary : tl; bounds[2] = tl; }
+    if (t == 0 && threadIdx.x == 0) { group_tiles[ngroups] = tl; bounds[0] = 0; bounds[1] = split ? first_boundary : tl; bounds[2] = tl; }
     if (!mine) return;
     if (threadIdx.x == 0) {       // this tile's bin row in the tap-count histogram: (window of `win` tiles within its part, part)
       const int part = (split && g >= 1) ? 1 : 0;
       s_or = 0; s_act = 0; s_part = (((t - (part ? first_boundary : 0)) / win) * 2 + part) * 32;
     }
-    tile = PlanTile{start, rows, split ? 0 : g, 0};      // wbase holds the child slot (the conv multiplies by Co); the two parts of a split plan share one weight set
+    tile = PlanTile{start, rows, slots ? g : 0, 0};      // wbase holds the child slot (the conv multiplies by Co); groups of any other kind share one weight set
   } else {
     if (t >= bounds[2]) return;
     tile = tiles[t];
@@ -202,10 +212,10 @@ int plan_tiles_table(t2sc_ctx* ctx, t2sc_plan* p, const int32_t* gray, const int
   if (p->n_out == 0) return T2SC_OK;
   if (p->tile_rows == 128)
     k_plan_tiles_table<128, HEADER><<<(unsigned)p->max_tiles, 256, 0, ctx->stream>>>(p->nbr, gray, p->src, p->order, gcnt, ngroups, p->split ? 1 : 0, p->n_out,
-                                                                                       p->tiles, p->bounds, p->stats, p->tnbr, (uint32_t*)(p->meta + META_MAX), hist, win);
+                                                                                       p->tiles, p->bounds, p->group_tiles, p->src != nullptr, p->stats, p->tnbr, (uint32_t*)(p->meta + META_MAX), hist, win);
   else
     k_plan_tiles_table<256, HEADER><<<(unsigned)p->max_tiles, 256, 0, ctx->stream>>>(p->nbr, gray, p->src, p->order, gcnt, ngroups, p->split ? 1 : 0, p->n_out,
-                                                                                       p->tiles, p->bounds, p->stats, p->tnbr, (uint32_t*)(p->meta + META_MAX), hist, win);
+                                                                                       p->tiles, p->bounds, p->group_tiles, p->src != nullptr, p->stats, p->tnbr, (uint32_t*)(p->meta + META_MAX), hist, win);
   T2_LAUNCHED(ctx);
   if (HEADER && hist) {
     const i64 bins = (cdiv_i(p->max_tiles, win) + 1) * 64;
@@ -237,7 +247,8 @@ extern "C" int t2sc_plan_check(t2sc_ctx* ctx, t2sc_plan* p, int64_t n_in) {
 }
 
 static int plan_create(t2sc_ctx* ctx, const uint32_t* nbr, const int32_t* gray, int64_t n_rows,
-                       const int32_t* src, int64_t m, int64_t halo_from, int64_t block_rows, int tile_rows, t2sc_plan** out) {
+                       const int32_t* src, int64_t m, int64_t halo_from, int64_t block_rows, int tile_rows, t2sc_plan** out,
+                       i64 chunk_rows = 0, int* late = nullptr, int* n_late = nullptr) {
   T2_REQ(ctx, ctx && out, "null context or out");
   *out = nullptr;
   T2_REQ(ctx, n_rows >= 0 && m >= 0 && m < (1ll << 30) && n_rows < (1ll << 30), "n_rows=%lld m=%lld", (long long)n_rows, (long long)m);
@@ -254,7 +265,9 @@ static int plan_create(t2sc_ctx* ctx, const uint32_t* nbr, const int32_t* gray, 
   const int split = halo_from > 0 ? 1 : 0;
   p->split = split != 0;
   int ngroups = src ? 8 : (split ? 2 : 1);
-  p->max_tiles = cdiv_i(m, TILE) + (src ? 8 : (split ? 2 : 0));
+  if (chunk_rows > 0) ngroups = cdiv_i(m, chunk_rows);
+  const int group_bits = ngroups > 2 ? 3 : (ngroups > 1 ? 1 : 0);
+  p->max_tiles = cdiv_i(m, TILE) + (ngroups > 1 ? ngroups : 0);
   Scratch scratch(ctx);            // sort buffers: back to the pool on every path out
   auto fail = [&](cudaError_t e) {
     t2sc_plan_destroy(ctx, p);
@@ -266,9 +279,10 @@ static int plan_create(t2sc_ctx* ctx, const uint32_t* nbr, const int32_t* gray, 
   PL(t2_alloc(ctx, &p->tiles, (size_t)p->max_tiles));
   PL(t2_alloc(ctx, &p->perm, (size_t)p->max_tiles));
   PL(t2_alloc(ctx, &p->tnbr, (size_t)p->max_tiles * 27 * tile_rows));
-  // one small block, one memset: group counts [0..8), part bounds [8..11), largest map entry and
+  // one small block, one memset: group counts [0..8), part bounds [8..11), first tile of every group [16..25), largest map entry and
   // tap statistics in META_SLOTS words each
   PL(t2_alloc(ctx, &p->meta, META_INTS));
+  p->group_tiles = p->meta + 16;
   p->bounds = p->meta + 8; p->ntiles = p->bounds + 2; p->stats = (unsigned long long*)(p->meta + META_STATS);
   PL(cudaMemsetAsync(p->meta, 0, META_INTS * sizeof(int), ctx->stream));
   if (m > 0) {
@@ -278,8 +292,8 @@ static int plan_create(t2sc_ctx* ctx, const uint32_t* nbr, const int32_t* gray, 
     // (active/computed 0.855 -> 0.853) and leaving them out saves a radix pass on maps sorted as one block
     // Up to five more go when that brings the key down to 32 bits (a large subdivision plan: 3 group bits + 6 block bits).
     int drop = 3;
-    while (27 + block_bits + (src ? 3 : (split ? 1 : 0)) - drop > 32 && drop < 8) drop++;
-    const int key_bits = 27 + block_bits + (src ? 3 : (split ? 1 : 0)) - drop;
+    while (27 + block_bits + group_bits - drop > 32 && drop < 8) drop++;
+    const int key_bits = 27 + block_bits + group_bits - drop;
     const bool narrow = key_bits <= 32;
     const size_t ksz = narrow ? sizeof(uint32_t) : sizeof(unsigned long long);
     char* buf = nullptr; char* tmp = nullptr; size_t tb = 0;
@@ -288,14 +302,14 @@ static int plan_create(t2sc_ctx* ctx, const uint32_t* nbr, const int32_t* gray, 
     int* iota = (int*)(buf + 2 * koff);
     if (narrow) {
       uint32_t *keys = (uint32_t*)buf, *keys2 = (uint32_t*)(buf + koff);
-      k_plan_keys<uint32_t><<<cdiv_i(m, 256), 256, 0, ctx->stream>>>(gray, src, nbr, (uint32_t)halo_from, m, (uint32_t)(block_rows < m ? block_rows : m), block_bits, drop, keys, iota, p->meta);
+      k_plan_keys<uint32_t><<<cdiv_i(m, 256), 256, 0, ctx->stream>>>(gray, src, nbr, (uint32_t)halo_from, (uint32_t)chunk_rows, late, n_late, m, (uint32_t)(block_rows < m ? block_rows : m), block_bits, drop, keys, iota, p->meta);
       ctx->launches++; PL(cudaGetLastError());
       PL(cub::DeviceRadixSort::SortPairs(nullptr, tb, keys, keys2, iota, p->order, (int)m, 0, key_bits, ctx->stream));
       PL(scratch.get(&tmp, tb));
       PL(cub::DeviceRadixSort::SortPairs(tmp, tb, keys, keys2, iota, p->order, (int)m, 0, key_bits, ctx->stream));
     } else {
       unsigned long long *keys = (unsigned long long*)buf, *keys2 = (unsigned long long*)(buf + koff);
-      k_plan_keys<unsigned long long><<<cdiv_i(m, 256), 256, 0, ctx->stream>>>(gray, src, nbr, (uint32_t)halo_from, m, (uint32_t)(block_rows < m ? block_rows : m), block_bits, drop, keys, iota, p->meta);
+      k_plan_keys<unsigned long long><<<cdiv_i(m, 256), 256, 0, ctx->stream>>>(gray, src, nbr, (uint32_t)halo_from, (uint32_t)chunk_rows, late, n_late, m, (uint32_t)(block_rows < m ? block_rows : m), block_bits, drop, keys, iota, p->meta);
       ctx->launches++; PL(cudaGetLastError());
       PL(cub::DeviceRadixSort::SortPairs(nullptr, tb, keys, keys2, iota, p->order, (int)m, 0, key_bits, ctx->stream));
       PL(scratch.get(&tmp, tb));
@@ -303,7 +317,7 @@ static int plan_create(t2sc_ctx* ctx, const uint32_t* nbr, const int32_t* gray, 
     }
     // The order the conv's CTAs take the tiles in (k_plan_perm): by tap count when the rows were sorted as one block; plan
     // order when they were sorted inside runs (large maps: the runs keep concurrently running tiles L2-local).
-    p->balanced = block_rows >= m;
+    p->balanced = block_rows >= m && chunk_rows == 0;        // (k_plan_perm knows two parts)
     const int win = 1 << 30;
     const i64 bins = 2 * 64;
     int* hist = nullptr;
@@ -316,6 +330,11 @@ static int plan_create(t2sc_ctx* ctx, const uint32_t* nbr, const int32_t* gray, 
 #undef PL
   *out = p;
   return T2SC_OK;
+}
+
+int plan_create_chunked(t2sc_ctx* ctx, const uint32_t* nbr, const int32_t* gray, i64 n, i64 chunk_rows, int* late, int* n_late, t2sc_plan** out) {
+  T2_REQ(ctx, n > 0 && chunk_rows > 0 && cdiv_i(n, chunk_rows) <= 8, "n=%lld chunk_rows=%lld", (long long)n, (long long)chunk_rows);
+  return plan_create(ctx, nbr, gray, n, nullptr, n, 0, 0, 0, out, chunk_rows, late, n_late);
 }
 
 extern "C" int t2sc_plan_create(t2sc_ctx* ctx, const uint32_t* nbr, const int32_t* gray, int64_t n_rows,
