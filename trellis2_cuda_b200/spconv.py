@@ -433,11 +433,14 @@ class Level:
                 and self.parent._tile_rows_for(256, x.shape[1]) == 128 and self.src.shape[0] > 2.7 * self.parent.N)
 
     def up_plan_for(self, Cc: int, Ci: int = 64) -> _Plan:
-        """Schedule of the subdivision conv into Cc child channels: 256-row tiles, two 128-row accumulators per weight slab
-        (the 8 child slots have 8 weight sets, so a slab is reused by fewer rows than in a submanifold conv; measured on
-        886,752 parents -> 3,288,465 children, 128 -> 64: 2.35 ms against 2.80 ms with 128-row tiles).  128-row tiles for input
-        rows that end in half a chunk, which have that form only."""
-        tr = 256 if Ci % 64 == 0 else 128
+        """Schedule of the subdivision conv into Cc child channels.  256-row tiles, two 128-row accumulators per weight slab, where
+        a slab is narrow and tiles are many: the 8 child slots have 8 weight sets, so a slab is reused by fewer rows than in a
+        submanifold conv (886,752 parents, 128 -> 64: 2.35 ms against 2.80 with 128-row tiles; 150,000, 256 -> 128: whole up block
+        1.81 against 1.87).  128-row tiles at 256 columns, where two halves leave no room for a second accumulator, and
+        below four 256-row tiles per SM, where their finer masks and shorter items fill the chip (whole up block: 1,500
+        parents, 1024 -> 512: 664 -> 450 us; 12,000: 1718 -> 1495; 8,000, 512 -> 256: 611 -> 525; 30,000, 256 -> 128: 607 ->
+        588), and for input rows that end in half a chunk, which have that form only."""
+        tr = 256 if Ci % 64 == 0 and Cc % 256 and self.src.shape[0] >= 4 * 256 * 148 else 128
         if self._up_plans is None:
             self._up_plans = {}
         if tr not in self._up_plans:
