@@ -306,12 +306,18 @@ static int plan_create(t2sc_ctx* ctx, const uint32_t* nbr, const int32_t* gray, 
   if (m > 0) {
     int block_bits = 0;
     while (((m + block_rows - 1) / block_rows) > (1ll << block_bits)) block_bits++;
-    // the 3 least significant key bits (centre tap and two face taps) do not change the tiles' masks measurably
-    // (active/computed 0.855 -> 0.853) and leaving them out saves a radix pass on maps sorted as one block
-    // Up to five more go when that brings the key down to 32 bits (a large subdivision plan: 3 group bits + 6 block bits).
-    int drop = 3;
-    while (27 + block_bits + group_bits - drop > 32 && drop < 8) drop++;
-    if (tap_groups) drop = 0;
+    // How many leading bits of the mask key the sort looks at.  Rows that are sorted together need the more of them the more they
+    // are: at 24 bits (without the centre tap and two face taps) against 20, 18, 16 and 14 the active / computed taps of shells are, on
+    // 14,534 rows, 0.665 / 0.665 / 0.665 / 0.665 / 0.665; on 30,011, 0.717 / 0.717 / 0.718 / 0.717 / 0.716; on 100,000, 0.796 /
+    // 0.796 / 0.791 / 0.786 / 0.780; on 217,821, 0.853 / 0.850 / 0.842 / 0.831 / 0.819.  A pass of the sort takes 8 bits and 11 us
+    // (36 us on 3,288,465 rows), so the bits needed are rounded up to whole passes and no further.
+    int drop = 0;
+    if (!tap_groups) {
+      const i64 together = (block_rows < m ? block_rows : m) / ngroups;
+      const int need = together <= 16384 ? 13 : together <= 49152 ? 16 : together <= 65536 ? 18 : 24;
+      const int bits = (block_bits + group_bits + need + 7) / 8 * 8 - block_bits - group_bits;
+      drop = bits < 24 ? 27 - bits : 3;
+    }
     const int key_bits = tap_groups ? 2 + TAP_GROUP_TAPS : 27 + block_bits + group_bits - drop;
     const bool narrow = key_bits <= 32;
     const size_t ksz = narrow ? sizeof(uint32_t) : sizeof(unsigned long long);
