@@ -38,9 +38,9 @@ using namespace umma;
 // Warp roles: 0-3 gather A (cp.async), 4 weights (TMA), 5 and the last warp of the base set fill the neighbour-index table,
 // 6 MMA issue + TMEM owner, 7.. epilogue (4 warps per 128-row half).
 // A unit is one (tap, 64-channel chunk): 16 KB of gathered rows per 128-row half, one weight slab, four MMAs per half.
-// One pipeline stage holds U consecutive units of a tile.  Every role pays one barrier round trip per STAGE (a wait
-// that answers after ~100 clocks, an arrival or commit), in order, whatever the stage holds; with one unit per stage
-// that is ~400 clocks per unit against 64 to 256 clocks of tensor time at Co <= 128, so narrow layers take U = 2 or 4.
+// A pipeline stage holds one unit.  Every role pays a barrier round trip per unit (a wait that answers after ~100 clocks, an
+// arrival or commit), in order: ~400 clocks against 64 to 256 clocks of tensor time at Co <= 128, so narrow tiles run with OCC = 2
+// CTAs per SM, whose roles fill each other's gaps.
 // G = gather groups of four warps.  G = 1: the four gather warps fill every stage together.  G = 2 (128-row tiles):
 // a second group of four warps sits behind the epilogue warps and the groups fill alternate stages, so one group's
 // barrier round trips and index reads overlap the other group's copies.
@@ -56,15 +56,15 @@ using namespace umma;
 //
 // CHILD > 0 (subdivision conv from the parents' tiles): the BN columns are BN / CHILD child slots of CHILD channels; the epilogue
 // treats each as a row of its own, of the child that sits there, and skips slots that are not kept.
-template <int BN, int MH, int G, int U, bool PEERS, bool TAIL, int CHILD, class T>
-__global__ void __launch_bounds__(num_threads(MH, G), 1) k_conv_umma(const __grid_constant__ CUtensorMap tmw, const ConvArgs a) {
+template <int BN, int MH, int G, bool PEERS, bool TAIL, int CHILD, int OCC, class T>
+__global__ void __launch_bounds__(num_threads(MH, G), OCC) k_conv_umma(const __grid_constant__ CUtensorMap tmw, const ConvArgs a) {
   static_assert(!TAIL || (MH == 1 && !PEERS), "half chunks run on 128-row tiles of local rows");
   static_assert(G == 1 || (G == 2 && MH == 1), "a second gather group only fits beside 128-row tiles");
-  constexpr int UNIT = stage_bytes(BN, MH);          // MH gathered A halves + one weight slab
-  constexpr int STAGE = U * UNIT;
-  constexpr int S = num_stages(BN, MH, U);
+  constexpr int STAGE = stage_bytes(BN, MH);          // one unit: MH gathered A halves + one weight slab
+  constexpr int S = num_stages(BN, MH, PEERS, OCC);
+  constexpr int NTAB = num_tabs(OCC);
   constexpr int B_BYTES = BN * 128;
-  constexpr int NB = num_acc_bufs(BN, MH);            // accumulator buffers, each MH halves of BN columns
+  constexpr int NB = num_acc_bufs(BN, MH, OCC);            // accumulator buffers, each MH halves of BN columns
   constexpr int TMEM_COLS = tmem_cols(NB * MH * BN);
   constexpr int ROWS = MH * TILE_M;
   constexpr int PITCH = PEERS ? tab_pitch(MH) : ROWS;  // the index warps write a map row per instruction: an odd pitch keeps that conflict-free
@@ -81,9 +81,9 @@ __global__ void __launch_bounds__(num_threads(MH, G), 1) k_conv_umma(const __gri
   uint32_t* tab_remote = (uint32_t*)(peer_base + 8);           // PEERS: [NTAB][2 index warps][32 taps] does the tap read any row of a peer?
   uint32_t* peer_rows = tab_remote + NTAB * 64;                // PEERS: rows of every peer's array (bounds of the map entries)
   // epilogue staging: LayerNorm gamma / beta of the row, and per epilogue warp the bias values of its current item
-  uint8_t* epi_s = (uint8_t*)(((uintptr_t)(smem + S * STAGE + aux_bytes(MH) - epi_bytes(MH)) + 15) & ~(uintptr_t)15);
-  float* gamma_s = (float*)epi_s; float* beta_s = gamma_s + 256;
-  T* bias_s = (T*)(beta_s + 256);                              // [4 * MH epilogue warps][256]
+  uint8_t* epi_s = (uint8_t*)(((uintptr_t)(smem + S * STAGE + aux_bytes(BN, MH, PEERS, OCC) - epi_bytes(BN, MH)) + 15) & ~(uintptr_t)15);
+  float* gamma_s = (float*)epi_s; float* beta_s = gamma_s + BN;
+  T* bias_s = (T*)(beta_s + BN);                               // [4 * MH epilogue warps][BN]
 
   const uint32_t smem_base = smem_u32(smem);
   const uint32_t bar_full = smem_u32(bars), bar_empty = bar_full + 8 * S, bar_accf = bar_empty + 8 * S, bar_acce = bar_accf + 16,
@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(num_threads(MH, G), 1) k_conv_umma(const __gri
     for (int s = 0; s < S; s++) { mbar_init(bar_full + 8 * s, NUM_PROD_THREADS + 1); mbar_init(bar_empty + 8 * s, 1); }
     for (int b = 0; b < 2; b++) { mbar_init(bar_accf + 8 * b, 1); mbar_init(bar_acce + 8 * b, 128 * MH); }
     for (int r = 0; r < NTAB; r++) { mbar_init(bar_tready + 8 * r, PEERS ? 2 : 1); mbar_init(bar_tfree + 8 * r, NGW); }   // two index warps (or the one loader lane) fill, every gather warp releases
-    for (int r = 0; r < NTAB * 64; r++) tab_remote[r] = 0;
+    if (PEERS) for (int r = 0; r < NTAB * 64; r++) tab_remote[r] = 0;
     abort_flag[0] = 0; abort_flag[1] = a.wait_limit;
     if (PEERS) for (int r = 0; r < 8; r++) { peer_base[r] = a.xp[r]; peer_rows[r] = a.xp_rows[r]; }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -167,65 +167,60 @@ __global__ void __launch_bounds__(num_threads(MH, G), 1) k_conv_umma(const __gri
       uint32_t idx[8 * MH], sz[8 * MH];       // rows jbase + 16 i; rows 128.. are the second half, stored right behind the first
       const T* rp[PEERS ? 8 * MH : 1];
       bool remote = false;
-      for (int u0 = 0; u0 < nunits; u0 += U, it++) {
-        const int nu = nunits - u0 < U ? nunits - u0 : U;      // a tile's last stage may be short
+      for (int u = 0; u < nunits; u++, it++) {
         // G == 2: the groups alternate stages.  A group waits on stages two apart, never more than the stage count apart,
         // so it cannot run two phases ahead of a stage, where a parity wait would pass by mistake.
         if (G == 2 && (int)(it & 1) != g) {
-          for (int k = 0; k < nu; k++) if (++c == nchunk) { c = 0; mk &= mk - 1; }
+          if (++c == nchunk) { c = 0; mk &= mk - 1; }
           continue;
         }
         const uint32_t st = it % S;
         alive &= mbar_wait_t(bar_empty + 8 * st, ((it / S) & 1) ^ 1, abort_flag, a.status, 1, prof, w_empty);
         if ((threadIdx.x & 127) == 0) trace(a, 4, 3, it);          // stage-level events (first 64 stages): the gather group holds a free stage
+        const int v = __ffs(mk) - 1;
+        if (v != held_tap) {
+          held_tap = v;
+          // Table entries: row number (PEERS: (owner << PEER_SHIFT) | row), or RING_ABSENT.  Everything that does not
+          // depend on the channel chunk is done here, once per tap, so that a copy costs two instructions (address,
+          // cp.async): the gather warps run these in order.
+          if (dense) {
 #pragma unroll
-        for (int k = 0; k < U; k++) {
-          if (k >= nu) break;
-          const int v = __ffs(mk) - 1;
-          if (v != held_tap) {
-            held_tap = v;
-            // Table entries: row number (PEERS: (owner << PEER_SHIFT) | row), or RING_ABSENT.  Everything that does not
-            // depend on the channel chunk is done here, once per tap, so that a copy costs two instructions (address,
-            // cp.async): the gather warps run these in order.
-            if (dense) {
+            for (int i = 0; i < 8 * MH; i++) idx[i] = jbase + 16 * i < tile.rows ? (uint32_t)(tile.start + jbase + 16 * i) : RING_ABSENT;
+          } else {
 #pragma unroll
-              for (int i = 0; i < 8 * MH; i++) idx[i] = jbase + 16 * i < tile.rows ? (uint32_t)(tile.start + jbase + 16 * i) : RING_ABSENT;
-            } else {
+            for (int i = 0; i < 8 * MH; i++) idx[i] = tab[v * PITCH + 16 * i];
+          }
+          // PEERS: almost every tap reads local rows only (the index warps say so per tap) and takes the plain path with
+          // the owner bits masked off.  For a tap with rows of a peer the addresses are formed here: a table load between
+          // the copies below would be ordered after each of them and serialise the loop.
+          if constexpr (PEERS) {
+            remote = (tab_remote[buf * 64 + v] | tab_remote[buf * 64 + 32 + v]) != 0;
+            if (__builtin_expect(remote, 0)) {
 #pragma unroll
-              for (int i = 0; i < 8 * MH; i++) idx[i] = tab[v * PITCH + 16 * i];
-            }
-            // PEERS: almost every tap reads local rows only (the index warps say so per tap) and takes the plain path with
-            // the owner bits masked off.  For a tap with rows of a peer the addresses are formed here: a table load between
-            // the copies below would be ordered after each of them and serialise the loop.
-            if constexpr (PEERS) {
-              remote = (tab_remote[buf * 64 + v] | tab_remote[buf * 64 + 32 + v]) != 0;
-              if (__builtin_expect(remote, 0)) {
-#pragma unroll
-                for (int i = 0; i < 8 * MH; i++)
-                  rp[i] = idx[i] != RING_ABSENT ? (const T*)peer_base[idx[i] >> PEER_SHIFT] + (i64)(idx[i] & PEER_ROW_MASK) * a.Ci + c16 * 8 : x;
-              }
-            }
-#pragma unroll
-            for (int i = 0; i < 8 * MH; i++) {
-              sz[i] = (~idx[i] >> 27) & 16u;                                 // 16 bytes, or 0 = zero-fill for an absent neighbour
-              idx[i] &= PEERS ? PEER_ROW_MASK : 0x7FFFFFFFu;                 // absent -> row 0, a valid address that is not read
+              for (int i = 0; i < 8 * MH; i++)
+                rp[i] = idx[i] != RING_ABSENT ? (const T*)peer_base[idx[i] >> PEER_SHIFT] + (i64)(idx[i] & PEER_ROW_MASK) * a.Ci + c16 * 8 : x;
             }
           }
-          // After a wait was given up this thread loads and signals nothing more: the table may hold anything, and an
-          // arrival on a barrier whose phase is still waiting for bytes in flight would overrun its count.
-          if (alive && !diag(a, 1) && (!TAIL || c16 < 4 || c + 1 < nchunk)) {
-            const uint32_t dst = smem_base + st * STAGE + k * UNIT + dst_thread;
-            const T* xs = x + c * KCH + c16 * 8;
-            if (PEERS && __builtin_expect(remote, 0)) {          // one branch per unit, not per copy: a P2P load when the owner is a peer
 #pragma unroll
-              for (int i = 0; i < 8 * MH; i++) cp_async16(dst + i * (16 * 128), rp[i] + c * KCH, sz[i]);
-            } else {
-#pragma unroll
-              for (int i = 0; i < 8 * MH; i++) cp_async16(dst + i * (16 * 128), xs + (i64)idx[i] * a.Ci, sz[i]);
-            }
+          for (int i = 0; i < 8 * MH; i++) {
+            sz[i] = (~idx[i] >> 27) & 16u;                                 // 16 bytes, or 0 = zero-fill for an absent neighbour
+            idx[i] &= PEERS ? PEER_ROW_MASK : 0x7FFFFFFFu;                 // absent -> row 0, a valid address that is not read
           }
-          if (++c == nchunk) { c = 0; mk &= mk - 1; }
         }
+        // After a wait was given up this thread loads and signals nothing more: the table may hold anything, and an
+        // arrival on a barrier whose phase is still waiting for bytes in flight would overrun its count.
+        if (alive && !diag(a, 1) && (!TAIL || c16 < 4 || c + 1 < nchunk)) {
+          const uint32_t dst = smem_base + st * STAGE + dst_thread;
+          const T* xs = x + c * KCH + c16 * 8;
+          if (PEERS && __builtin_expect(remote, 0)) {          // one branch per unit, not per copy: a P2P load when the owner is a peer
+#pragma unroll
+            for (int i = 0; i < 8 * MH; i++) cp_async16(dst + i * (16 * 128), rp[i] + c * KCH, sz[i]);
+          } else {
+#pragma unroll
+            for (int i = 0; i < 8 * MH; i++) cp_async16(dst + i * (16 * 128), xs + (i64)idx[i] * a.Ci, sz[i]);
+          }
+        }
+        if (++c == nchunk) { c = 0; mk &= mk - 1; }
         if (alive) cp_async_arrive_noinc(bar_full + 8 * st);     // this thread's arrival, delivered when its copies have landed
         if ((threadIdx.x & 127) == 0) trace(a, 0, 3, it);          // ... has issued its copies
       }
@@ -253,8 +248,7 @@ __global__ void __launch_bounds__(num_threads(MH, G), 1) k_conv_umma(const __gri
         const int nunits = __popc(tile.mask) * nchunk;
         uint32_t mk = tile.mask;
         int c = 0;
-        for (int u0 = 0; u0 < nunits; u0 += U, it++) {
-          const int nu = nunits - u0 < U ? nunits - u0 : U;
+        for (int u = 0; u < nunits; u++, it++) {
           const uint32_t st = it % S;
           alive &= mbar_wait(bar_empty + 8 * st, ((it / S) & 1) ^ 1, abort_flag, a.status, 2);
           if (!alive) break;
@@ -262,15 +256,11 @@ __global__ void __launch_bounds__(num_threads(MH, G), 1) k_conv_umma(const __gri
           const bool mute = diag(a, 16) && it == 0;      // bounded-wait test: this stage never fills, the MMA lane's wait runs out
           if (!mute) {
             if (diag(a, 2)) mbar_arrive(bar_full + 8 * st);
-            else mbar_arrive_expect_tx(bar_full + 8 * st, nu * B_BYTES);
+            else mbar_arrive_expect_tx(bar_full + 8 * st, B_BYTES);
           }
-#pragma unroll
-          for (int k = 0; k < U; k++) {
-            if (k >= nu) break;
-            if (!mute && !diag(a, 2))
-              tma_load_3d(smem_base + st * STAGE + k * UNIT + MH * A_BYTES, &tmw, c * KCH, __ffs(mk) - 1, wrow, bar_full + 8 * st);
-            if (++c == nchunk) { c = 0; mk &= mk - 1; }
-          }
+          if (!mute && !diag(a, 2))
+            tma_load_3d(smem_base + st * STAGE + MH * A_BYTES, &tmw, c * KCH, __ffs(mk) - 1, wrow, bar_full + 8 * st);
+          if (++c == nchunk) { c = 0; mk &= mk - 1; }
         }
         trace(a, 1, 0, (uint32_t)k);
       }
@@ -399,8 +389,7 @@ __global__ void __launch_bounds__(num_threads(MH, G), 1) k_conv_umma(const __gri
         const int halves = tile.rows > TILE_M ? MH : 1;
         const int nunits = __popc(tile.mask) * nchunk;
         [[maybe_unused]] int c = 0;
-        for (int u0 = 0; u0 < nunits; u0 += U, it++) {
-          const int nu = nunits - u0 < U ? nunits - u0 : U;
+        for (int u = 0; u < nunits; u++, it++) {
           const uint32_t s = it % S, ph = (it / S) & 1;
           // No tcgen05 fence after this wait (the operands are shared-memory data published by the barrier, not tcgen05
           // results) and no proxy fence either: the copies' completion is delivered through the barrier itself
@@ -412,20 +401,16 @@ __global__ void __launch_bounds__(num_threads(MH, G), 1) k_conv_umma(const __gri
           long long ti0 = prof ? clock64() : 0;
           if (!diag(a, 4)) {
             const uint64_t ds = desc0 + (uint64_t)(s * (STAGE >> 4));          // descriptor of the stage's first byte
-#pragma unroll
-            for (int k = 0; k < U; k++) {
-              if (k >= nu) break;
-              if constexpr (TAIL) {
-                if (++c == nchunk) {
-                  c = 0;
-                  tc_mma_k32(d_tmem, ds + ((k * UNIT) >> 4), ds + ((k * UNIT + MH * A_BYTES) >> 4), idesc, u0 + k > 0 ? 1u : 0u);
-                  continue;
-                }
-              }
+            const uint32_t acc = u > 0 ? 1u : 0u;
+            bool half = false;
+            if constexpr (TAIL) {
+              half = ++c == nchunk;
+              if (half) { c = 0; tc_mma_k32(d_tmem, ds, ds + ((MH * A_BYTES) >> 4), idesc, acc); }
+            }
+            if (!half) {
 #pragma unroll
               for (int h = 0; h < MH; h++) {
-                if (h < halves)
-                  tc_mma_k64(d_tmem + h * BN, ds + ((k * UNIT + h * A_BYTES) >> 4), ds + ((k * UNIT + MH * A_BYTES) >> 4), idesc, u0 + k > 0 ? 1u : 0u);
+                if (h < halves) tc_mma_k64(d_tmem + h * BN, ds + ((h * A_BYTES) >> 4), ds + ((MH * A_BYTES) >> 4), idesc, acc);
               }
             }
           }
@@ -463,7 +448,7 @@ __global__ void __launch_bounds__(num_threads(MH, G), 1) k_conv_umma(const __gri
       int sp = 0, ss = 0;
       if (has_skip && orow >= 0) { int sv = a.ep.skip_src[orow]; sp = sv >> 3; ss = sv & 7; }
       // this warp's copy of the item's bias values, in flight while it waits for the accumulator
-      T* const bias_w = bias_s + (warp - WARP_EPI0) * 256;
+      T* const bias_w = bias_s + (warp - WARP_EPI0) * BN;
       if (a.ep.bias) {
         __syncwarp();                                     // the previous item's reads of the copy are done
         if (lane < BN / 8) ((uint4*)bias_w)[lane] = __ldg((const uint4*)((const T*)a.ep.bias + wcol0) + lane);
@@ -520,48 +505,42 @@ static EncodeTiledFn encode_fn() {
   return fn;
 }
 
-template <int BN, int MH, int G, int U, bool PEERS, class T, bool TAIL = false, int CHILD = 0>
+template <int BN, int MH, int G, bool PEERS, class T, bool TAIL = false, int CHILD = 0, int OCC = 1>
 int launch_p(t2sc_ctx* ctx, const CUtensorMap& tm, const ConvArgs& args, i64 max_items) {
-  constexpr int smem = num_stages(BN, MH, U) * U * stage_bytes(BN, MH) + aux_bytes(MH) + 1024;
-  static_assert(smem <= SMEM_BUDGET && num_stages(BN, MH, U) >= 2, "shared memory budget");
+  constexpr int stages = num_stages(BN, MH, PEERS, OCC), smem = stages * stage_bytes(BN, MH) + aux_bytes(BN, MH, PEERS, OCC) + 1024;
+  static_assert(smem <= smem_budget(OCC) && stages >= 2, "shared memory budget");
   static bool attr_set[16] = {};
   if (!attr_set[ctx->device & 15]) {
-    T2_CUDA(ctx, cudaFuncSetAttribute(k_conv_umma<BN, MH, G, U, PEERS, TAIL, CHILD, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    T2_CUDA(ctx, cudaFuncSetAttribute(k_conv_umma<BN, MH, G, PEERS, TAIL, CHILD, OCC, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     attr_set[ctx->device & 15] = true;
   }
-  int grid = (int)(max_items < ctx->num_sms ? max_items : ctx->num_sms);
-  k_conv_umma<BN, MH, G, U, PEERS, TAIL, CHILD, T><<<grid, num_threads(MH, G), smem, ctx->stream>>>(tm, args);
+  int grid = (int)(max_items < OCC * ctx->num_sms ? max_items : OCC * ctx->num_sms);
+  k_conv_umma<BN, MH, G, PEERS, TAIL, CHILD, OCC, T><<<grid, num_threads(MH, G), smem, ctx->stream>>>(tm, args);
   T2_LAUNCHED(ctx);
   return T2SC_OK;
 }
 
-// Which form runs.  128-row tiles with Co <= 128 (accumulator tiles of 32..128 columns): two gather groups and two units
-// per stage (measured 5-12 % faster than one unit per stage at 64 and 128 channels; four units per stage are no better
-// than two).  Wider tiles: one unit per stage (a stage is 36 to 48 KB there), the second gather group only for Ci = 64.
-// 256-row tiles and the peer-memory form: one group, one unit per stage.  The diagnostic build can force one unit per
-// stage (T2SC_UNITS=1) to compare the forms.
+// Which form runs.  128-row tiles of fewer than 256 columns: two CTAs per SM, each with four gather warps, one index table and two to
+// four stages.  Every role of a CTA is a serial path of waits, copies or MMAs with gaps in it (the MMA lane alone needs 460 to 560
+// clocks per unit, 375 to 500 of which are shared-memory bandwidth), and a second CTA fills the gaps.  One CTA with two gather
+// groups and two units per stage against this, two stacked layers: 727,949 x 64 521 -> 413 us, 200,000 x 64 153 -> 131, 200,000 x 128
+// 278 -> 254, 2,000,000 x 128 2550-2720 -> 2340-2380 (with two tables and so two stages at 128 columns: 2420-2560); map, plan and
+// conv of 60,000 x 224: 234 -> 221.  256 columns: one CTA (two stages, the table and the parameters do not fit twice), the
+// second gather group only for Ci = 64.  256-row tiles and the peer-memory form: one CTA, one group.
 template <int BN, int MH, class T>
 int launch_bn(t2sc_ctx* ctx, const CUtensorMap& tm, const ConvArgs& args, i64 max_items) {
   if constexpr ((BN & (BN - 1)) == 0) {
-    if (args.npeers > 0) return launch_p<BN, MH, 1, 1, true, T>(ctx, tm, args, max_items);
+    if (args.npeers > 0) return launch_p<BN, MH, 1, true, T>(ctx, tm, args, max_items);
   }
   if constexpr (MH == 1) {
-    if (args.Ci % KCH != 0) {
-      if constexpr (BN <= 128) return launch_p<BN, MH, 2, 2, false, T, true>(ctx, tm, args, max_items);
-      else return launch_p<BN, MH, 1, 1, false, T, true>(ctx, tm, args, max_items);
+    constexpr int OCC = BN < 256 ? 2 : 1;
+    if (args.Ci % KCH != 0) return launch_p<BN, MH, 1, false, T, true, 0, OCC>(ctx, tm, args, max_items);
+    if constexpr (OCC == 1) {
+      if (args.Ci == KCH) return launch_p<BN, MH, 2, false, T>(ctx, tm, args, max_items);
     }
-  }
-  if constexpr (MH == 1 && BN <= 128) {
-#ifdef T2SC_DIAG
-    static const int force_u = [] { const char* e = getenv("T2SC_UNITS"); return e ? atoi(e) : 0; }();
-    if (force_u == 1) return args.Ci == KCH ? launch_p<BN, MH, 2, 1, false, T>(ctx, tm, args, max_items) : launch_p<BN, MH, 1, 1, false, T>(ctx, tm, args, max_items);
-#endif
-    return launch_p<BN, MH, 2, 2, false, T>(ctx, tm, args, max_items);
+    return launch_p<BN, MH, 1, false, T, false, 0, OCC>(ctx, tm, args, max_items);
   } else {
-    if constexpr (MH == 1) {
-      if (args.Ci == KCH) return launch_p<BN, MH, 2, 1, false, T>(ctx, tm, args, max_items);
-    }
-    return launch_p<BN, MH, 1, 1, false, T>(ctx, tm, args, max_items);
+    return launch_p<BN, MH, 1, false, T>(ctx, tm, args, max_items);
   }
 }
 
@@ -646,8 +625,8 @@ int conv_umma_launch(t2sc_ctx* ctx, const t2sc_plan* plan, const void* x, const 
   i64 max_items = plan->max_tiles * args.n_cot;
   int rc;
   if (child_info)
-    rc = dtype == T2SC_BF16 ? launch_p<256, 1, 1, 1, false, __nv_bfloat16, false, CONV_CHILD_CO>(ctx, tm, args, max_items)
-                            : launch_p<256, 1, 1, 1, false, __half, false, CONV_CHILD_CO>(ctx, tm, args, max_items);
+    rc = dtype == T2SC_BF16 ? launch_p<256, 1, 1, false, __nv_bfloat16, false, CONV_CHILD_CO>(ctx, tm, args, max_items)
+                            : launch_p<256, 1, 1, false, __half, false, CONV_CHILD_CO>(ctx, tm, args, max_items);
   else if (plan->tile_rows == 2 * TILE_M)
     rc = dtype == T2SC_BF16 ? launch_t<2, __nv_bfloat16>(ctx, BN, tm, args, max_items) : launch_t<2, __half>(ctx, BN, tm, args, max_items);
   else

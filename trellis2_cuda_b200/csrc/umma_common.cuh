@@ -21,7 +21,6 @@ constexpr bool kDiag = false;
 #endif
 constexpr bool kProfileWaits = kDiag;
 constexpr int IDX_SLOTS = 8;                       // index ring of the two-SM kernel: one slot per (tile, tap)
-constexpr int NTAB = 2;                            // neighbour-index tables of the single-CTA kernel: one per tile in flight
 constexpr uint32_t RING_ABSENT = 0x80000000u;      // index entry of an absent neighbour (row numbers are below 2^30)
 // Peer-memory form: a present map entry is (owner << PEER_SHIFT) | row with owner < 8 and row < 2^28, so bit 31 stays
 // free for RING_ABSENT whatever the owner.
@@ -40,19 +39,27 @@ __host__ __device__ constexpr int stage_bytes(int BN, int MH) { return MH * A_BY
 // A tile's neighbour indices, [27 taps][rows], tap-major with an odd pitch: the index warps write one map row (27 taps)
 // per instruction and the gather warps read 16 rows of one tap, both without bank conflicts.
 __host__ __device__ constexpr int tab_pitch(int MH) { return MH * TILE_M + 1; }
-__host__ __device__ constexpr int tab_words(int MH) { return 27 * tab_pitch(MH); }
-// Epilogue staging behind the tables and barriers: LayerNorm gamma and beta (fp32, up to 256 columns each) and one block of up
-// to 256 bias values per epilogue warp.
-__host__ __device__ constexpr int epi_bytes(int MH) { return 2048 + MH * 2048 + 16; }
-__host__ __device__ constexpr int aux_bytes(int MH) { return NTAB * tab_words(MH) * 4 + 1024 + epi_bytes(MH); }
-__host__ __device__ constexpr int num_stages(int BN, int MH, int U = 1) {
-  int s = (SMEM_BUDGET - 1024 - aux_bytes(MH)) / (U * stage_bytes(BN, MH));
+// [27][rows], with the odd pitch in the peer-memory form, whose index warps write a map row per instruction
+__host__ __device__ constexpr int tab_words(int MH, bool PEERS) { return 27 * (PEERS ? tab_pitch(MH) : MH * TILE_M); }
+// Index tables: one per tile in flight, two of them; a CTA that shares its SM makes do with one (the other CTA works while the
+// next tile's table arrives), which leaves room for one more stage.
+__host__ __device__ constexpr int num_tabs(int OCC) { return OCC == 2 ? 1 : 2; }
+// Barriers and small words; epilogue staging behind them: LayerNorm gamma and beta (fp32, one per column) and one block of a
+// column's bias values per epilogue warp.
+__host__ __device__ constexpr int bar_bytes(bool PEERS) { return PEERS ? 1024 : 256; }
+__host__ __device__ constexpr int epi_bytes(int BN, int MH) { return 8 * BN + MH * 8 * BN + 16; }
+__host__ __device__ constexpr int aux_bytes(int BN, int MH, bool PEERS, int OCC) {
+  return num_tabs(OCC) * tab_words(MH, PEERS) * 4 + bar_bytes(PEERS) + epi_bytes(BN, MH);
+}
+__host__ __device__ constexpr int smem_budget(int OCC) { return OCC == 2 ? 113 * 1024 : SMEM_BUDGET; }      // of a CTA, OCC of them per SM
+__host__ __device__ constexpr int num_stages(int BN, int MH, bool PEERS, int OCC) {
+  int s = (smem_budget(OCC) - 1024 - aux_bytes(BN, MH, PEERS, OCC)) / stage_bytes(BN, MH);
 #ifdef T2SC_MAX_STAGES
   if (s > T2SC_MAX_STAGES) s = T2SC_MAX_STAGES;      // measurement aid
 #endif
   return s > 8 ? 8 : s;
 }
-__host__ __device__ constexpr int num_acc_bufs(int BN, int MH) { return 2 * MH * BN <= 512 ? 2 : 1; }
+__host__ __device__ constexpr int num_acc_bufs(int BN, int MH, int OCC) { return 2 * MH * BN * OCC <= 512 ? 2 : 1; }
 // TMEM is allocated in powers of two from 32 columns up
 __host__ __device__ constexpr int tmem_cols(int used) { int c = 32; while (c < used) c *= 2; return c; }
 
