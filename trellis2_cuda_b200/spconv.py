@@ -426,21 +426,19 @@ class Level:
     def _from_parents(self, x: torch.Tensor, Cc: int) -> bool:
         """Whether the subdivision conv runs over the parents' tiles with all 8 slots (t2sc_subdiv_conv_parents) or over the
         children's.  At 64 child channels a tile of children takes as long to gather as a tile of parents does, and
-        computes a quarter of what the 256-column tile of four slots computes: all 8 slots cost what about 2.7 cost
-        one by one, and the children need no schedule of their own."""
+        computes a quarter of what the 256-column tile of four slots computes; the children's tiles also need a schedule of
+        their own.  Whole up block at 3.7 children per parent, children's tiles against parents': 60,000 parents, 128 -> 64: 539 ->
+        449 us; 880,000: 4411 -> 4031, of which the conv and its schedule are about 2150 against 1770: even at 3 children."""
         return (self._info is not None and self.src is self._info[1] and _version(self.src) == self._info[2] and Cc == 64
                 and x.dtype in (torch.float16, torch.bfloat16) and x.shape[1] % 64 == 0
-                and self.parent._tile_rows_for(256, x.shape[1]) == 128 and self.src.shape[0] > 2.7 * self.parent.N)
+                and self.parent._tile_rows_for(256, x.shape[1]) == 128 and self.src.shape[0] > 3 * self.parent.N)
 
-    def up_plan_for(self, Cc: int, Ci: int = 64) -> _Plan:
-        """Schedule of the subdivision conv into Cc child channels.  256-row tiles, two 128-row accumulators per weight slab, where
-        a slab is narrow and tiles are many: the 8 child slots have 8 weight sets, so a slab is reused by fewer rows than in a
-        submanifold conv (886,752 parents, 128 -> 64: 2.35 ms against 2.80 with 128-row tiles; 150,000, 256 -> 128: whole up block
-        1.81 against 1.87).  128-row tiles at 256 columns, where two halves leave no room for a second accumulator, and
-        below four 256-row tiles per SM, where their finer masks and shorter items fill the chip (whole up block: 1,500
-        parents, 1024 -> 512: 664 -> 450 us; 12,000: 1718 -> 1495; 8,000, 512 -> 256: 611 -> 525; 30,000, 256 -> 128: 607 ->
-        588), and for input rows that end in half a chunk, which have that form only."""
-        tr = 256 if Ci % 64 == 0 and Cc % 256 and self.src.shape[0] >= 4 * 256 * 148 else 128
+    def up_plan_for(self, Cc: int) -> _Plan:
+        """Schedule of the subdivision conv into Cc child channels: 128-row tiles, whose finer masks and shorter items fill the chip
+        on small levels and whose narrow forms run two CTAs per SM (whole up block against 256-row tiles: 1,500 parents,
+        1024 -> 512: 664 -> 450 us; 12,000: 1718 -> 1495; 8,000, 512 -> 256: 611 -> 525; 30,000, 256 -> 128: 558 -> 518; 150,000:
+        1802 -> 1690; 250,000: 2794 -> 2785)."""
+        tr = 128
         if self._up_plans is None:
             self._up_plans = {}
         if tr not in self._up_plans:
@@ -496,7 +494,7 @@ def subdiv_conv(x: torch.Tensor, w: torch.Tensor, b: Optional[torch.Tensor], lev
         raise T2scError(-1, f"spconv shapes: x has {x.shape[0]} rows, parent cache has {level.parent.N}")
     if variant == "auto" and level._from_parents(x, w.shape[0] // 8):
         return _conv_parents(level, x, w, b, ln, act, out)
-    return _conv(level.parent.ctx, level.up_plan_for(w.shape[0] // 8, w.shape[-1]), x, w, b, w.shape[0] // 8, ln, act, None, None, variant, out)
+    return _conv(level.parent.ctx, level.up_plan_for(w.shape[0] // 8), x, w, b, w.shape[0] // 8, ln, act, None, None, variant, out)
 
 
 def gather_rows(x: torch.Tensor, src: torch.Tensor, C: int, out: Optional[torch.Tensor] = None) -> torch.Tensor:
