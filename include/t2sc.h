@@ -112,7 +112,7 @@ int t2sc_subdivide_count_info(t2sc_ctx* ctx, const void* sub, int sub_dtype, con
                               int64_t n, int32_t* off, uint32_t* info, int64_t* m_host, int* whole_host);
 int t2sc_subdivide_emit_info(t2sc_ctx* ctx, const void* sub, int sub_dtype, const int32_t* coords, const int32_t* off,
                              int64_t n, int32_t* child_coords, int32_t* src, uint32_t* info);
-int t2sc_subdivide_neighbors(t2sc_ctx* ctx, const uint32_t* parent_nbr, const uint32_t* info, const int32_t* src, int64_t m,
+int t2sc_subdivide_neighbors(t2sc_ctx* ctx, const uint32_t* parent_nbr, const uint32_t* info, int64_t n,
                              uint32_t* nbr, int32_t* gray);
 
 /* Replaces k_gather_rows (src/sdec.cu:34-37): y[r,:] = x.view(-1,C)[src[r],:]. */

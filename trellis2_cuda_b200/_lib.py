@@ -46,7 +46,7 @@ SYMBOLS = [
     ("t2sc_subdivide_emit", _i32, [_vp, _vp, _i32, _vp, _vp, _i64, _vp, _vp]),
     ("t2sc_subdivide_count_info", _i32, [_vp, _vp, _i32, _vp, _vp, _i32, _i32, _i32, _i64, _vp, _vp, _pi64, ctypes.POINTER(_i32)]),
     ("t2sc_subdivide_emit_info", _i32, [_vp, _vp, _i32, _vp, _vp, _i64, _vp, _vp, _vp]),
-    ("t2sc_subdivide_neighbors", _i32, [_vp, _vp, _vp, _vp, _i64, _vp, _vp]),
+    ("t2sc_subdivide_neighbors", _i32, [_vp, _vp, _vp, _i64, _vp, _vp]),
     ("t2sc_subdiv_conv_parents", _i32, [_vp, _vp, _vp, _vp, ctypes.POINTER(Epilogue), _vp, _i32, _i64, _i32, _i32, _vp]),
     ("t2sc_gather_rows", _i32, [_vp, _vp, _vp, _i64, _i32, _i32, _vp]),
     ("t2sc_add_skip", _i32, [_vp, _vp, _vp, _vp, _i64, _i32, _i32, _i32, _i32]),

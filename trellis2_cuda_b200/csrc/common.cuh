@@ -47,7 +47,8 @@ struct t2sc_plan {
   int* perm = nullptr;          // [max_tiles]: positions -> tile numbers, each part's tiles by falling tap count: the order the
                                 // tcgen05 kernel's CTAs take them in, so that every SM gets long and short tiles alike
   bool balanced = false;        // perm is filled (maps sorted as one block); large maps keep plan order for L2 locality
-  int* meta = nullptr;          // device: group counts, bounds, stats, group bounds (one allocation, one memset)
+  char* block = nullptr;        // the one allocation that meta, order, tiles, perm and tnbr lie in
+  int* meta = nullptr;          // device: group counts, bounds, stats, group bounds, tap-count bins (one memset)
   int* bounds = nullptr;        // = meta + 8, device [3]: {0, first boundary tile, realised tile count}; parts are [b0,b1) and [b1,b2)
   int* ntiles = nullptr;        // = bounds + 2: realised tile count (<= max_tiles)
   int* group_tiles = nullptr;   // = meta + 16, device [9]: first tile of every group and the tile count (chunked plans)

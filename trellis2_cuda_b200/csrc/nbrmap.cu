@@ -94,7 +94,7 @@ __global__ void k_brick_insert(const int4* __restrict__ coords, int n, int Wb, i
   }
 }
 
-// Where a voxel's 8 bricks come from: the hash table, or (a subdivided level) the parent level, whose voxels ARE the bricks.
+// Where a voxel's 8 bricks come from: the hash table.
 struct HashBricks {
   const int4* coords; int W, H, D, Wb, Hb, Db; const unsigned long long* keys; const BrickVals* vals; uint32_t mask;
   // parity of the voxel in its brick, and the 8 rows of brick t = (sx, sy, sz) of its 2x2x2 neighbourhood of bricks: along one
@@ -122,31 +122,46 @@ struct HashBricks {
   }
 };
 
-// A child's brick t is its parent or one of the parent's neighbours; info[q] = {row of q's first child, 8-bit set of its
-// children}, and a parent's children lie in slot order one behind the other.
-struct ParentBricks {
-  const int* src; const uint32_t* nbr; const uint2* info;
-  __device__ __forceinline__ int load(i64 row, int t, uint32_t* v) const {
-    const int sv = __ldg(src + row), p = sv >> 3, slot = sv & 7;
-    // offset of the brick from the parent along an axis: slot bit 0 -> {-1, 0}, 1 -> {0, +1}
-    const int ox = (t & 1) + (slot & 1), oy = ((t >> 1) & 1) + ((slot >> 1) & 1), oz = (t >> 2) + (slot >> 2);
-    const uint32_t q = __ldg(nbr + (i64)p * 27 + ox * 9 + oy * 3 + oz);
-    if (q != NBR_EMPTY) {
-      const uint2 f = __ldg(info + q);
+// The map of a subdivided level: one warp per parent, lane = tap.  A lane holds info[q] = {row of the first child, 8-bit set of
+// children} of the parent's neighbour in its tap's direction, loaded once for all of the parent's children (which lie in slot order one
+// behind the other); the neighbour of child s in direction v is child (s + v) & 1 of the parent's neighbour (s + v) >> 1 along
+// each axis, so its row is a shuffle and a popcount away.  (Through the hash kernel's form, 8 threads per child that each
+// look a brick up by way of src, map and info: 275 us for 3,288,465 children.)
+__global__ void __launch_bounds__(256) k_child_neighbors(const uint32_t* __restrict__ pnbr, const uint2* __restrict__ info, int n,
+                                                         uint32_t* __restrict__ nbr, int* __restrict__ gray) {
+  const int p = (int)((blockIdx.x * 256ll + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  if (p >= n) return;
+  const uint2 own = __ldg(info + p);
+  if (!own.y) return;
+  const uint32_t q = lane < 27 ? __ldg(pnbr + (i64)p * 27 + lane) : NBR_EMPTY;
+  uint2 f = make_uint2(0u, 0u);
+  if (q != NBR_EMPTY) f = __ldg(info + q);
+  // per axis and slot bit b: with d = tap offset + 1 (0..2), b + d + 1 is twice the neighbour's offset + 1, plus its slot bit; parent tap in
+  // the low byte, slot above
+  const int v = lane < 27 ? lane : 26, d[3] = {v / 9, (v / 3) % 3, v % 3}, mul[3] = {9, 3, 1};
+  int to[3][2];
 #pragma unroll
-      for (int e = 0; e < 8; e++)
-        if (f.y >> e & 1) v[e] = f.x + __popc(f.y & ((1u << e) - 1));
-    }
-    return slot;
+  for (int a = 0; a < 3; a++)
+#pragma unroll
+    for (int b = 0; b < 2; b++) to[a][b] = ((b + d[a] + 1) >> 1) * mul[a] | ((b + d[a] + 1) & 1) << (8 + a);
+  uint32_t row = own.x;
+  for (uint32_t kids = own.y; kids; kids &= kids - 1, row++) {
+    const int s = __ffs(kids) - 1;
+    const int at = (s & 1 ? to[0][1] : to[0][0]) + (s & 2 ? to[1][1] : to[1][0]) + (s & 4 ? to[2][1] : to[2][0]);
+    const uint32_t first = __shfl_sync(0xffffffffu, f.x, at & 31), set = __shfl_sync(0xffffffffu, f.y, at & 31);
+    const int slot = at >> 8;
+    const uint32_t r = set >> slot & 1 ? first + __popc(set & ((1u << slot) - 1)) : NBR_EMPTY;
+    if (lane < 27) nbr[(i64)row * 27 + lane] = r;
+    const uint32_t m = __ballot_sync(0xffffffffu, lane < 27 && r != NBR_EMPTY);
+    if (lane == 0) gray[row] = (int)m;
   }
-};
+}
 
 // 8 threads per row fetch the rows of its 8 bricks (64 cells) into shared memory; then a warp writes four rows of the map, lane = tap:
 // 27 consecutive words per store, and the presence mask is the ballot.  Bound by instruction issue, so the work per entry is
 // what was cut: the fetching threads used to pick their taps out of the 8 cells and store them one by one (1,000,003 rows:
 // 130 -> 107 us; with the CTA's rows gathered in shared memory and stored in 16-byte pieces: 125).
-template <class Bricks>
-__global__ void __launch_bounds__(256) k_brick_neighbors(const Bricks bricks, int n, uint32_t* __restrict__ nbr, int* __restrict__ gray,
+__global__ void __launch_bounds__(256) k_brick_neighbors(const HashBricks bricks, int n, uint32_t* __restrict__ nbr, int* __restrict__ gray,
                                                          int* __restrict__ bin, int* __restrict__ iota) {
   __shared__ __align__(16) uint32_t s_cell[32][64];
   __shared__ int s_par[32];
@@ -453,14 +468,14 @@ extern "C" int t2sc_subdivide_emit_info(t2sc_ctx* ctx, const void* sub, int sub_
 // The children's neighbour map without a hash table: every neighbour of a child is a child of its parent or of one of the
 // parent's 26 neighbours.  (On 3,288,465 children the table took a memset of 335 MB, an atomic insertion per row and eight
 // probes per row.)
-extern "C" int t2sc_subdivide_neighbors(t2sc_ctx* ctx, const uint32_t* parent_nbr, const uint32_t* info, const int32_t* src, int64_t m,
+extern "C" int t2sc_subdivide_neighbors(t2sc_ctx* ctx, const uint32_t* parent_nbr, const uint32_t* info, int64_t n,
                                         uint32_t* nbr, int32_t* gray) {
   T2_REQ(ctx, ctx != nullptr, "null context");
-  T2_REQ(ctx, m >= 0 && m < (1ll << 30), "m=%lld", (long long)m);
-  if (m == 0) return T2SC_OK;
-  T2_REQ(ctx, parent_nbr && info && src && nbr && gray && (uintptr_t)info % 8 == 0, "null or unaligned tensor");
+  T2_REQ(ctx, n >= 0 && n < (1ll << 28), "n=%lld", (long long)n);
+  if (n == 0) return T2SC_OK;
+  T2_REQ(ctx, parent_nbr && info && nbr && gray && (uintptr_t)info % 8 == 0, "null or unaligned tensor");
   T2_CUDA(ctx, cudaSetDevice(ctx->device));
-  k_brick_neighbors<<<cdiv_i(m, 32), 256, 0, ctx->stream>>>(ParentBricks{src, parent_nbr, (const uint2*)info}, (int)m, nbr, gray, nullptr, nullptr);
+  k_child_neighbors<<<cdiv_i(n, 8), 256, 0, ctx->stream>>>(parent_nbr, (const uint2*)info, (int)n, nbr, gray);
   T2_LAUNCHED(ctx);
   return T2SC_OK;
 }

@@ -479,7 +479,7 @@ def subdivide(parent: SpConvCache, sub: torch.Tensor, want_sorted: bool = False)
     # every parent is in the grid and alone at its place: the children's map follows from the parents'
     nbr = torch.empty((m.value, 27), dtype=torch.int32, device=sub.device)
     gray = torch.empty(m.value, dtype=torch.int32, device=sub.device)
-    ctx.check(ctx.lib.t2sc_subdivide_neighbors(ctx.h, _ptr(parent.nbr), _ptr(info), _ptr(src), m.value, _ptr(nbr), _ptr(gray)))
+    ctx.check(ctx.lib.t2sc_subdivide_neighbors(ctx.h, _ptr(parent.nbr), _ptr(info), n, _ptr(nbr), _ptr(gray)))
     return Level(coords, src, SpConvCache(ctx, coords, nbr, gray, None)._built((4096, 4096, 4096)), parent, None, known)
 
 
