@@ -107,3 +107,17 @@ def test_tap_groups_sum_to_the_whole_conv(sp, n, Ci, Co, dt):
     cache = sp.build_neighbors(torch.from_numpy(cube(1000, 12, 3)).cuda())
     assert cache.conv_plan_for(1024, 1024, dt) is not cache.plan_for(1024, 1024) and cache.conv_plan_for(64, 64, dt) is cache.plan_for(64, 64)
     sp.context().device_status()
+
+
+@pytest.mark.parametrize("Cin,Co,n", [(128, 64, 700), (512, 256, 300), (2048, 1024, 200), (256, 32, 700), (128, 128, 700), (64, 32, 333), (128, 32, 500)])
+def test_fused_skip_is_conv_then_add(sp, Cin, Co, n):
+    """rep = 4 in one load per block (8 or 16 bytes apart), other factors element by element, in the conv's epilogue and in the row pass: the
+    bits of the conv followed by add_skip."""
+    rep = Co // (Cin // 8)
+    g = torch.Generator(device="cuda").manual_seed(Cin + Co)
+    cache = sp.build_neighbors(torch.from_numpy(cube(n, 8, 4)).cuda())
+    x, parent = (torch.randn((m, c), generator=g, device="cuda").to(torch.bfloat16) for m, c in ((n, 64), (40, Cin)))
+    src = torch.randint(0, 40 * 8, (n,), generator=g, device="cuda", dtype=torch.int32)
+    w = (torch.randn((Co, 27, 64), generator=g, device="cuda") * 0.03).to(torch.bfloat16)
+    for kw in (dict(), dict(ln=(None, None, 1e-6))):
+        assert torch.equal(sp.subm_conv(x, w, None, cache, skip=(parent, src, rep), **kw), sp.add_skip(sp.subm_conv(x, w, None, cache, **kw), parent, src, rep))

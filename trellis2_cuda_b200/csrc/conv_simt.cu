@@ -311,8 +311,14 @@ __global__ void __launch_bounds__(256, 4) k_row_epilogue_vec(const T* x, EpiDev 
     if (skx) {
       const int sv = ep.skip_src[row];
       const T* sx = skx + (i64)(sv >> 3) * ep.skip_cin + (sv & 7) * (ep.skip_cin / 8);
+      if (ep.skip_rep == 4) {           // the decoder's: two values, no divisions
+        const float lo = to_f<T>(sx[vi * 2]), hi = to_f<T>(sx[vi * 2 + 1]);
 #pragma unroll
-      for (int i = 0; i < 8; i++) h[i] = rnd<T>(h[i] + to_f<T>(sx[(vi * 8 + i) / ep.skip_rep]));
+        for (int i = 0; i < 8; i++) h[i] = rnd<T>(h[i] + (i < 4 ? lo : hi));
+      } else {
+#pragma unroll
+        for (int i = 0; i < 8; i++) h[i] = rnd<T>(h[i] + to_f<T>(sx[(vi * 8 + i) / ep.skip_rep]));
+      }
     }
     store8<T>(y + row * C + vi * 8, h);
   }

@@ -56,7 +56,7 @@ using namespace umma;
 //
 // CHILD > 0 (subdivision conv from the parents' tiles): the BN columns are BN / CHILD child slots of CHILD channels; the epilogue
 // treats each as a row of its own, of the child that sits there, and skips slots that are not kept.
-template <int BN, int MH, int G, bool PEERS, bool TAIL, int CHILD, int OCC, class T>
+template <int BN, int MH, int G, bool PEERS, bool TAIL, int CHILD, int OCC, bool SKIP, class T>
 __global__ void __launch_bounds__(num_threads(MH, G), OCC) k_conv_umma(const __grid_constant__ CUtensorMap tmw, const ConvArgs a) {
   static_assert(!TAIL || (MH == 1 && !PEERS), "half chunks run on 128-row tiles of local rows");
   static_assert(G == 1 || (G == 2 && MH == 1), "a second gather group only fits beside 128-row tiles");
@@ -429,7 +429,7 @@ __global__ void __launch_bounds__(num_threads(MH, G), OCC) k_conv_umma(const __g
     __syncwarp();
   } else {
     // ===================================================================== epilogue
-    const bool has_skip = a.ep.skip_x != nullptr;
+    const bool has_skip = SKIP && a.ep.skip_x != nullptr;
     const int q = warp & 3, half = (warp - WARP_EPI0) >> 2, j = half * TILE_M + q * 32 + lane;
     uint32_t acc_it = 0;
     const bool prof = diag(a, 8); long long w_accf = 0, t_role = clock64();
@@ -466,10 +466,10 @@ __global__ void __launch_bounds__(num_threads(MH, G), OCC) k_conv_umma(const __g
           const int slot = cot * (BN / CHILD) + s;
           const int crow = kids.y >> slot & 1 ? (int)kids.x + __popc(kids.y & ((1u << slot) - 1)) : -1;
           if (__any_sync(0xffffffffu, crow >= 0))
-            epilogue_row<CHILD, T>(a, taddr + s * CHILD, crow, 0, a.ep.bias ? bias_w + s * CHILD : nullptr, gamma_s, beta_s, 0, 0);
+            epilogue_row<CHILD, T, SKIP>(a, taddr + s * CHILD, crow, 0, a.ep.bias ? bias_w + s * CHILD : nullptr, gamma_s, beta_s, 0, 0);
         }
       } else {
-        if (!diag(a, 64)) epilogue_row<BN, T>(a, taddr, orow, cot, a.ep.bias ? bias_w : nullptr, gamma_s, beta_s, sp, ss);
+        if (!diag(a, 64)) epilogue_row<BN, T, SKIP>(a, taddr, orow, cot, a.ep.bias ? bias_w : nullptr, gamma_s, beta_s, sp, ss);
       }
       tc_fence_before();
       mbar_arrive(bar_acce + 8 * buf);
@@ -505,17 +505,17 @@ static EncodeTiledFn encode_fn() {
   return fn;
 }
 
-template <int BN, int MH, int G, bool PEERS, class T, bool TAIL = false, int CHILD = 0, int OCC = 1>
+template <int BN, int MH, int G, bool PEERS, class T, bool TAIL = false, int CHILD = 0, int OCC = 1, bool SKIP = true>
 int launch_p(t2sc_ctx* ctx, const CUtensorMap& tm, const ConvArgs& args, i64 max_items) {
   constexpr int stages = num_stages(BN, MH, PEERS, OCC), smem = stages * stage_bytes(BN, MH) + aux_bytes(BN, MH, PEERS, OCC) + 1024;
   static_assert(smem <= smem_budget(OCC) && stages >= 2, "shared memory budget");
   static bool attr_set[16] = {};
   if (!attr_set[ctx->device & 15]) {
-    T2_CUDA(ctx, cudaFuncSetAttribute(k_conv_umma<BN, MH, G, PEERS, TAIL, CHILD, OCC, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    T2_CUDA(ctx, cudaFuncSetAttribute(k_conv_umma<BN, MH, G, PEERS, TAIL, CHILD, OCC, SKIP, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     attr_set[ctx->device & 15] = true;
   }
   int grid = (int)(max_items < OCC * ctx->num_sms ? max_items : OCC * ctx->num_sms);
-  k_conv_umma<BN, MH, G, PEERS, TAIL, CHILD, OCC, T><<<grid, num_threads(MH, G), smem, ctx->stream>>>(tm, args);
+  k_conv_umma<BN, MH, G, PEERS, TAIL, CHILD, OCC, SKIP, T><<<grid, num_threads(MH, G), smem, ctx->stream>>>(tm, args);
   T2_LAUNCHED(ctx);
   return T2SC_OK;
 }
@@ -535,10 +535,11 @@ int launch_bn(t2sc_ctx* ctx, const CUtensorMap& tm, const ConvArgs& args, i64 ma
   if constexpr (MH == 1) {
     constexpr int OCC = BN < 256 ? 2 : 1;
     if (args.Ci % KCH != 0) return launch_p<BN, MH, 1, false, T, true, 0, OCC>(ctx, tm, args, max_items);
+    if (args.ep.skip_x) return launch_p<BN, MH, 1, false, T, false, 0, OCC, true>(ctx, tm, args, max_items);
     if constexpr (OCC == 1) {
-      if (args.Ci == KCH) return launch_p<BN, MH, 2, false, T>(ctx, tm, args, max_items);
+      if (args.Ci == KCH) return launch_p<BN, MH, 2, false, T, false, 0, 1, false>(ctx, tm, args, max_items);
     }
-    return launch_p<BN, MH, 1, false, T, false, 0, OCC>(ctx, tm, args, max_items);
+    return launch_p<BN, MH, 1, false, T, false, 0, OCC, false>(ctx, tm, args, max_items);
   } else {
     return launch_p<BN, MH, 1, false, T>(ctx, tm, args, max_items);
   }
@@ -625,8 +626,8 @@ int conv_umma_launch(t2sc_ctx* ctx, const t2sc_plan* plan, const void* x, const 
   i64 max_items = plan->max_tiles * args.n_cot;
   int rc;
   if (child_info)
-    rc = dtype == T2SC_BF16 ? launch_p<256, 1, 1, false, __nv_bfloat16, false, CONV_CHILD_CO>(ctx, tm, args, max_items)
-                            : launch_p<256, 1, 1, false, __half, false, CONV_CHILD_CO>(ctx, tm, args, max_items);
+    rc = dtype == T2SC_BF16 ? launch_p<256, 1, 1, false, __nv_bfloat16, false, CONV_CHILD_CO, 1, false>(ctx, tm, args, max_items)
+                            : launch_p<256, 1, 1, false, __half, false, CONV_CHILD_CO, 1, false>(ctx, tm, args, max_items);
   else if (plan->tile_rows == 2 * TILE_M)
     rc = dtype == T2SC_BF16 ? launch_t<2, __nv_bfloat16>(ctx, BN, tm, args, max_items) : launch_t<2, __half>(ctx, BN, tm, args, max_items);
   else

@@ -122,20 +122,25 @@ struct HashBricks {
   }
 };
 
-// The map of a subdivided level: one warp per parent, lane = tap.  A lane holds info[q] = {row of the first child, 8-bit set of
-// children} of the parent's neighbour in its tap's direction, loaded once for all of the parent's children (which lie in slot order one
+// The map of a subdivided level: one warp per four parents, lane = tap.  A lane holds info[q] = {row of the first child, 8-bit set of
+// children} of a parent's neighbour in its tap's direction, loaded once for all of the parent's children (which lie in slot order one
 // behind the other); the neighbour of child s in direction v is child (s + v) & 1 of the parent's neighbour (s + v) >> 1 along
-// each axis, so its row is a shuffle and a popcount away.  (Through the hash kernel's form, 8 threads per child that each
-// look a brick up by way of src, map and info: 275 us for 3,288,465 children.)
+// each axis, so its row is a shuffle and a popcount away.  Three loads depend on one another here, which with one parent per
+// warp was the whole time (269 us for 3,288,465 children, as much as 8 threads per child that each look a brick up); four
+// parents' loads are in flight together (218 us).
+constexpr int CHILD_PARENTS = 4;
 __global__ void __launch_bounds__(256) k_child_neighbors(const uint32_t* __restrict__ pnbr, const uint2* __restrict__ info, int n,
                                                          uint32_t* __restrict__ nbr, int* __restrict__ gray) {
-  const int p = (int)((blockIdx.x * 256ll + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-  if (p >= n) return;
-  const uint2 own = __ldg(info + p);
-  if (!own.y) return;
-  const uint32_t q = lane < 27 ? __ldg(pnbr + (i64)p * 27 + lane) : NBR_EMPTY;
-  uint2 f = make_uint2(0u, 0u);
-  if (q != NBR_EMPTY) f = __ldg(info + q);
+  const int p0 = (int)((blockIdx.x * 256ll + threadIdx.x) >> 5) * CHILD_PARENTS, lane = threadIdx.x & 31;
+  uint32_t q[CHILD_PARENTS];
+  uint2 own[CHILD_PARENTS], f[CHILD_PARENTS];
+#pragma unroll
+  for (int k = 0; k < CHILD_PARENTS; k++) {
+    own[k] = p0 + k < n ? __ldg(info + p0 + k) : make_uint2(0u, 0u);
+    q[k] = p0 + k < n && lane < 27 ? __ldg(pnbr + (i64)(p0 + k) * 27 + lane) : NBR_EMPTY;
+  }
+#pragma unroll
+  for (int k = 0; k < CHILD_PARENTS; k++) f[k] = q[k] != NBR_EMPTY ? __ldg(info + q[k]) : make_uint2(0u, 0u);
   // per axis and slot bit b: with d = tap offset + 1 (0..2), b + d + 1 is twice the neighbour's offset + 1, plus its slot bit; parent tap in
   // the low byte, slot above
   const int v = lane < 27 ? lane : 26, d[3] = {v / 9, (v / 3) % 3, v % 3}, mul[3] = {9, 3, 1};
@@ -144,16 +149,19 @@ __global__ void __launch_bounds__(256) k_child_neighbors(const uint32_t* __restr
   for (int a = 0; a < 3; a++)
 #pragma unroll
     for (int b = 0; b < 2; b++) to[a][b] = ((b + d[a] + 1) >> 1) * mul[a] | ((b + d[a] + 1) & 1) << (8 + a);
-  uint32_t row = own.x;
-  for (uint32_t kids = own.y; kids; kids &= kids - 1, row++) {
-    const int s = __ffs(kids) - 1;
-    const int at = (s & 1 ? to[0][1] : to[0][0]) + (s & 2 ? to[1][1] : to[1][0]) + (s & 4 ? to[2][1] : to[2][0]);
-    const uint32_t first = __shfl_sync(0xffffffffu, f.x, at & 31), set = __shfl_sync(0xffffffffu, f.y, at & 31);
-    const int slot = at >> 8;
-    const uint32_t r = set >> slot & 1 ? first + __popc(set & ((1u << slot) - 1)) : NBR_EMPTY;
-    if (lane < 27) nbr[(i64)row * 27 + lane] = r;
-    const uint32_t m = __ballot_sync(0xffffffffu, lane < 27 && r != NBR_EMPTY);
-    if (lane == 0) gray[row] = (int)m;
+#pragma unroll
+  for (int k = 0; k < CHILD_PARENTS; k++) {
+    uint32_t row = own[k].x;
+    for (uint32_t kids = own[k].y; kids; kids &= kids - 1, row++) {
+      const int s = __ffs(kids) - 1;
+      const int at = (s & 1 ? to[0][1] : to[0][0]) + (s & 2 ? to[1][1] : to[1][0]) + (s & 4 ? to[2][1] : to[2][0]);
+      const uint32_t first = __shfl_sync(0xffffffffu, f[k].x, at & 31), set = __shfl_sync(0xffffffffu, f[k].y, at & 31);
+      const int slot = at >> 8;
+      const uint32_t r = set >> slot & 1 ? first + __popc(set & ((1u << slot) - 1)) : NBR_EMPTY;
+      if (lane < 27) nbr[(i64)row * 27 + lane] = r;
+      const uint32_t m = __ballot_sync(0xffffffffu, lane < 27 && r != NBR_EMPTY);
+      if (lane == 0) gray[row] = (int)m;
+    }
   }
 }
 
@@ -475,7 +483,7 @@ extern "C" int t2sc_subdivide_neighbors(t2sc_ctx* ctx, const uint32_t* parent_nb
   if (n == 0) return T2SC_OK;
   T2_REQ(ctx, parent_nbr && info && nbr && gray && (uintptr_t)info % 8 == 0, "null or unaligned tensor");
   T2_CUDA(ctx, cudaSetDevice(ctx->device));
-  k_child_neighbors<<<cdiv_i(n, 8), 256, 0, ctx->stream>>>(parent_nbr, (const uint2*)info, (int)n, nbr, gray);
+  k_child_neighbors<<<cdiv_i(n, 8 * CHILD_PARENTS), 256, 0, ctx->stream>>>(parent_nbr, (const uint2*)info, (int)n, nbr, gray);
   T2_LAUNCHED(ctx);
   return T2SC_OK;
 }

@@ -279,21 +279,10 @@ __device__ __forceinline__ void add_packed32(uint32_t* hp, const uint4* src) {  
 // bias points at the item's first column (or is null); gamma / beta at the row's first column (LayerNorm only, may be null).
 // The kernels hand in copies in shared memory: a per-element load from global memory here costs its full latency once per
 // block, because one epilogue warp per scheduler has nothing else to run meanwhile.
-template <int BN, class T>
-__device__ __forceinline__ void epilogue_row(const ConvArgs& a, uint32_t taddr, int orow, int cot, const T* bias, const float* gamma, const float* beta, int sp, int ss) {
-  if (a.partial) {
-    float* const p = a.partial + (i64)orow * a.Co + cot * BN;
-#pragma unroll 1
-    for (int cc = 0; cc < BN / 32; cc++) {
-      uint32_t r[32]; tc_ld32(taddr + cc * 32, r); tc_wait_ld();
-      if (orow < 0) continue;
-#pragma unroll
-      for (int g = 0; g < 4; g++)       // a row starts on a multiple of 128 bytes
-        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p + cc * 32 + g * 8), "r"(r[g * 8]), "r"(r[g * 8 + 1]), "r"(r[g * 8 + 2]),
-                     "r"(r[g * 8 + 3]), "r"(r[g * 8 + 4]), "r"(r[g * 8 + 5]), "r"(r[g * 8 + 6]), "r"(r[g * 8 + 7]) : "memory");
-    }
-    return;
-  }
+// SKIP: the row may have a skip.  Kernels without one are forms of their own, because its registers and code cost them 8 to 11 % (ConvNeXt
+// block 727,949 x 64: 626 -> 676 us, with both forms in one kernel 694, with kernels of their own 609).
+template <int BN, class T, bool SKIP>
+__device__ __forceinline__ void epilogue_form(const ConvArgs& a, uint32_t taddr, int orow, int cot, const T* bias, const float* gamma, const float* beta, int sp, int ss) {
   T* y = (T*)a.y;
   const T* res = (const T*)a.ep.residual; const T* skx = (const T*)a.ep.skip_x;
   float mean = 0.f, rstd = 1.f;
@@ -328,8 +317,15 @@ __device__ __forceinline__ void epilogue_row(const ConvArgs& a, uint32_t taddr, 
 #pragma unroll
     for (int g = 0; g < 4; g++) rnext[g] = __ldg(rp + g);
   }
+  // The skip row of a subdivided level: each of its channels is added to `rep` neighbouring columns.  With rep = 4, what halving the channels
+  // per level gives, a block's 8 values are one 16-byte load, in flight while the block comes out of TMEM; a load and
+  // a division per element were a third of a conv with skip (3,288,465 x 64: 1486 -> 957 us; 148,000 x 256: 384 -> 267).
+  const T* const sx = SKIP && skx ? skx + (i64)sp * a.ep.skip_cin + ss * (a.ep.skip_cin / 8) : nullptr;
+  const bool skip4 = SKIP && skx && a.ep.skip_rep == 4 && ((uintptr_t)sx & 15) == 0;
   for (int cc = 0; cc < BN / 32; cc++) {
     uint32_t r[32]; tc_ld32(taddr + cc * 32, r);
+    uint4 scur = make_uint4(0u, 0u, 0u, 0u);
+    if (skip4 && orow >= 0) scur = __ldg((const uint4*)(sx + (cot * BN + cc * 32) / 4));
     uint4 rcur[4];
     if (rp) {
 #pragma unroll
@@ -370,8 +366,15 @@ __device__ __forceinline__ void epilogue_row(const ConvArgs& a, uint32_t taddr, 
       }
     }
     if (rp) add_packed32<T>(hp, rcur);
-    if (skx) {
-      const T* sx = skx + (i64)sp * a.ep.skip_cin + ss * (a.ep.skip_cin / 8);
+    if (skip4) {
+      const uint32_t* w32 = (const uint32_t*)&scur;
+#pragma unroll
+      for (int i = 0; i < 16; i++) {
+        const float2 h = unpack2<T>(hp[i]), pair = unpack2<T>(w32[i / 4]);
+        const float v = i / 2 % 2 ? pair.y : pair.x;
+        hp[i] = pack2<T>(h.x + v, h.y + v);
+      }
+    } else if (SKIP && skx) {
 #pragma unroll
       for (int i = 0; i < 16; i++) {
         const float2 h = unpack2<T>(hp[i]);
@@ -391,6 +394,24 @@ __device__ __forceinline__ void epilogue_row(const ConvArgs& a, uint32_t taddr, 
       for (int g = 0; g < 4; g++) yp[g] = make_uint4(hp[g * 4], hp[g * 4 + 1], hp[g * 4 + 2], hp[g * 4 + 3]);
     }
   }
+}
+
+template <int BN, class T, bool SKIP>
+__device__ __forceinline__ void epilogue_row(const ConvArgs& a, uint32_t taddr, int orow, int cot, const T* bias, const float* gamma, const float* beta, int sp, int ss) {
+  if (a.partial) {
+    float* const p = a.partial + (i64)orow * a.Co + cot * BN;
+#pragma unroll 1
+    for (int cc = 0; cc < BN / 32; cc++) {
+      uint32_t r[32]; tc_ld32(taddr + cc * 32, r); tc_wait_ld();
+      if (orow < 0) continue;
+#pragma unroll
+      for (int g = 0; g < 4; g++)       // a row starts on a multiple of 128 bytes
+        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p + cc * 32 + g * 8), "r"(r[g * 8]), "r"(r[g * 8 + 1]), "r"(r[g * 8 + 2]),
+                     "r"(r[g * 8 + 3]), "r"(r[g * 8 + 4]), "r"(r[g * 8 + 5]), "r"(r[g * 8 + 6]), "r"(r[g * 8 + 7]) : "memory");
+    }
+    return;
+  }
+  epilogue_form<BN, T, SKIP>(a, taddr, orow, cot, bias, gamma, beta, sp, ss);
 }
 
 }  // namespace umma
