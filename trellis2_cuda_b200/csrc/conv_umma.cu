@@ -4,20 +4,19 @@
 // present in its tile, y[row, co] += x[nbr[row, v], :] . w[co, v, :].  The reference runs 32-64 row tiles
 // through mma.sync with register-staged copies; this kernel is organised around the Blackwell units:
 //
-//   * persistent CTAs, one per SM, walk (plan tile x BN output channels) work items.  A plan tile is MH
+//   * persistent CTAs, one per SM (two for tiles of fewer than 256 columns), walk (plan tile x BN output channels) work items.  A plan tile is MH
 //     128-row halves (MH = 1 or 2); each half has its own TMEM accumulator and all halves consume the
 //     same weight slab, which halves the L2 -> SM weight traffic of the 128-row schedule;
 //   * warps 0-3 gather the A operand: one 16-byte cp.async per (row, 8 channels), zero-filled for absent
 //     neighbours, written straight into the 128-byte-swizzled K-major layout tcgen05 reads.  (TMA
 //     tile::gather4 was measured for this job and moves 128-byte rows three times slower.)  Everything that
 //     does not depend on the channel chunk is done once per tap, so a copy is two instructions;
-//   * warp 5 and the last warp of the base set copy each tile's neighbour-map rows into a [27 taps][rows] table in
-//     shared memory (4-byte cp.async, a whole tile in flight at once), one tile ahead of the gather warps, so
-//     that neither a tap nor a new tile starts with a chain of dependent loads;
+//   * one lane of warp 5 fetches each tile's [27 taps][rows] index table with one bulk copy, so that no tap starts with a chain
+//     of dependent loads (the peer-memory form builds it from map rows with two warps);
 //   * one lane of warp 4 streams the B operand (the tap's [BN x 64] weight slab) with a 3-D TMA tile load
 //     from the weights in their checkpoint layout [Co,27,Ci] - no re-layout, no cluster multicast;
 //   * one lane of warp 6 issues tcgen05.mma (M=128, N=BN, K=16) per half into TMEM and releases smem stages /
-//     publishes accumulators with tcgen05.commit; when 2*MH*BN <= 512 columns the accumulators are double
+//     publishes accumulators with tcgen05.commit; where TMEM has room for two the accumulators are double
 //     buffered so the epilogue of one tile overlaps the main loop of the next;
 //   * 4*MH epilogue warps drain the accumulators with tcgen05.ld and apply the fused epilogue (bias,
 //     LayerNorm, activation, residual, skip) with the reference's rounding points, one thread per output
