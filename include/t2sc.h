@@ -149,12 +149,6 @@ int t2sc_plan_check(t2sc_ctx* ctx, t2sc_plan* plan, int64_t n_in);
  * output row exactly once, with the bits t2sc_subm_conv gives on an unsplit plan. */
 int t2sc_plan_create_split(t2sc_ctx* ctx, const uint32_t* nbr, const int32_t* gray, int64_t n_rows, int64_t n_own,
                            int64_t block_rows, int tile_rows, t2sc_plan** out);
-/* Plan for a small map of wide rows: the three planes of 9 taps are sorted, tiled and summed apart, and a row pass adds the fp32
- * partial sums before the epilogue (the reference's split-K, src/spconv.cu:153-157, with an order of its own per part).  Taken by
- * t2sc_subm_conv on the tcgen05 path (whole plan, Co <= 2048); results differ from those of a t2sc_plan_create plan by the order
- * of an fp32 sum.  Also borrows gray.  wants_tap_groups: 1 where such a plan is the faster one. */
-int t2sc_plan_create_taps(t2sc_ctx* ctx, const uint32_t* nbr, const int32_t* gray, int64_t n_rows, t2sc_plan** out);
-int t2sc_plan_wants_tap_groups(t2sc_ctx* ctx, int64_t n_rows, int dtype, int Ci, int Co);
 enum { T2SC_PART_ALL = 0, T2SC_PART_INTERIOR = 1, T2SC_PART_BOUNDARY = 2 };
 /* tiles of the two parts (syncs); a plan not made by t2sc_plan_create_split is all interior */
 int t2sc_plan_parts(t2sc_ctx* ctx, t2sc_plan* plan, int64_t* interior_tiles, int64_t* boundary_tiles);

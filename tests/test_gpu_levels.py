@@ -79,36 +79,6 @@ def test_subdivision_conv_over_the_parents_tiles(sp, n, Ci, dt):
     assert not level._from_parents(x, 64)
 
 
-@pytest.mark.parametrize("n,Ci,Co,dt", [(1, 64, 64, torch.float16), (130, 96, 160, torch.bfloat16), (700, 512, 256, torch.bfloat16), (1800, 1024, 512, torch.float16),
-                                        (900, 64, 1056, torch.bfloat16)])
-def test_tap_groups_sum_to_the_whole_conv(sp, n, Ci, Co, dt):
-    """The three planes of taps summed apart and added in fp32, against the one accumulator: a partial sum may differ by K 2^-24 of
-    its terms, and each later op rounds once (the bias, the activation and the residual at a size of the terms they add)."""
-    g = torch.Generator(device="cuda").manual_seed(n)
-    c = cube(n, max(2, round((n / 0.6) ** (1 / 3))), 2)
-    far = c.copy(); far[:, 1] += 1000 + 3 * np.arange(n)                      # every row alone: no partial sum but the middle one
-    x, res = torch.randn((n, Ci), generator=g, device="cuda").to(dt), torch.randn((n, Co), generator=g, device="cuda").to(dt)
-    w = (torch.randn((Co, 27, Ci), generator=g, device="cuda") / (27 * Ci) ** 0.5).to(dt)
-    b = torch.randn(Co + 2, generator=g, device="cuda")
-    step = 2.0 ** (-10 if dt == torch.float16 else -7)
-    from trellis2_cuda_b200 import spconv
-    for coords in (c, far):
-        cache = sp.build_neighbors(torch.from_numpy(coords).cuda())
-        taps = spconv._Plan(cache.ctx, cache.nbr, cache.gray, None, 0, 128, taps=True)
-        conv = lambda b, ln=None, act=None, residual=None: spconv._conv(cache.ctx, taps, x, w, b, Co, ln, act, residual, None, "auto", None)
-        for kw in (dict(), dict(act="silu", residual=res)):
-            y, want = conv(b[:Co].to(dt), **kw).double(), sp.subm_conv(x, w, b[:Co].to(dt), cache, variant="umma" if Ci % 64 == 0 else "simt", **kw).double()
-            size = want.abs() + b[:Co].double().abs() + res.double().abs() + 1
-            assert ((y - want).abs() <= (4 * step + 27 * Ci * 2.0 ** -24) * size).all()
-        # LayerNorm with parameters that start in the middle of 16 bytes
-        got = conv(None, ln=(b[1:Co + 1], b[2:Co + 2], 1e-6)).double()
-        h = torch.nn.functional.layer_norm(conv(None).double(), (Co,), eps=1e-6) * b[1:Co + 1].double()
-        assert ((got - h - b[2:Co + 2].double()).abs() <= 2 * step * (h.abs() + b[2:Co + 2].double().abs() + 1e-3)).all()
-    cache = sp.build_neighbors(torch.from_numpy(cube(1000, 12, 3)).cuda())
-    assert cache.conv_plan_for(1024, 1024, dt) is not cache.plan_for(1024, 1024) and cache.conv_plan_for(64, 64, dt) is cache.plan_for(64, 64)
-    sp.context().device_status()
-
-
 @pytest.mark.parametrize("Cin,Co,n", [(128, 64, 700), (512, 256, 300), (2048, 1024, 200), (256, 32, 700), (128, 128, 700), (64, 32, 333), (128, 32, 500)])
 def test_fused_skip_is_conv_then_add(sp, Cin, Co, n):
     """rep = 4 in one load per block (8 or 16 bytes apart), other factors element by element, in the conv's epilogue and in the row pass: the

@@ -52,8 +52,6 @@ SYMBOLS = [
     ("t2sc_add_skip", _i32, [_vp, _vp, _vp, _vp, _i64, _i32, _i32, _i32, _i32]),
     ("t2sc_plan_create", _i32, [_vp, _vp, _vp, _i64, _vp, _i64, _i64, _i32, _pp]),
     ("t2sc_plan_create_split", _i32, [_vp, _vp, _vp, _i64, _i64, _i64, _i32, _pp]),
-    ("t2sc_plan_create_taps", _i32, [_vp, _vp, _vp, _i64, _pp]),
-    ("t2sc_plan_wants_tap_groups", _i32, [_vp, _i64, _i32, _i32, _i32]),
     ("t2sc_plan_parts", _i32, [_vp, _vp, _pi64, _pi64]),
     ("t2sc_plan_destroy", _i32, [_vp, _vp]),
     ("t2sc_plan_set_input_rows", _i32, [_vp, _vp, _i64]),

@@ -138,16 +138,6 @@ int conv_dispatch(t2sc_ctx* ctx, t2sc_plan* plan, const void* x, const void* w, 
   // (multiples of 32 up to 256; for one part of a plan, and for 256-row tiles, the powers of two), else conv + bias first and LayerNorm ->
   // activation -> residual -> skip in a row pass
   bool fuse_all = use_umma && (!e.ln || conv_umma_fuses_ln(Co, part != T2SC_PART_ALL || plan->tile_rows != 128));
-  if (plan->tap_groups) {
-    if (!use_umma || variant == T2SC_VARIANT_UMMA_PAIR || part != T2SC_PART_ALL || Co > 2048)
-      return t2sc_fail(ctx, T2SC_ERR_UNSUPPORTED, "a tap-group plan needs the tcgen05 form, the whole plan and Co <= 2048 (Ci=%d Co=%d dtype=%d part=%d)", Ci, Co, dtype, part);
-    Scratch scratch(ctx);
-    float* partial = nullptr;
-    T2_CUDA(ctx, scratch.get(&partial, (size_t)TAP_GROUPS * plan->n_out * Co));
-    EpiDev none; memset(&none, 0, sizeof(none));
-    const int rc = conv_umma_launch(ctx, plan, x, w, w_rows, none, y, dtype, n_in, Ci, Co, part, nullptr, nullptr, 0, 0, nullptr, nullptr, partial);
-    return rc != T2SC_OK ? rc : partial_sums_launch(ctx, partial, plan->gray, e, y, plan->n_out, Co, dtype);
-  }
   if (variant == T2SC_VARIANT_UMMA_PAIR) {
     if (!conv_umma2_supported(plan, dtype, Ci, Co, e))
       return t2sc_fail(ctx, T2SC_ERR_UNSUPPORTED, "two-SM tcgen05 variant needs fp16/bf16, a 256-row plan, Ci %% 64 == 0, Co %% 256 == 0 (Ci=%d Co=%d tile_rows=%d)", Ci, Co, plan->tile_rows);
@@ -172,7 +162,7 @@ extern "C" int t2sc_subdiv_conv_parents(t2sc_ctx* ctx, t2sc_plan* plan, const vo
   T2_REQ(ctx, ctx && plan, "null context or plan");
   T2_REQ(ctx, n_in == plan->n_in, "spconv shapes: x has %lld rows, the plan's neighbour map is over %lld", (long long)n_in, (long long)plan->n_in);
   EpiDev e = epi_dev(ep);
-  if ((dtype != T2SC_F16 && dtype != T2SC_BF16) || Ci <= 0 || Ci % 64 || Cc != CONV_CHILD_CO || plan->src || plan->tile_rows != 128 || plan->split || plan->tap_groups || e.skip_x)
+  if ((dtype != T2SC_F16 && dtype != T2SC_BF16) || Ci <= 0 || Ci % 64 || Cc != CONV_CHILD_CO || plan->src || plan->tile_rows != 128 || plan->split || e.skip_x)
     return t2sc_fail(ctx, T2SC_ERR_UNSUPPORTED, "subdivision conv from the parents' plan needs fp16/bf16, Ci %% 64 == 0, Cc == %d, a submanifold plan with 128-row tiles, no skip (Ci=%d Cc=%d dtype=%d)",
                      CONV_CHILD_CO, Ci, Cc, dtype);
   if (plan->n_out == 0) return T2SC_OK;
@@ -199,8 +189,8 @@ extern "C" int t2sc_subm_conv_peers_part(t2sc_ctx* ctx, t2sc_plan* plan, const u
   T2_REQ(ctx, w && y, "null tensor");
   for (int r = 0; r < n_peers; r++) T2_REQ(ctx, x_peers[r] && (uintptr_t)x_peers[r] % 16 == 0, "peer array %d is null or not 16-byte aligned", r);
   EpiDev e = epi_dev(ep);
-  if (!conv_umma_supported(dtype, Ci, Co, 256) || (e.ln && !conv_umma_fuses_ln(Co, true)) || plan->src || plan->tap_groups)
-    return t2sc_fail(ctx, T2SC_ERR_UNSUPPORTED, "peer conv needs a submanifold plan without tap groups, fp16/bf16, Ci %% 64 == 0, Co %% 32 == 0, LayerNorm only for Co in {32,64,128,256} (Ci=%d Co=%d dtype=%d)", Ci, Co, dtype);
+  if (!conv_umma_supported(dtype, Ci, Co, 256) || (e.ln && !conv_umma_fuses_ln(Co, true)) || plan->src)
+    return t2sc_fail(ctx, T2SC_ERR_UNSUPPORTED, "peer conv needs a submanifold plan, fp16/bf16, Ci %% 64 == 0, Co %% 32 == 0, LayerNorm only for Co in {32,64,128,256} (Ci=%d Co=%d dtype=%d)", Ci, Co, dtype);
   return conv_umma_launch(ctx, plan, x_peers[self_rank], w, Co, e, y, dtype, rows_peers[self_rank], Ci, Co, part, x_peers, rows_peers, n_peers,
                           self_rank, peer_nbr);
 }
@@ -359,9 +349,7 @@ extern "C" int t2sc_subm_conv_host(t2sc_ctx* ctx, const int32_t* coords_host, in
     T2_CUDA(ctx, cudaMemcpyAsync(c.w, w_host, wbytes, cudaMemcpyHostToDevice, ctx->stream));
     if (bias_host) T2_CUDA(ctx, cudaMemcpyAsync(c.b, bias_host, yrow, cudaMemcpyHostToDevice, ctx->stream));
     if ((rc = t2sc_build_neighbors(ctx, c.coords, n, W, H, D, c.nbr, c.gray, nullptr)) != T2SC_OK) return rc;
-    rc = t2sc_plan_wants_tap_groups(ctx, n, dtype, Ci, Co) ? t2sc_plan_create_taps(ctx, c.nbr, c.gray, n, &c.plan)
-                                                           : t2sc_plan_create(ctx, c.nbr, c.gray, n, nullptr, n, 0, 0, &c.plan);
-    if (rc != T2SC_OK) return rc;
+    if ((rc = t2sc_plan_create(ctx, c.nbr, c.gray, n, nullptr, n, 0, 0, &c.plan)) != T2SC_OK) return rc;
     if ((rc = t2sc_subm_conv(ctx, c.plan, c.x, c.w, &ep, c.y, dtype, n, Ci, Co, T2SC_VARIANT_AUTO)) != T2SC_OK) return rc;
     T2_CUDA(ctx, cudaMemcpyAsync(y_host, c.y, (size_t)n * yrow, cudaMemcpyDeviceToHost, ctx->stream));
   } else {

@@ -52,9 +52,6 @@ struct t2sc_plan {
   int* bounds = nullptr;        // = meta + 8, device [3]: {0, first boundary tile, realised tile count}; parts are [b0,b1) and [b1,b2)
   int* ntiles = nullptr;        // = bounds + 2: realised tile count (<= max_tiles)
   int* group_tiles = nullptr;   // = meta + 16, device [9]: first tile of every group and the tile count (chunked plans)
-  int tap_groups = 0;           // 3: order[] holds entries group * n_out + row, every tile has the taps of one group, and a conv makes a
-                                // partial sum per entry that the row pass adds (t2sc_plan_create_taps)
-  const int32_t* gray = nullptr;  // borrowed (tap-group plans: which partial sums a row has)
   bool split = false;           // made by t2sc_plan_create_split: interior tiles first, boundary tiles last
   unsigned long long* stats = nullptr;  // device: pairs of computed taps, active taps, to be added up
   i64 max_tiles = 0;
@@ -180,14 +177,10 @@ bool conv_umma_fuses_ln(int Co, bool pow2 = false);
 int conv_umma_launch(t2sc_ctx* ctx, const t2sc_plan* plan, const void* x, const void* w, i64 w_rows, const EpiDev& ep, void* y,
                      int dtype, i64 n_in, int Ci, int Co, int part = T2SC_PART_ALL, const void* const* x_peers = nullptr,
                      const int64_t* rows_peers = nullptr, int n_peers = 0, int self_rank = 0, const uint32_t* peer_nbr = nullptr,
-                     const uint32_t* child_info = nullptr, float* partial = nullptr);
-int conv_umma_slabs(int Co);          // column slabs a tile's rows are gathered for
+                     const uint32_t* child_info = nullptr);
 constexpr int CONV_CHILD_CO = 64;     // child width of the parents' form of the subdivision conv (t2sc_subdiv_conv_parents)
 int linear_umma_launch(t2sc_ctx* ctx, const void* x, const void* w, const EpiDev& ep, void* y, int dtype, i64 n, int Ci, int Co);
 bool conv_umma2_supported(const t2sc_plan* plan, int dtype, int Ci, int Co, const EpiDev& ep);
 int conv_umma2_launch(t2sc_ctx* ctx, const t2sc_plan* plan, const void* x, const void* w, i64 w_rows, const EpiDev& ep, void* y,
                       int dtype, i64 n_in, int Ci, int Co, int part = T2SC_PART_ALL);
-// the row pass over the sum of a tap-group plan's partial sums [3][n][C]
-int partial_sums_launch(t2sc_ctx* ctx, const float* partial, const int32_t* gray, const EpiDev& ep, void* y, i64 n, int C, int dtype);
-constexpr int TAP_GROUPS = 3, TAP_GROUP_TAPS = 9;     // the planes x-1, x, x+1 of the neighbourhood
 int row_epilogue_launch(t2sc_ctx* ctx, const void* x, const EpiDev& ep, void* y, i64 n, int C, int dtype);

@@ -205,11 +205,8 @@ template <class T> __device__ __forceinline__ float act_row(float v, int act) {
 // fetched again for every row (64 bytes for 16 of x) and IEEE divisions that pass took 387 us, now 157: the lanes fit the
 // row, a thread keeps its piece of gamma and beta over the rows of a grid-stride loop, and the next row is in flight while one is
 // worked on.  Rows of several pieces per lane left a small map with too few warps (3,727 x 1024: less than one per scheduler slot).
-// PART: the rows are sums of up to three fp32 partial sums (`part` [3][n][C], those whose taps the row has), rounded to the storage
-// type as the conv's epilogue rounds its accumulators; x is not read.
-template <class T, int LPR, int WPR, bool PART = false>
-__global__ void __launch_bounds__(256, 4) k_row_epilogue_vec(const T* x, EpiDev ep, T* y, i64 n, int C,   // y may alias x
-                                                             const float* part = nullptr, const int* gray = nullptr) {
+template <class T, int LPR, int WPR>
+__global__ void __launch_bounds__(256, 4) k_row_epilogue_vec(const T* x, EpiDev ep, T* y, i64 n, int C) {   // y may alias x
   static_assert(WPR == 1 || LPR == 32, "several warps per row only for whole warps");
   constexpr int TPR = LPR * WPR, RPB = 256 / TPR;       // threads per row, rows per block
   __shared__ float s_sum[2][8];
@@ -236,44 +233,21 @@ __global__ void __launch_bounds__(256, 4) k_row_epilogue_vec(const T* x, EpiDev 
 #pragma unroll
   for (int i = 0; i < 8; i++) { g[i] = 1.f; be[i] = 0.f; }
   if (ep.ln && mine) {
-    if (PART && (((uintptr_t)ep.gamma | (uintptr_t)ep.beta) & 15)) {      // a caller's slice of a longer array
-#pragma unroll
-      for (int i = 0; i < 8; i++) { if (ep.gamma) g[i] = ep.gamma[vi * 8 + i]; if (ep.beta) be[i] = ep.beta[vi * 8 + i]; }
-    } else {
-      if (ep.gamma) load8<float>(ep.gamma + vi * 8, g);
-      if (ep.beta) load8<float>(ep.beta + vi * 8, be);
-    }
+    if (ep.gamma) load8<float>(ep.gamma + vi * 8, g);
+    if (ep.beta) load8<float>(ep.beta + vi * 8, be);
   }
   const i64 step = gridDim.x * (i64)RPB;
   i64 row = blockIdx.x * (i64)RPB + threadIdx.x / TPR;
   Raw8<T> next;
-  if (!PART && row < n && mine) next.load(x + row * C + vi * 8);
+  if (row < n && mine) next.load(x + row * C + vi * 8);
   // The trip count is the block's, because of the barriers: a thread whose row lies past the end works on nothing.
   for (i64 base = blockIdx.x * (i64)RPB; base < n; base += step, row += step) {
     const bool live = row < n && mine;
     float h[8];
 #pragma unroll
     for (int i = 0; i < 8; i++) h[i] = 0.f;
-    if constexpr (PART) {
-      if (live) {
-        const uint32_t taps = (uint32_t)gray[row];
-        float v[TAP_GROUPS][8];
-#pragma unroll
-        for (int q = 0; q < TAP_GROUPS; q++)
-          if (taps >> (TAP_GROUP_TAPS * q) & 0x1ffu) load8<float>(part + (q * n + row) * C + vi * 8, v[q]);
-#pragma unroll
-        for (int q = 0; q < TAP_GROUPS; q++)
-          if (taps >> (TAP_GROUP_TAPS * q) & 0x1ffu) {
-#pragma unroll
-            for (int i = 0; i < 8; i++) h[i] += v[q][i];
-          }
-#pragma unroll
-        for (int i = 0; i < 8; i++) h[i] = rnd<T>(h[i]);
-      }
-    } else {
-      if (live) next.unpack(h);
-      if (row + step < n && mine) next.load(x + (row + step) * C + vi * 8);
-    }
+    if (live) next.unpack(h);
+    if (row + step < n && mine) next.load(x + (row + step) * C + vi * 8);
     if (bias && live) {
       float b[8]; load8<T>(bias + vi * 8, b);
 #pragma unroll
@@ -349,26 +323,7 @@ void row_epilogue_pick(t2sc_ctx* ctx, const void* x, const EpiDev& ep, void* y, 
   }
 }
 
-template <class T>
-void partial_sums_pick(t2sc_ctx* ctx, const float* part, const int* gray, const EpiDev& ep, void* y, i64 n, int C) {
-#define T2_ROWS(LPR, WPR) k_row_epilogue_vec<T, LPR, WPR, true><<<row_grid(ctx, n, 256 / (LPR * WPR)), 256, 0, ctx->stream>>>(nullptr, ep, (T*)y, n, C, part, gray)
-  if (C <= 128) T2_ROWS(16, 1);
-  else if (C <= 256) T2_ROWS(32, 1);
-  else if (C <= 512) T2_ROWS(32, 2);
-  else if (C <= 1024) T2_ROWS(32, 4);
-  else T2_ROWS(32, 8);
-#undef T2_ROWS
-}
-
 }  // namespace
-
-int partial_sums_launch(t2sc_ctx* ctx, const float* partial, const int32_t* gray, const EpiDev& ep, void* y, i64 n, int C, int dtype) {
-  T2_REQ(ctx, C % 8 == 0 && C <= 2048, "C=%d", C);
-  if (dtype == T2SC_F16) partial_sums_pick<__half>(ctx, partial, gray, ep, y, n, C);
-  else partial_sums_pick<__nv_bfloat16>(ctx, partial, gray, ep, y, n, C);
-  T2_LAUNCHED(ctx);
-  return T2SC_OK;
-}
 
 int conv_simt_launch(t2sc_ctx* ctx, const t2sc_plan* plan, const void* x, const void* w, const EpiDev& ep, void* y,
                      int dtype, i64 n_in, int Ci, int Co, int part) {

@@ -577,13 +577,11 @@ bool conv_umma_supported(int dtype, int Ci, int Co, int tile_rows) {
   return (dtype == T2SC_F16 || dtype == T2SC_BF16) && Ci % (tile_rows == TILE_M ? KCH / 2 : KCH) == 0 && Co % 32 == 0;
 }
 
-int conv_umma_slabs(int Co) { return Co / pick_bn(Co); }
-
 bool conv_umma_fuses_ln(int Co, bool pow2) { return pick_bn(Co, pow2) == Co; }
 
 int conv_umma_launch(t2sc_ctx* ctx, const t2sc_plan* plan, const void* x, const void* w, i64 w_rows, const EpiDev& ep, void* y,
                      int dtype, i64 n_in, int Ci, int Co, int part, const void* const* x_peers, const int64_t* rows_peers, int n_peers,
-                     int self_rank, const uint32_t* peer_nbr, const uint32_t* child_info, float* partial) {
+                     int self_rank, const uint32_t* peer_nbr, const uint32_t* child_info) {
   T2_CUDA(ctx, cudaSetDevice(ctx->device));
   const int BN = child_info ? 256 : pick_bn(Co, n_peers > 0 || plan->tile_rows != TILE_M);
   T2_REQ(ctx, BN > 0, "Co=%d", Co);
@@ -621,7 +619,6 @@ int conv_umma_launch(t2sc_ctx* ctx, const t2sc_plan* plan, const void* x, const 
   args.tiles = plan->tiles; args.tile_lo = tile_part(plan, part).lo; args.tile_hi = tile_part(plan, part).hi; args.status = ctx->status;
   args.Ci = Ci; args.Co = Co; args.n_cot = (child_info ? 8 * Co : Co) / BN; args.is_bf16 = dtype == T2SC_BF16; args.ep = ep;
   args.child_info = (const uint2*)child_info;
-  args.partial = partial;
   i64 max_items = plan->max_tiles * args.n_cot;
   int rc;
   if (child_info)

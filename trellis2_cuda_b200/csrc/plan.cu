@@ -33,16 +33,15 @@ __device__ __forceinline__ uint32_t mask_key(uint32_t g) {
 // key = group | block (block_bits wide) | mask key (27 bits), most significant first, with the `drop` least significant
 // mask-key bits left out; K is uint32_t when that fits in 32 bits (half the sort traffic), else unsigned long long.
 // halo_from > 0 (split plan, no src): group 1 = rows with a map entry >= halo_from (a row of a peer), group 0 = the rest
-// tap_rows > 0 (no src): entry i is row i % tap_rows with the taps of group i / tap_rows; one without any goes to the group behind them
 // chunk_rows > 0 (no src): group = chunk of the largest map entry; rows whose group lies behind their own chunk go to late[]
 template <class K>
 __global__ void k_plan_keys(const int* __restrict__ gray, const int* __restrict__ src, const uint32_t* __restrict__ nbr, uint32_t halo_from,
-                            uint32_t tap_rows, uint32_t chunk_rows, int* __restrict__ late, int* __restrict__ n_late, i64 m, uint32_t block_rows, int block_bits, int drop,
+                            uint32_t chunk_rows, int* __restrict__ late, int* __restrict__ n_late, i64 m, uint32_t block_rows, int block_bits, int drop,
                             K* __restrict__ keys, int* __restrict__ iota, int* __restrict__ group_cnt) {
   // group sizes: counted per CTA in shared memory first (millions of rows on eight counters in global memory were the
   // whole time of this kernel)
   __shared__ int s_cnt[8];
-  const bool grouped = src || halo_from || chunk_rows || tap_rows;
+  const bool grouped = src || halo_from || chunk_rows;
   if (grouped && threadIdx.x < 8) s_cnt[threadIdx.x] = 0;
   if (grouped) __syncthreads();
   i64 i = blockIdx.x * (i64)blockDim.x + threadIdx.x;
@@ -62,22 +61,8 @@ __global__ void k_plan_keys(const int* __restrict__ gray, const int* __restrict_
       grp = (int)(min(last, (uint32_t)(m - 1)) / chunk_rows);
       if (grp > (int)((uint32_t)i / chunk_rows)) late[atomicAdd(n_late, 1)] = (int)i;
     }
-    uint32_t taps = 0x7ffffffu;
-    if (tap_rows) {
-      grp = (int)((uint32_t)i / tap_rows); nrow = i - (i64)grp * tap_rows;
-      taps = 0x1ffu << (TAP_GROUP_TAPS * grp);
-    }
-    const uint32_t m_row = (uint32_t)gray[nrow] & taps;
-    if (tap_rows && !m_row) grp = TAP_GROUPS;
-    const unsigned long long blk = (uint32_t)(tap_rows ? nrow : i) / block_rows;          // rows are below 2^30: no 64-bit division
-    // a tap group's key is 11 bits: the group and its 9 taps, corners, edges, faces, centre as above (the same places in every plane)
-    uint32_t own = 0;
-    if (tap_rows) {
-      const uint32_t t = (m_row | m_row >> TAP_GROUP_TAPS | m_row >> (2 * TAP_GROUP_TAPS)) & 0x1ffu;
-      own = (t & 1) << 8 | (t >> 2 & 1) << 7 | (t >> 6 & 1) << 6 | (t >> 8 & 1) << 5 | (t >> 1 & 1) << 4 | (t >> 3 & 1) << 3 | (t >> 5 & 1) << 2 | (t >> 7 & 1) << 1 | (t >> 4 & 1);
-      own ^= own >> 8; own ^= own >> 4; own ^= own >> 2; own ^= own >> 1;
-    }
-    const unsigned long long k = tap_rows ? (unsigned long long)(grp << TAP_GROUP_TAPS | own) : ((unsigned long long)grp << (27 + block_bits)) | (blk << 27) | mask_key(m_row);
+    const unsigned long long blk = (uint32_t)i / block_rows;          // rows are below 2^30: no 64-bit division
+    const unsigned long long k = ((unsigned long long)grp << (27 + block_bits)) | (blk << 27) | mask_key((uint32_t)gray[nrow]);
     keys[i] = (K)(k >> drop);
     iota[i] = (int)i;
     if (grouped) atomicAdd(&s_cnt[grp], 1);
@@ -100,7 +85,7 @@ constexpr int META_SLOTS = 32, META_MAX = 32, META_STATS = META_MAX + META_SLOTS
 template <int TILE, bool HEADER>
 __global__ void __launch_bounds__(256) k_plan_tiles_table(const uint32_t* __restrict__ nbr, const int* __restrict__ gray, const int* __restrict__ src,
                                                           const int* __restrict__ order, const int* __restrict__ group_cnt, int ngroups, int split,
-                                                          i64 m, uint32_t tap_rows, PlanTile* __restrict__ tiles, int* __restrict__ bounds, int* __restrict__ group_tiles, bool slots,
+                                                          i64 m, PlanTile* __restrict__ tiles, int* __restrict__ bounds, int* __restrict__ group_tiles, bool slots,
                                                           unsigned long long* __restrict__ stats, uint32_t* __restrict__ table,
                                                           uint32_t* __restrict__ max_entry, int* __restrict__ hist, int win) {
   const int t = blockIdx.x;
@@ -133,15 +118,13 @@ __global__ void __launch_bounds__(256) k_plan_tiles_table(const uint32_t* __rest
     tile = tiles[t];
   }
   if (threadIdx.x == 0) s_big = 0;
-  uint32_t taps = 0x7ffffffu;
-  if constexpr (HEADER) { if (tap_rows) taps = 0x1ffu << (TAP_GROUP_TAPS * (order[tile.start] / tap_rows)); }      // a tile's entries are of one group
   __syncthreads();
   uint32_t o = 0; int act = 0;
   for (int j = threadIdx.x; j < TILE; j += 256) {
     int nr = -1;
     if (j < tile.rows) {
-      const int r = order[tile.start + j]; nr = src ? (src[r] >> 3) : tap_rows ? (int)((uint32_t)r % tap_rows) : r;
-      if constexpr (HEADER) { const uint32_t gm = (uint32_t)gray[nr] & taps; o |= gm; act += __popc(gm); }
+      const int r = order[tile.start + j]; nr = src ? (src[r] >> 3) : r;
+      if constexpr (HEADER) { const uint32_t gm = (uint32_t)gray[nr]; o |= gm; act += __popc(gm); }
     }
     s_row[j] = nr;
   }
@@ -228,10 +211,10 @@ template <bool HEADER>
 int plan_tiles_table(t2sc_ctx* ctx, t2sc_plan* p, const int32_t* gray, const int* gcnt, int ngroups, int* hist = nullptr, int win = 1) {
   if (p->n_out == 0) return T2SC_OK;
   if (p->tile_rows == 128)
-    k_plan_tiles_table<128, HEADER><<<(unsigned)p->max_tiles, 256, 0, ctx->stream>>>(p->nbr, gray, p->src, p->order, gcnt, ngroups, p->split ? 1 : 0, p->n_out, p->tap_groups ? (uint32_t)p->n_out : 0u,
+    k_plan_tiles_table<128, HEADER><<<(unsigned)p->max_tiles, 256, 0, ctx->stream>>>(p->nbr, gray, p->src, p->order, gcnt, ngroups, p->split ? 1 : 0, p->n_out,
                                                                                        p->tiles, p->bounds, p->group_tiles, p->src != nullptr, p->stats, p->tnbr, (uint32_t*)(p->meta + META_MAX), hist, win);
   else
-    k_plan_tiles_table<256, HEADER><<<(unsigned)p->max_tiles, 256, 0, ctx->stream>>>(p->nbr, gray, p->src, p->order, gcnt, ngroups, p->split ? 1 : 0, p->n_out, p->tap_groups ? (uint32_t)p->n_out : 0u,
+    k_plan_tiles_table<256, HEADER><<<(unsigned)p->max_tiles, 256, 0, ctx->stream>>>(p->nbr, gray, p->src, p->order, gcnt, ngroups, p->split ? 1 : 0, p->n_out,
                                                                                        p->tiles, p->bounds, p->group_tiles, p->src != nullptr, p->stats, p->tnbr, (uint32_t*)(p->meta + META_MAX), hist, win);
   T2_LAUNCHED(ctx);
   if (HEADER && hist) {
@@ -265,7 +248,7 @@ extern "C" int t2sc_plan_check(t2sc_ctx* ctx, t2sc_plan* p, int64_t n_in) {
 
 static int plan_create(t2sc_ctx* ctx, const uint32_t* nbr, const int32_t* gray, int64_t n_rows,
                        const int32_t* src, int64_t m, int64_t halo_from, int64_t block_rows, int tile_rows, t2sc_plan** out,
-                       i64 chunk_rows = 0, int* late = nullptr, int* n_late = nullptr, bool tap_groups = false) {
+                       i64 chunk_rows = 0, int* late = nullptr, int* n_late = nullptr) {
   T2_REQ(ctx, ctx && out, "null context or out");
   *out = nullptr;
   T2_REQ(ctx, n_rows >= 0 && m >= 0 && m < (1ll << 30) && n_rows < (1ll << 30), "n_rows=%lld m=%lld", (long long)n_rows, (long long)m);
@@ -283,7 +266,6 @@ static int plan_create(t2sc_ctx* ctx, const uint32_t* nbr, const int32_t* gray, 
   p->split = split != 0;
   int ngroups = src ? 8 : (split ? 2 : 1);
   if (chunk_rows > 0) ngroups = cdiv_i(m, chunk_rows);
-  if (tap_groups) { ngroups = TAP_GROUPS; p->tap_groups = TAP_GROUPS; p->gray = gray; m *= TAP_GROUPS; }      // from here on m counts entries
   const int group_bits = ngroups > 2 ? 3 : (ngroups > 1 ? 1 : 0);
   p->max_tiles = cdiv_i(m, TILE) + (ngroups > 1 ? ngroups : 0);
   Scratch scratch(ctx);            // sort buffers: back to the pool on every path out
@@ -315,14 +297,11 @@ static int plan_create(t2sc_ctx* ctx, const uint32_t* nbr, const int32_t* gray, 
     // 14,534 rows, 0.665 / 0.665 / 0.665 / 0.665 / 0.665; on 30,011, 0.717 / 0.717 / 0.718 / 0.717 / 0.716; on 100,000, 0.796 /
     // 0.796 / 0.791 / 0.786 / 0.780; on 217,821, 0.853 / 0.850 / 0.842 / 0.831 / 0.819.  A pass of the sort takes 8 bits and 11 us
     // (36 us on 3,288,465 rows), so the bits needed are rounded up to whole passes and no further.
-    int drop = 0;
-    if (!tap_groups) {
-      const i64 together = (block_rows < m ? block_rows : m) / ngroups;
-      const int need = together <= 16384 ? 13 : together <= 49152 ? 16 : together <= 65536 ? 18 : 24;
-      const int bits = (block_bits + group_bits + need + 7) / 8 * 8 - block_bits - group_bits;
-      drop = bits < 24 ? 27 - bits : 3;
-    }
-    const int key_bits = tap_groups ? 2 + TAP_GROUP_TAPS : 27 + block_bits + group_bits - drop;
+    const i64 together = (block_rows < m ? block_rows : m) / ngroups;
+    const int need = together <= 16384 ? 13 : together <= 49152 ? 16 : together <= 65536 ? 18 : 24;
+    const int bits = (block_bits + group_bits + need + 7) / 8 * 8 - block_bits - group_bits;
+    const int drop = bits < 24 ? 27 - bits : 3;
+    const int key_bits = 27 + block_bits + group_bits - drop;
     const bool narrow = key_bits <= 32;
     const size_t ksz = narrow ? sizeof(uint32_t) : sizeof(unsigned long long);
     char* buf = nullptr; char* tmp = nullptr; size_t tb = 0;
@@ -331,14 +310,14 @@ static int plan_create(t2sc_ctx* ctx, const uint32_t* nbr, const int32_t* gray, 
     int* iota = (int*)(buf + 2 * koff);
     if (narrow) {
       uint32_t *keys = (uint32_t*)buf, *keys2 = (uint32_t*)(buf + koff);
-      k_plan_keys<uint32_t><<<cdiv_i(m, 256), 256, 0, ctx->stream>>>(gray, src, nbr, (uint32_t)halo_from, tap_groups ? (uint32_t)p->n_out : 0u, (uint32_t)chunk_rows, late, n_late, m, (uint32_t)(block_rows < m ? block_rows : m), block_bits, drop, keys, iota, p->meta);
+      k_plan_keys<uint32_t><<<cdiv_i(m, 256), 256, 0, ctx->stream>>>(gray, src, nbr, (uint32_t)halo_from, (uint32_t)chunk_rows, late, n_late, m, (uint32_t)(block_rows < m ? block_rows : m), block_bits, drop, keys, iota, p->meta);
       ctx->launches++; PL(cudaGetLastError());
       PL(cub::DeviceRadixSort::SortPairs(nullptr, tb, keys, keys2, iota, p->order, (int)m, 0, key_bits, ctx->stream));
       PL(scratch.get(&tmp, tb));
       PL(cub::DeviceRadixSort::SortPairs(tmp, tb, keys, keys2, iota, p->order, (int)m, 0, key_bits, ctx->stream));
     } else {
       unsigned long long *keys = (unsigned long long*)buf, *keys2 = (unsigned long long*)(buf + koff);
-      k_plan_keys<unsigned long long><<<cdiv_i(m, 256), 256, 0, ctx->stream>>>(gray, src, nbr, (uint32_t)halo_from, tap_groups ? (uint32_t)p->n_out : 0u, (uint32_t)chunk_rows, late, n_late, m, (uint32_t)(block_rows < m ? block_rows : m), block_bits, drop, keys, iota, p->meta);
+      k_plan_keys<unsigned long long><<<cdiv_i(m, 256), 256, 0, ctx->stream>>>(gray, src, nbr, (uint32_t)halo_from, (uint32_t)chunk_rows, late, n_late, m, (uint32_t)(block_rows < m ? block_rows : m), block_bits, drop, keys, iota, p->meta);
       ctx->launches++; PL(cudaGetLastError());
       PL(cub::DeviceRadixSort::SortPairs(nullptr, tb, keys, keys2, iota, p->order, (int)m, 0, key_bits, ctx->stream));
       PL(scratch.get(&tmp, tb));
@@ -346,7 +325,7 @@ static int plan_create(t2sc_ctx* ctx, const uint32_t* nbr, const int32_t* gray, 
     }
     // The order the conv's CTAs take the tiles in (k_plan_perm): by tap count when the rows were sorted as one block; plan
     // order when they were sorted inside runs (large maps: the runs keep concurrently running tiles L2-local).
-    p->balanced = block_rows >= p->n_out && chunk_rows == 0;        // (k_plan_perm knows two parts)
+    p->balanced = block_rows >= m && chunk_rows == 0;        // (k_plan_perm knows two parts)
     const int win = 1 << 30;
     int* const hist = p->balanced ? p->meta + META_INTS : nullptr;
     if (plan_tiles_table<true>(ctx, p, gray, p->meta, ngroups, hist, win) != T2SC_OK) return fail(cudaGetLastError());
@@ -359,26 +338,6 @@ static int plan_create(t2sc_ctx* ctx, const uint32_t* nbr, const int32_t* gray, 
 int plan_create_chunked(t2sc_ctx* ctx, const uint32_t* nbr, const int32_t* gray, i64 n, i64 chunk_rows, int* late, int* n_late, t2sc_plan** out) {
   T2_REQ(ctx, n > 0 && chunk_rows > 0 && cdiv_i(n, chunk_rows) <= 8, "n=%lld chunk_rows=%lld", (long long)n, (long long)chunk_rows);
   return plan_create(ctx, nbr, gray, n, nullptr, n, 0, 0, 0, out, chunk_rows, late, n_late);
-}
-
-// Which maps run with tap groups.  A small map of wide rows has few tiles and each of them computes most of the 27 taps (3,727 voxels
-// of a shell: 30 tiles, 738 tile-taps for 444 tiles' worth of present taps), so a conv takes as long as its longest tile while
-// other SMs idle.  With the three planes of taps sorted, tiled and summed apart the same map has 86 tiles of at most 9 taps and
-// 584 tile-taps; the price is three fp32 partial sums per output, written and read again.  The two sides below are the
-// longest SM's taps, in microseconds of one 64-channel unit (0.45 at 256 columns, 0.38 below), with the tile-tap averages of
-// shells of 1 k to 40 k voxels; the partial sums at 8 TB/s (they stay in the L2, and the writes run beside the main loop), and 8 us
-// for the second kernel.
-extern "C" int t2sc_plan_wants_tap_groups(t2sc_ctx* ctx, int64_t n_rows, int dtype, int Ci, int Co) {
-  if (!ctx || n_rows <= 0 || Ci <= 0 || Co <= 0 || Co > 2048 || n_rows > (1 << 20) || !conv_umma_supported(dtype, Ci, Co, 128)) return 0;
-  const double sms = ctx->num_sms, items = (double)cdiv_i(n_rows, 128) * conv_umma_slabs(Co), unit = (Co / conv_umma_slabs(Co) > 128 ? 0.45 : 0.38) * ((Ci + 63) / 64);
-  const double whole = unit * (items * 26 / sms > 27 ? items * 26 / sms : 27), apart = unit * (items * 20 / sms > 9 ? items * 20 / sms : 9);
-  return whole > apart + 24e-6 * (double)n_rows * Co / 8 + 8;
-}
-
-extern "C" int t2sc_plan_create_taps(t2sc_ctx* ctx, const uint32_t* nbr, const int32_t* gray, int64_t n_rows, t2sc_plan** out) {
-  T2_REQ(ctx, ctx != nullptr, "null context");
-  T2_REQ(ctx, n_rows < (1ll << 28), "n_rows=%lld", (long long)n_rows);
-  return plan_create(ctx, nbr, gray, n_rows, nullptr, n_rows, 0, 0, 128, out, 0, nullptr, nullptr, true);
 }
 
 extern "C" int t2sc_plan_create(t2sc_ctx* ctx, const uint32_t* nbr, const int32_t* gray, int64_t n_rows,
@@ -434,7 +393,6 @@ extern "C" int t2sc_plan_stats(t2sc_ctx* ctx, t2sc_plan* p, int64_t* tiles, int6
 
 extern "C" int t2sc_plan_order(t2sc_ctx* ctx, t2sc_plan* p, int32_t* order_out) {
   T2_REQ(ctx, ctx && p && (order_out || p->n_out == 0), "null argument");
-  T2_REQ(ctx, !p->tap_groups, "a tap-group plan has an order per group");
   if (p->n_out) T2_CUDA(ctx, cudaMemcpyAsync(order_out, p->order, (size_t)p->n_out * sizeof(int), cudaMemcpyDeviceToDevice, ctx->stream));
   return T2SC_OK;
 }

@@ -75,7 +75,6 @@ struct ConvArgs {
   uint32_t xp_rows[8];      // PEERS: rows of every peer's array
   int dense_rows;           // > 0: no neighbour map at all - a plain row-major GEMM over this many rows (t2sc_linear): tile t is rows
                             // [t * tile rows, ...), its one "tap" reads input row = output row, weights are [Co, 1, Ci]
-  float* partial;           // tap-group plan: the accumulators go here as they are, [entry][Co], and nothing else is done
   const uint2* child_info;  // CHILD form: {row of the first child, set of children} per parent row
   long long* trace;         // diagnostic build only (T2SC_TRACE=file): per-tile timestamps of CTA 0's roles, [role][event][tile < 64]
   int wait_limit;           // bounded waits give up after this many cycles >> WAIT_LIMIT_SHIFT
@@ -99,7 +98,6 @@ static inline void diag_args(ConvArgs& args) {
   args.dense_rows = 0;
   args.perm = nullptr;
   args.child_info = nullptr;
-  args.partial = nullptr;
   args.wait_limit = (int)(WAIT_LIMIT_CYCLES >> WAIT_LIMIT_SHIFT);
 #ifdef T2SC_DIAG
   static const int dbg_skip = [] { const char* e = getenv("T2SC_DEBUG_SKIP"); return e ? atoi(e) : 0; }();
@@ -282,7 +280,7 @@ __device__ __forceinline__ void add_packed32(uint32_t* hp, const uint4* src) {  
 // SKIP: the row may have a skip.  Kernels without one are forms of their own, because its registers and code cost them 8 to 11 % (ConvNeXt
 // block 727,949 x 64: 626 -> 676 us, with both forms in one kernel 694, with kernels of their own 609).
 template <int BN, class T, bool SKIP>
-__device__ __forceinline__ void epilogue_form(const ConvArgs& a, uint32_t taddr, int orow, int cot, const T* bias, const float* gamma, const float* beta, int sp, int ss) {
+__device__ __forceinline__ void epilogue_row(const ConvArgs& a, uint32_t taddr, int orow, int cot, const T* bias, const float* gamma, const float* beta, int sp, int ss) {
   T* y = (T*)a.y;
   const T* res = (const T*)a.ep.residual; const T* skx = (const T*)a.ep.skip_x;
   float mean = 0.f, rstd = 1.f;
@@ -394,24 +392,6 @@ __device__ __forceinline__ void epilogue_form(const ConvArgs& a, uint32_t taddr,
       for (int g = 0; g < 4; g++) yp[g] = make_uint4(hp[g * 4], hp[g * 4 + 1], hp[g * 4 + 2], hp[g * 4 + 3]);
     }
   }
-}
-
-template <int BN, class T, bool SKIP>
-__device__ __forceinline__ void epilogue_row(const ConvArgs& a, uint32_t taddr, int orow, int cot, const T* bias, const float* gamma, const float* beta, int sp, int ss) {
-  if (a.partial) {
-    float* const p = a.partial + (i64)orow * a.Co + cot * BN;
-#pragma unroll 1
-    for (int cc = 0; cc < BN / 32; cc++) {
-      uint32_t r[32]; tc_ld32(taddr + cc * 32, r); tc_wait_ld();
-      if (orow < 0) continue;
-#pragma unroll
-      for (int g = 0; g < 4; g++)       // a row starts on a multiple of 128 bytes
-        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p + cc * 32 + g * 8), "r"(r[g * 8]), "r"(r[g * 8 + 1]), "r"(r[g * 8 + 2]),
-                     "r"(r[g * 8 + 3]), "r"(r[g * 8 + 4]), "r"(r[g * 8 + 5]), "r"(r[g * 8 + 6]), "r"(r[g * 8 + 7]) : "memory");
-    }
-    return;
-  }
-  epilogue_form<BN, T, SKIP>(a, taddr, orow, cot, bias, gamma, beta, sp, ss);
 }
 
 }  // namespace umma

@@ -99,13 +99,11 @@ def spconv_cfg(N: int, Ci: int, Co: int) -> SpConvCfg:
 
 
 class _Plan:
-    def __init__(self, ctx: Context, nbr, gray, src=None, block_rows: int = 0, tile_rows: int = 0, n_own: int = 0, taps: bool = False):
+    def __init__(self, ctx: Context, nbr, gray, src=None, block_rows: int = 0, tile_rows: int = 0, n_own: int = 0):
         self.ctx, self.nbr, self.gray, self.src = ctx, nbr, gray, src     # keep the borrowed tensors alive
         m = src.shape[0] if src is not None else nbr.shape[0]
         h = ctypes.c_void_p()
-        if taps:        # the three planes of taps apart
-            ctx.check(ctx.lib.t2sc_plan_create_taps(ctx.h, _ptr(nbr), _ptr(gray), nbr.shape[0], ctypes.byref(h)))
-        elif n_own:     # one rank of a partitioned scene: interior tiles first, tiles that read halo rows (entries >= n_own) last
+        if n_own:       # one rank of a partitioned scene: interior tiles first, tiles that read halo rows (entries >= n_own) last
             ctx.check(ctx.lib.t2sc_plan_create_split(ctx.h, _ptr(nbr), _ptr(gray), nbr.shape[0], n_own, block_rows, tile_rows, ctypes.byref(h)))
         else:
             ctx.check(ctx.lib.t2sc_plan_create(ctx.h, _ptr(nbr), _ptr(gray), nbr.shape[0], _ptr(src), m, block_rows, tile_rows, ctypes.byref(h)))
@@ -206,17 +204,6 @@ class SpConvCache:
         if tr not in self._plan:
             self._plan[tr] = _Plan(self.ctx, self.nbr, self.gray, None, self._block_rows, tr)
         return self._plan[tr]
-
-    def conv_plan_for(self, Co: int, Ci: int, dtype) -> _Plan:
-        """The schedule subm_conv takes: that of :meth:`plan_for`, or on a small map of wide rows the one with tap groups
-        (t2sc_plan_wants_tap_groups), unless the caller has chosen tiles or runs of its own."""
-        if self._tile_rows or self._block_rows or not self.ctx.lib.t2sc_plan_wants_tap_groups(self.ctx.h, self.N, _DT[dtype], Ci, Co):
-            return self.plan_for(Co, Ci)
-        if self._plan is None:
-            self._plan = {}
-        if "taps" not in self._plan:
-            self._plan["taps"] = _Plan(self.ctx, self.nbr, self.gray, None, 0, 128, taps=True)
-        return self._plan["taps"]
 
     def split_plan_for(self, Co: int, Ci: int, n_own: int) -> _Plan:
         """The schedule of one rank of a partitioned scene whose map indexes owned rows (< n_own) and appended halo rows:
@@ -406,10 +393,7 @@ def subm_conv(x: torch.Tensor, w: torch.Tensor, b: Optional[torch.Tensor], c: Sp
     (``add_``), ``skip=(x_parent, src, rep)`` (``k_add_skip``)."""
     if x.shape[0] != c.N:
         raise T2scError(-1, f"spconv shapes: x has {x.shape[0]} rows, cache has {c.N}")
-    # a shape or type that the checks in _conv refuse goes there with any plan
-    auto = variant == "auto" and w.dim() == 3 and x.dtype in (torch.float16, torch.bfloat16)
-    plan = c.conv_plan_for(w.shape[0], w.shape[2], x.dtype) if auto else c.plan_for(w.shape[0], w.shape[2])
-    return _conv(c.ctx, plan, x, w, b, w.shape[0], ln, act, residual, skip, variant, out)
+    return _conv(c.ctx, c.plan_for(w.shape[0], w.shape[2]), x, w, b, w.shape[0], ln, act, residual, skip, variant, out)
 
 
 @dataclasses.dataclass
