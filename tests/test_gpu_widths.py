@@ -105,3 +105,14 @@ def test_row_pass_over_its_lane_groups(sp, dt, n, C):
     size = v.abs() + beta.double().abs() + want.abs() + r.double().abs()        # the terms of every sum along the way
     assert ((y.double() - want).abs() <= (4 if dt != "f32" else 16) * STEP[dt] * (size + 2.0 ** -6)).all()
     assert torch.equal(sp.row_epilogue(x, ln=(gamma, beta, 1e-6), act="silu", residual=r, out=x), y)        # in place
+
+
+@pytest.mark.parametrize("dt", ["f16", "bf16"])
+@pytest.mark.parametrize("act", ["silu", "gelu", "gelu_tanh"])
+def test_row_pass_gives_the_same_bits_at_any_alignment(sp, dt, act):
+    """A tensor that starts in the middle of 16 bytes takes the element-by-element kernel.  The values reach past the point where
+    exp(-x) leaves fp32's normal range."""
+    n, C = 501, 64
+    x = torch.linspace(-100, 100, n * C, device="cuda").to(TD[dt]).view(n, C)
+    shifted = torch.empty(n * C + 1, dtype=TD[dt], device="cuda")[1:].view(n, C).copy_(x)
+    assert torch.equal(sp.row_epilogue(x, act=act), sp.row_epilogue(shifted, act=act))

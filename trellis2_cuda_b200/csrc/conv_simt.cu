@@ -191,13 +191,6 @@ template <> __device__ __forceinline__ void store8<__nv_bfloat16>(__nv_bfloat16*
   *(uint4*)p = o;
 }
 
-// SiLU of the 16-bit storage types: ex2.approx and rcp.approx, as the tcgen05 kernel's epilogue takes it (about 2^-21 relative,
-// against 2^-11 of the rounding that follows)
-template <class T> __device__ __forceinline__ float act_row(float v, int act) {
-  if constexpr (sizeof(T) == 2) { if (act == T2SC_ACT_SILU) return __fdividef(v, 1.f + __expf(-v)); }
-  return act_apply(v, act);
-}
-
 // The same pass for rows of up to 2048 channels, C % 8 == 0, the row read ONCE in pieces of 8 channels (16-byte loads for the 16-bit
 // types), one per thread, and held in registers through the statistics and the transform: LPR lanes (4, 8, 16, 32) for a row of at most 32,
 // 64, 128, 256 channels, WPR = 2, 4, 8 warps for a longer one.  Bound by HBM when the instructions allow it: 886,752 x 128 fp16 with
@@ -275,7 +268,7 @@ __global__ void __launch_bounds__(256, 4) k_row_epilogue_vec(const T* x, EpiDev 
     if (!live) continue;
     if (ep.act) {
 #pragma unroll
-      for (int i = 0; i < 8; i++) h[i] = rnd<T>(act_row<T>(h[i], ep.act));
+      for (int i = 0; i < 8; i++) h[i] = rnd<T>(act_apply(h[i], ep.act));
     }
     if (res) {
       float r[8]; load8<T>(res + row * C + vi * 8, r);
