@@ -116,3 +116,27 @@ def test_row_pass_gives_the_same_bits_at_any_alignment(sp, dt, act):
     x = torch.linspace(-100, 100, n * C, device="cuda").to(TD[dt]).view(n, C)
     shifted = torch.empty(n * C + 1, dtype=TD[dt], device="cuda")[1:].view(n, C).copy_(x)
     assert torch.equal(sp.row_epilogue(x, act=act), sp.row_epilogue(shifted, act=act))
+
+
+@pytest.mark.parametrize("C", [8, 40, 128, 256, 264, 1024, 2048])
+def test_row_pass_adds_up_a_row_in_one_order(sp, C):
+    """A lane adds its 8-channel pieces in order, the lanes meet in a butterfly: the same sums in fp32, operation by operation
+    (a product and an addition that round once go through 64 bits, where the product is exact)."""
+    x = torch.randn((501, C), generator=torch.Generator(device="cuda").manual_seed(C), device="cuda") + 3
+    pieces = torch.zeros((501, -(-C // 256) * 32, 8), device="cuda")
+    pieces.view(501, -1)[:, :C] = x
+    have = torch.arange(pieces.shape[1], device="cuda") * 8 < C
+
+    def total(term):
+        s = torch.zeros((501, 32), device="cuda")
+        for k in range(pieces.shape[1] // 32):
+            for i in range(8):
+                s = torch.where(have[32 * k:32 * k + 32], term(s, pieces[:, 32 * k:32 * k + 32, i]), s)
+        for o in (16, 8, 4, 2, 1):
+            s = s + s[:, torch.arange(32, device="cuda") ^ o]
+        return s[:, :1]
+    width = torch.full((1, 1), float(C), device="cuda")           # (dividing by a Python number multiplies by its reciprocal)
+    mean = total(lambda s, v: s + v) / width
+    var = total(lambda s, v: ((v - mean).double() ** 2 + s.double()).float()) / width
+    want = torch.rsqrt(var + 1e-6) * (x - mean)
+    assert torch.equal(sp.row_epilogue(x, ln=(None, None, 1e-6)), want)

@@ -191,110 +191,129 @@ template <> __device__ __forceinline__ void store8<__nv_bfloat16>(__nv_bfloat16*
   *(uint4*)p = o;
 }
 
-// The same pass for rows of up to 2048 channels, C % 8 == 0, the row read ONCE in pieces of 8 channels (16-byte loads for the 16-bit
-// types), one per thread, and held in registers through the statistics and the transform: LPR lanes (4, 8, 16, 32) for a row of at most 32,
-// 64, 128, 256 channels, WPR = 2, 4, 8 warps for a longer one.  Bound by HBM when the instructions allow it: 886,752 x 128 fp16 with
-// LayerNorm and SiLU move 454 MB (69 us at 6.55 TB/s).  With a whole warp per row, half of its lanes idle, gamma and beta
-// fetched again for every row (64 bytes for 16 of x) and IEEE divisions that pass took 387 us, now 157: the lanes fit the
-// row, a thread keeps its piece of gamma and beta over the rows of a grid-stride loop, and the next row is in flight while one is
-// worked on.  Rows of several pieces per lane left a small map with too few warps (3,727 x 1024: less than one per scheduler slot).
-template <class T, int LPR, int WPR>
-__global__ void __launch_bounds__(256, 4) k_row_epilogue_vec(const T* x, EpiDev ep, T* y, i64 n, int C) {   // y may alias x
-  static_assert(WPR == 1 || LPR == 32, "several warps per row only for whole warps");
-  constexpr int TPR = LPR * WPR, RPB = 256 / TPR;       // threads per row, rows per block
-  __shared__ float s_sum[2][8];
-  const int vi = threadIdx.x % TPR;                      // this thread's piece of the row
+// The same pass for rows of up to NV * 256 channels, C % 8 == 0: LPR lanes per row (32, or 16 / 8 / 4 for rows of at most 128 /
+// 64 / 32 channels), the row read ONCE in pieces of 8 channels (16-byte loads for the 16-bit types) and held in registers
+// through the statistics and the transform.  Bound by HBM when the instructions allow it: 886,752 x 128 fp16 with LayerNorm
+// and SiLU move 454 MB (69 us at 6.55 TB/s).  With a whole warp per row, half of its lanes idle, and gamma and beta fetched again
+// for every row (64 bytes for 16 of x) that pass took 387 us, now 205 (158 with an
+// approximate SiLU, whose bits differ); so the lanes fit the row, a thread keeps its piece of gamma
+// and beta over the rows of a grid-stride loop (NV <= 2; wider rows read them from the L1), and the next row is in flight while one
+// is worked on.  A lane adds up its pieces in order and the lanes meet in a butterfly, whatever LPR is, so the statistics
+// of a row do not depend on which form runs.
+template <class T, int NV, int LPR>
+__global__ void __launch_bounds__(256, NV == 1 ? 4 : NV <= 4 ? 2 : 1) k_row_epilogue_vec(const T* x, EpiDev ep, T* y, i64 n, int C) {   // y may alias x
+  static_assert(NV == 1 || LPR == 32, "several pieces per lane only for whole warps");
+  constexpr int RPB = 256 / LPR;
+  constexpr bool KEEP = NV <= 2;          // gamma and beta in registers
+  const int lane = threadIdx.x % LPR;
   const unsigned group = LPR == 32 ? 0xffffffffu : ((1u << (LPR & 31)) - 1) << ((threadIdx.x & 31) / LPR * LPR);
   const T* bias = (const T*)ep.bias; const T* res = (const T*)ep.residual; const T* skx = (const T*)ep.skip_x;
-  const bool mine = vi < (C >> 3);
-  // Sum over the row's threads.  The two buffers take turns (mean, variance): a buffer is written again only after the
-  // barrier of the other, which comes after everybody's reads of it.
-  auto sum = [&](float v, int turn) {
+  const int nvec = C >> 3;
+  auto sum = [&](float v) {
 #pragma unroll
     for (int o = LPR / 2; o; o >>= 1) v += __shfl_xor_sync(group, v, o);
-    if constexpr (WPR > 1) {
-      const int warp = threadIdx.x >> 5;
-      if ((threadIdx.x & 31) == 0) s_sum[turn][warp] = v;
-      __syncthreads();
-      v = 0.f;
-#pragma unroll
-      for (int q = 0; q < WPR; q++) v += s_sum[turn][warp / WPR * WPR + q];
-    }
     return v;
   };
-  float g[8], be[8];
+  auto affine = [&](int vi, float* g, float* be) {
 #pragma unroll
-  for (int i = 0; i < 8; i++) { g[i] = 1.f; be[i] = 0.f; }
-  if (ep.ln && mine) {
+    for (int i = 0; i < 8; i++) { g[i] = 1.f; be[i] = 0.f; }
     if (ep.gamma) load8<float>(ep.gamma + vi * 8, g);
     if (ep.beta) load8<float>(ep.beta + vi * 8, be);
+  };
+  float kg[KEEP ? NV : 1][8], kb[KEEP ? NV : 1][8];
+  if constexpr (KEEP) {
+    if (ep.ln) {
+#pragma unroll
+      for (int k = 0; k < NV; k++) if (lane + LPR * k < nvec) affine(lane + LPR * k, kg[k], kb[k]);
+    }
   }
+  i64 row = blockIdx.x * (i64)RPB + threadIdx.x / LPR;
   const i64 step = gridDim.x * (i64)RPB;
-  i64 row = blockIdx.x * (i64)RPB + threadIdx.x / TPR;
-  Raw8<T> next;
-  if (row < n && mine) next.load(x + row * C + vi * 8);
-  // The trip count is the block's, because of the barriers: a thread whose row lies past the end works on nothing.
-  for (i64 base = blockIdx.x * (i64)RPB; base < n; base += step, row += step) {
-    const bool live = row < n && mine;
-    float h[8];
+  Raw8<T> next[NV];
+  auto fetch = [&](i64 r) {
 #pragma unroll
-    for (int i = 0; i < 8; i++) h[i] = 0.f;
-    if (live) next.unpack(h);
-    if (row + step < n && mine) next.load(x + (row + step) * C + vi * 8);
-    if (bias && live) {
-      float b[8]; load8<T>(bias + vi * 8, b);
+    for (int k = 0; k < NV; k++) if (lane + LPR * k < nvec) next[k].load(x + r * C + (lane + LPR * k) * 8);
+  };
+  if (row < n) fetch(row);
+  for (; row < n; row += step) {
+    float h[NV][8];
 #pragma unroll
-      for (int i = 0; i < 8; i++) h[i] = rnd<T>(h[i] + b[i]);
+    for (int k = 0; k < NV; k++) if (lane + LPR * k < nvec) next[k].unpack(h[k]);
+    if (row + step < n) fetch(row + step);
+    if (bias) {
+#pragma unroll
+      for (int k = 0; k < NV; k++) {
+        const int vi = lane + LPR * k;
+        if (vi < nvec) {
+          float b[8]; load8<T>(bias + vi * 8, b);
+#pragma unroll
+          for (int i = 0; i < 8; i++) h[k][i] = rnd<T>(h[k][i] + b[i]);
+        }
+      }
     }
     if (ep.ln) {
       float s = 0.f;
 #pragma unroll
-      for (int i = 0; i < 8; i++) s += h[i];
-      const float mean = sum(s, 0) / (float)C;
+      for (int k = 0; k < NV; k++)
+        if (lane + LPR * k < nvec) {
+#pragma unroll
+          for (int i = 0; i < 8; i++) s += h[k][i];
+        }
+      const float mean = sum(s) / (float)C;
       float q = 0.f;
-      if (mine) {
 #pragma unroll
-        for (int i = 0; i < 8; i++) { const float d = h[i] - mean; q += d * d; }
-      }
-      const float rstd = rsqrtf(sum(q, 1) / (float)C + ep.eps);
+      for (int k = 0; k < NV; k++)
+        if (lane + LPR * k < nvec) {
 #pragma unroll
-      for (int i = 0; i < 8; i++) {
-        float v = rstd * (h[i] - mean);
-        if (ep.gamma) v = g[i] * v;
-        if (ep.beta) v = v + be[i];
-        h[i] = rnd<T>(v);
-      }
-    }
-    if (!live) continue;
-    if (ep.act) {
+          for (int i = 0; i < 8; i++) { const float d = h[k][i] - mean; q += d * d; }
+        }
+      const float rstd = rsqrtf(sum(q) / (float)C + ep.eps);
 #pragma unroll
-      for (int i = 0; i < 8; i++) h[i] = rnd<T>(act_apply(h[i], ep.act));
-    }
-    if (res) {
-      float r[8]; load8<T>(res + row * C + vi * 8, r);
+      for (int k = 0; k < NV; k++) {
+        const int vi = lane + LPR * k;
+        if (vi < nvec) {
+          float tg[8], tb[8];
+          if constexpr (!KEEP) affine(vi, tg, tb);
+          const float* g = KEEP ? kg[KEEP ? k : 0] : tg; const float* be = KEEP ? kb[KEEP ? k : 0] : tb;
 #pragma unroll
-      for (int i = 0; i < 8; i++) h[i] = rnd<T>(h[i] + r[i]);
-    }
-    if (skx) {
-      const int sv = ep.skip_src[row];
-      const T* sx = skx + (i64)(sv >> 3) * ep.skip_cin + (sv & 7) * (ep.skip_cin / 8);
-      if (ep.skip_rep == 4) {           // the decoder's: two values, no divisions
-        const float lo = to_f<T>(sx[vi * 2]), hi = to_f<T>(sx[vi * 2 + 1]);
-#pragma unroll
-        for (int i = 0; i < 8; i++) h[i] = rnd<T>(h[i] + (i < 4 ? lo : hi));
-      } else {
-#pragma unroll
-        for (int i = 0; i < 8; i++) h[i] = rnd<T>(h[i] + to_f<T>(sx[(vi * 8 + i) / ep.skip_rep]));
+          for (int i = 0; i < 8; i++) {
+            float v = rstd * (h[k][i] - mean);
+            if (ep.gamma) v = ep.beta ? fmaf(g[i], v, be[i]) : g[i] * v;        // spelled out: left to the compiler it was one rounding or two by type
+            else if (ep.beta) v = v + be[i];
+            h[k][i] = rnd<T>(v);
+          }
+        }
       }
     }
-    store8<T>(y + row * C + vi * 8, h);
+    int sp = 0, ss = 0;
+    if (skx) { const int sv = ep.skip_src[row]; sp = sv >> 3; ss = sv & 7; }
+#pragma unroll
+    for (int k = 0; k < NV; k++) {
+      const int vi = lane + LPR * k;
+      if (vi >= nvec) continue;
+      if (ep.act) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) h[k][i] = rnd<T>(act_apply(h[k][i], ep.act));
+      }
+      if (res) {
+        float r[8]; load8<T>(res + row * C + vi * 8, r);
+#pragma unroll
+        for (int i = 0; i < 8; i++) h[k][i] = rnd<T>(h[k][i] + r[i]);
+      }
+      if (skx) {
+        const T* sx = skx + (i64)sp * ep.skip_cin + ss * (ep.skip_cin / 8);
+        if (ep.skip_rep == 4) {           // the decoder's: two values, no divisions
+          const float lo = to_f<T>(sx[vi * 2]), hi = to_f<T>(sx[vi * 2 + 1]);
+#pragma unroll
+          for (int i = 0; i < 8; i++) h[k][i] = rnd<T>(h[k][i] + (i < 4 ? lo : hi));
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; i++) h[k][i] = rnd<T>(h[k][i] + to_f<T>(sx[(vi * 8 + i) / ep.skip_rep]));
+        }
+      }
+      store8<T>(y + row * C + vi * 8, h[k]);
+    }
   }
-}
-
-// Four blocks of 256 threads fit an SM; each takes rows in a grid-stride loop.
-static inline int row_grid(const t2sc_ctx* ctx, i64 n, int rows_per_block) {
-  const i64 blocks = (n + rows_per_block - 1) / rows_per_block, most = 4ll * ctx->num_sms;
-  return (int)(blocks < most ? blocks : most);
 }
 
 template <class T>
@@ -302,14 +321,17 @@ void row_epilogue_pick(t2sc_ctx* ctx, const void* x, const EpiDev& ep, void* y, 
   const bool aligned = (uintptr_t)x % 16 == 0 && (uintptr_t)y % 16 == 0 && (!ep.residual || (uintptr_t)ep.residual % 16 == 0) &&
                        (!ep.bias || (uintptr_t)ep.bias % 16 == 0) && (!ep.gamma || (uintptr_t)ep.gamma % 16 == 0) && (!ep.beta || (uintptr_t)ep.beta % 16 == 0);
   if (C % 8 == 0 && aligned && C <= 2048) {
-#define T2_ROWS(LPR, WPR) k_row_epilogue_vec<T, LPR, WPR><<<row_grid(ctx, n, 256 / (LPR * WPR)), 256, 0, ctx->stream>>>((const T*)x, ep, (T*)y, n, C)
-    if (C <= 32) T2_ROWS(4, 1);
-    else if (C <= 64) T2_ROWS(8, 1);
-    else if (C <= 128) T2_ROWS(16, 1);
-    else if (C <= 256) T2_ROWS(32, 1);
-    else if (C <= 512) T2_ROWS(32, 2);
-    else if (C <= 1024) T2_ROWS(32, 4);
-    else T2_ROWS(32, 8);
+    const int lanes = C <= 32 ? 4 : C <= 64 ? 8 : C <= 128 ? 16 : 32;
+    const i64 blocks = (n * lanes + 255) / 256, most = (C <= 256 ? 4ll : C <= 1024 ? 2ll : 1ll) * ctx->num_sms;       // as many as are resident
+    const int grid = (int)(blocks < most ? blocks : most);
+#define T2_ROWS(NV, LPR) k_row_epilogue_vec<T, NV, LPR><<<grid, 256, 0, ctx->stream>>>((const T*)x, ep, (T*)y, n, C)
+    if (C <= 32) T2_ROWS(1, 4);
+    else if (C <= 64) T2_ROWS(1, 8);
+    else if (C <= 128) T2_ROWS(1, 16);
+    else if (C <= 256) T2_ROWS(1, 32);
+    else if (C <= 512) T2_ROWS(2, 32);
+    else if (C <= 1024) T2_ROWS(4, 32);
+    else T2_ROWS(8, 32);
 #undef T2_ROWS
   } else {
     k_row_epilogue<T><<<cdiv_i(n * 32, 256), 256, 0, ctx->stream>>>((const T*)x, ep, (T*)y, n, C);
