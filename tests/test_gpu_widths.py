@@ -140,3 +140,18 @@ def test_row_pass_adds_up_a_row_in_one_order(sp, C):
     var = total(lambda s, v: ((v - mean).double() ** 2 + s.double()).float()) / width
     want = torch.rsqrt(var + 1e-6) * (x - mean)
     assert torch.equal(sp.row_epilogue(x, ln=(None, None, 1e-6)), want)
+
+
+@pytest.mark.parametrize("dt", ["f16", "bf16"])
+@pytest.mark.parametrize("Co", [96, 160, 192, 224])
+def test_layer_norm_over_widths_between_powers_of_two(sp, dt, Co):
+    """Two passes over the row, as for any width that the epilogue does not hold: a first value far from the others must not cost the
+    variance its bits.  The fused call gives the bits of the conv (the Linear layer) and then the row pass."""
+    c, x, w, b = scene(700, 64, Co, dt)
+    b[0] = 3000
+    xd, wd, bd = (torch.from_numpy(t).cuda().to(TD[dt]) for t in (x, w, b))
+    ln = (torch.rand(Co, device="cuda") + 0.5, torch.randn(Co, device="cuda"), 1e-6)
+    cache = sp.build_neighbors(torch.from_numpy(c).cuda())
+    assert torch.equal(sp.subm_conv(xd, wd, bd, cache, ln=ln, act="silu"), sp.row_epilogue(sp.subm_conv(xd, wd, bd, cache), ln=ln, act="silu"))
+    wl = wd[:, 0].contiguous()
+    assert torch.equal(sp.linear(xd, wl, bd, ln=ln), sp.row_epilogue(sp.linear(xd, wl, bd), ln=ln))

@@ -134,10 +134,10 @@ int conv_dispatch(t2sc_ctx* ctx, t2sc_plan* plan, const void* x, const void* w, 
   if (variant == T2SC_VARIANT_UMMA && !(umma_ok && Ci % 64 == 0))
     return t2sc_fail(ctx, T2SC_ERR_UNSUPPORTED, "tcgen05 variant needs fp16/bf16, Ci %% 64 == 0, Co %% 32 == 0 (Ci=%d Co=%d dtype=%d)", Ci, Co, dtype);
   bool use_umma = variant == T2SC_VARIANT_UMMA || variant == T2SC_VARIANT_UMMA_PAIR || (variant == T2SC_VARIANT_AUTO && umma_ok);
-  // LayerNorm needs the whole output row in one accumulator: fused on the tcgen05 path when Co is one of its tile widths
-  // (multiples of 32 up to 256; for one part of a plan, and for 256-row tiles, the powers of two), else conv + bias first and LayerNorm ->
-  // activation -> residual -> skip in a row pass
-  bool fuse_all = use_umma && (!e.ln || conv_umma_fuses_ln(Co, part != T2SC_PART_ALL || plan->tile_rows != 128));
+  // LayerNorm needs the whole output row in one accumulator: fused on the tcgen05 path when Co is 32, 64, 128 or 256, else conv + bias
+  // first and LayerNorm -> activation -> residual -> skip in a row pass.  (96, 160, 192 and 224 fit one accumulator too, but the epilogue
+  // reads it once for both sums, which costs bits where a row's first value lies far from the others; the row pass goes twice.)
+  bool fuse_all = use_umma && (!e.ln || conv_umma_fuses_ln(Co));
   if (variant == T2SC_VARIANT_UMMA_PAIR) {
     if (!conv_umma2_supported(plan, dtype, Ci, Co, e))
       return t2sc_fail(ctx, T2SC_ERR_UNSUPPORTED, "two-SM tcgen05 variant needs fp16/bf16, a 256-row plan, Ci %% 64 == 0, Co %% 256 == 0 (Ci=%d Co=%d tile_rows=%d)", Ci, Co, plan->tile_rows);
@@ -189,7 +189,7 @@ extern "C" int t2sc_subm_conv_peers_part(t2sc_ctx* ctx, t2sc_plan* plan, const u
   T2_REQ(ctx, w && y, "null tensor");
   for (int r = 0; r < n_peers; r++) T2_REQ(ctx, x_peers[r] && (uintptr_t)x_peers[r] % 16 == 0, "peer array %d is null or not 16-byte aligned", r);
   EpiDev e = epi_dev(ep);
-  if (!conv_umma_supported(dtype, Ci, Co, 256) || (e.ln && !conv_umma_fuses_ln(Co, true)) || plan->src)
+  if (!conv_umma_supported(dtype, Ci, Co, 256) || (e.ln && !conv_umma_fuses_ln(Co)) || plan->src)
     return t2sc_fail(ctx, T2SC_ERR_UNSUPPORTED, "peer conv needs a submanifold plan, fp16/bf16, Ci %% 64 == 0, Co %% 32 == 0, LayerNorm only for Co in {32,64,128,256} (Ci=%d Co=%d dtype=%d)", Ci, Co, dtype);
   return conv_umma_launch(ctx, plan, x_peers[self_rank], w, Co, e, y, dtype, rows_peers[self_rank], Ci, Co, part, x_peers, rows_peers, n_peers,
                           self_rank, peer_nbr);

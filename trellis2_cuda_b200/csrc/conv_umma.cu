@@ -577,7 +577,7 @@ bool conv_umma_supported(int dtype, int Ci, int Co, int tile_rows) {
   return (dtype == T2SC_F16 || dtype == T2SC_BF16) && Ci % (tile_rows == TILE_M ? KCH / 2 : KCH) == 0 && Co % 32 == 0;
 }
 
-bool conv_umma_fuses_ln(int Co, bool pow2) { return pick_bn(Co, pow2) == Co; }
+bool conv_umma_fuses_ln(int Co) { return pick_bn(Co, true) == Co; }
 
 int conv_umma_launch(t2sc_ctx* ctx, const t2sc_plan* plan, const void* x, const void* w, i64 w_rows, const EpiDev& ep, void* y,
                      int dtype, i64 n_in, int Ci, int Co, int part, const void* const* x_peers, const int64_t* rows_peers, int n_peers,
