@@ -91,3 +91,17 @@ def test_fused_skip_is_conv_then_add(sp, Cin, Co, n):
     w = (torch.randn((Co, 27, 64), generator=g, device="cuda") * 0.03).to(torch.bfloat16)
     for kw in (dict(), dict(ln=(None, None, 1e-6))):
         assert torch.equal(sp.subm_conv(x, w, None, cache, skip=(parent, src, rep), **kw), sp.add_skip(sp.subm_conv(x, w, None, cache, **kw), parent, src, rep))
+
+
+def test_two_sm_variant_of_the_subdivision_conv(sp):
+    """It takes 256-row tiles, which the other variants of a subdivided level do not: the same bits from either."""
+    g = torch.Generator(device="cuda").manual_seed(3)
+    n, Ci, Cc = 700, 128, 256
+    level = sp.subdivide(sp.build_neighbors(torch.from_numpy(cube(n, 8, 5)).cuda()), (torch.rand((n, 8), generator=g, device="cuda") < 0.5).to(torch.uint8))
+    x = torch.randn((n, Ci), generator=g, device="cuda").to(torch.bfloat16)
+    w = (torch.randn((8 * Cc, 27, Ci), generator=g, device="cuda") * 0.03).to(torch.bfloat16)
+    b = torch.randn(8 * Cc, generator=g, device="cuda").to(torch.bfloat16)
+    for kw in (dict(), dict(ln=(None, None, 1e-6), act="silu")):
+        y = sp.subdiv_conv(x, w, b, level, variant="umma_pair", **kw)
+        sp.context().device_status()
+        assert torch.equal(y, sp.subdiv_conv(x, w, b, level, variant="umma", **kw))

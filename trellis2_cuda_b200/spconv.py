@@ -417,17 +417,16 @@ class Level:
                 and x.dtype in (torch.float16, torch.bfloat16) and x.shape[1] % 64 == 0
                 and self.parent._tile_rows_for(256, x.shape[1]) == 128 and self.src.shape[0] > 3 * self.parent.N)
 
-    def up_plan_for(self, Cc: int) -> _Plan:
-        """Schedule of the subdivision conv into Cc child channels: 128-row tiles, whose finer masks and shorter items fill the chip
+    def up_plan_for(self, Cc: int, tile_rows: int = 128) -> _Plan:
+        """Schedule of the subdivision conv into Cc child channels: 128-row tiles (256 for the two-SM variant, which takes no others), whose finer masks and shorter items fill the chip
         on small levels and whose narrow forms run two CTAs per SM (whole up block against 256-row tiles: 1,500 parents,
         1024 -> 512: 664 -> 450 us; 12,000: 1718 -> 1495; 8,000, 512 -> 256: 611 -> 525; 30,000, 256 -> 128: 558 -> 518; 150,000:
         1802 -> 1690; 250,000: 2794 -> 2785)."""
-        tr = 128
         if self._up_plans is None:
             self._up_plans = {}
-        if tr not in self._up_plans:
-            self._up_plans[tr] = _Plan(self.parent.ctx, self.parent.nbr, self.parent.gray, self.src, 0, tr)
-        return self._up_plans[tr]
+        if tile_rows not in self._up_plans:
+            self._up_plans[tile_rows] = _Plan(self.parent.ctx, self.parent.nbr, self.parent.gray, self.src, 0, tile_rows)
+        return self._up_plans[tile_rows]
 
     @property
     def up_plan(self) -> _Plan:
@@ -478,7 +477,8 @@ def subdiv_conv(x: torch.Tensor, w: torch.Tensor, b: Optional[torch.Tensor], lev
         raise T2scError(-1, f"spconv shapes: x has {x.shape[0]} rows, parent cache has {level.parent.N}")
     if variant == "auto" and level._from_parents(x, w.shape[0] // 8):
         return _conv_parents(level, x, w, b, ln, act, out)
-    return _conv(level.parent.ctx, level.up_plan_for(w.shape[0] // 8), x, w, b, w.shape[0] // 8, ln, act, None, None, variant, out)
+    plan = level.up_plan_for(w.shape[0] // 8, 256 if variant == "umma_pair" else 128)
+    return _conv(level.parent.ctx, plan, x, w, b, w.shape[0] // 8, ln, act, None, None, variant, out)
 
 
 def gather_rows(x: torch.Tensor, src: torch.Tensor, C: int, out: Optional[torch.Tensor] = None) -> torch.Tensor:
