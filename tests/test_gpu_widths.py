@@ -155,3 +155,16 @@ def test_layer_norm_over_widths_between_powers_of_two(sp, dt, Co):
     assert torch.equal(sp.subm_conv(xd, wd, bd, cache, ln=ln, act="silu"), sp.row_epilogue(sp.subm_conv(xd, wd, bd, cache), ln=ln, act="silu"))
     wl = wd[:, 0].contiguous()
     assert torch.equal(sp.linear(xd, wl, bd, ln=ln), sp.row_epilogue(sp.linear(xd, wl, bd), ln=ln))
+
+
+@pytest.mark.parametrize("Co", [64, 130])
+def test_fp32_sums_do_not_depend_on_the_rows_beside_them(sp, Co):
+    """The first rows of a map by themselves, at numbers of rows that split the taps over 8, 4 and 1 CTAs: the bits of the whole."""
+    n, Ci = 30000, 64
+    c, x, w, b = scene(n, Ci, Co, "f32")
+    x, w, b = (torch.from_numpy(t).cuda() for t in (x, w, b))
+    whole = sp.build_neighbors(torch.from_numpy(c).cuda())
+    want = sp.subm_conv(x, w, b, whole)
+    for m in (1, 700, 2500, 6000, 9000, 15000, 28000):
+        part = sp.cache_from_map(whole.coords[:m], whole.nbr[:m].contiguous(), whole.gray[:m].contiguous())
+        assert torch.equal(sp.subm_conv_local(x, w, b, part), want[:m]), m

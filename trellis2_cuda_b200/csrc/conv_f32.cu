@@ -11,9 +11,11 @@
 // with fma.rn.f32x2, which needs no operand to be packed or duplicated: 12 shared loads per 64 FMA instructions.
 //
 // A small map has too few tiles for the 148 SMs (14,534 rows: 228 tiles of 64), so the taps of a tile are split over a
-// cluster of S = 2, 4 or 8 CTAs; the partial sums meet in distributed shared memory and are added in rank order, so the
-// result depends neither on timing nor on the plan (S comes from the number of rows).  S grows until there are three CTAs per SM, as many as fit: below that the chip idles,
-// above it the reduction costs more than it gives.
+// cluster of S = 4 or 8 CTAs, whose sums meet in distributed shared memory.  S grows until there are three CTAs per SM, as many as
+// fit: below that the chip idles, above it the reduction costs more than it gives.
+// Every S adds in one order, so a row's bits depend neither on timing nor on the plan nor on how many rows come with it (a scene
+// and its parts give the same): tap v belongs to group v % 8, a group is summed by itself, and the eight sums are added in order.
+// With S = 1 a CTA adds them up as it goes, with S = 4 it hands on two, with S = 8 one; S = 2 would have to keep four apart.
 #include "common.cuh"
 #include <cooperative_groups.h>
 
@@ -24,8 +26,10 @@ namespace {
 constexpr int FM = 64, FN = 64, FK = 32, FPITCH = FK + 4, FSTAGES = 3, FTHREADS = 128;
 constexpr int F_OPERAND = FM * FPITCH;                          // floats of one operand of one stage (FM == FN)
 constexpr int F_SMEM = FSTAGES * 2 * F_OPERAND * (int)sizeof(float);
-constexpr int FRED = FN + 4;                                    // row pitch of the partial sums, which reuse the ring
-static_assert(FM * FRED <= FSTAGES * 2 * F_OPERAND, "the partial sums fit in the ring");
+constexpr int FRED = FN + 4;                                    // row pitch of the groups' sums, which reuse the ring
+static_assert(2 * FM * FRED <= FSTAGES * 2 * F_OPERAND, "the sums of two groups fit in the ring");
+constexpr int FGROUPS = 8;
+constexpr uint32_t FGROUP0 = 0x01010101u;                       // taps of group 0; those of group g are FGROUP0 << g
 constexpr uint32_t F_ABSENT = 0x80000000u;
 
 __device__ __forceinline__ void f_copy16(float* dst, const float* src, uint32_t bytes) {       // bytes = 0: zero-fill, src is not read
@@ -35,10 +39,13 @@ __device__ __forceinline__ void fma2(unsigned long long& d, unsigned long long a
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
 }
 
+template <int S>
 __global__ void __launch_bounds__(FTHREADS, 3) k_conv_f32(const float* __restrict__ x, const float* __restrict__ w, const uint32_t* __restrict__ tnbr,
                                                           const int* __restrict__ order, const PlanTile* __restrict__ tiles, const int* __restrict__ perm,
                                                           const int* __restrict__ tile_lo, const int* __restrict__ tile_hi, EpiDev ep,
-                                                          float* __restrict__ y, int Ci, int Co, int tile_rows, int S) {
+                                                          float* __restrict__ y, int Ci, int Co, int tile_rows) {
+  constexpr int PER = FGROUPS / S, SUMS = S == 1 ? 1 : PER;      // groups of this CTA, and how many sums it hands on
+  static_assert(SUMS <= 2, "a CTA of a cluster has one or two groups");
   extern __shared__ __align__(16) float ring[];
   __shared__ uint32_t s_idx[27 * FM];
   __shared__ uint32_t s_mask;
@@ -64,9 +71,11 @@ __global__ void __launch_bounds__(FTHREADS, 3) k_conv_f32(const float* __restric
     if (__any_sync(0xffffffffu, s_idx[v * FM + lane] != F_ABSENT || s_idx[v * FM + 32 + lane] != F_ABSENT)) have |= 1u << v;
   if (lane == 0 && have) atomicOr(&s_mask, have);
   __syncthreads();
-  // this CTA's taps: every S-th of the 27, not a share of the present ones, so that a row's sums do not depend on the rows it shares a tile with
-  const uint32_t mask = s_mask & ((S == 1 ? 0x7ffffffu : S == 2 ? 0x5555555u : S == 4 ? 0x1111111u : 0x1010101u) << rank);
-  if (tid < 27 && (mask >> tid & 1)) s_tap[__popc(mask & ((1u << tid) - 1))] = tid;
+  // this CTA's taps, group by group
+  const int g0 = rank * PER;
+  const uint32_t mask = s_mask & (FGROUP0 * ((1u << PER) - 1) << g0);
+  if (tid < 27 && (mask >> tid & 1))
+    s_tap[__popc(mask & FGROUP0 * ((1u << tid % FGROUPS) - 1)) + __popc(mask & FGROUP0 << tid % FGROUPS & ((1u << tid) - 1))] = tid;
   __syncthreads();
   const int nchunk = Ci / FK, steps = __popc(mask) * nchunk;
 
@@ -105,38 +114,58 @@ __global__ void __launch_bounds__(FTHREADS, 3) k_conv_f32(const float* __restric
     if (s < steps) fetch();
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
-  int stage = 0;
-  for (int it = 0; it < steps; it++) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(FSTAGES - 2) : "memory");
-    __syncthreads();                       // this step's copies have landed for everybody, and everybody has read the stage that is filled next
-    if (it + FSTAGES - 1 < steps) fetch();
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    const float* A = ring + stage * 2 * F_OPERAND + r0 * FPITCH;
-    const float* B = ring + stage * 2 * F_OPERAND + F_OPERAND + c0 * FPITCH;
+  float tot[8][4];                         // the sum of the groups before this one (S = 1), or of this CTA's first group
 #pragma unroll
-    for (int k = 0; k < FK; k += 4) {
-      ulonglong2 b[4];
+  for (int i = 0; i < 8; i++)
 #pragma unroll
-      for (int j = 0; j < 4; j++) b[j] = *(const ulonglong2*)(B + 8 * j * FPITCH + k);
+    for (int j = 0; j < 4; j++) tot[i][j] = 0.f;
+  int stage = 0, it = 0;
+#pragma unroll 1
+  for (int g = 0; g < PER; g++) {
+    for (const int end = it + __popc(mask & FGROUP0 << (g0 + g)) * nchunk; it < end; it++) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(FSTAGES - 2) : "memory");
+      __syncthreads();                       // this step's copies have landed for everybody, and everybody has read the stage that is filled next
+      if (it + FSTAGES - 1 < steps) fetch();
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      const float* A = ring + stage * 2 * F_OPERAND + r0 * FPITCH;
+      const float* B = ring + stage * 2 * F_OPERAND + F_OPERAND + c0 * FPITCH;
 #pragma unroll
-      for (int i = 0; i < 8; i++) {
-        const ulonglong2 a = *(const ulonglong2*)(A + 4 * i * FPITCH + k);
+      for (int k = 0; k < FK; k += 4) {
+        ulonglong2 b[4];
 #pragma unroll
-        for (int j = 0; j < 4; j++) { fma2(acc[i][j], a.x, b[j].x); fma2(acc[i][j], a.y, b[j].y); }
+        for (int j = 0; j < 4; j++) b[j] = *(const ulonglong2*)(B + 8 * j * FPITCH + k);
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+          const ulonglong2 a = *(const ulonglong2*)(A + 4 * i * FPITCH + k);
+#pragma unroll
+          for (int j = 0; j < 4; j++) { fma2(acc[i][j], a.x, b[j].x); fma2(acc[i][j], a.y, b[j].y); }
+        }
       }
+      if (++stage == FSTAGES) stage = 0;
     }
-    if (++stage == FSTAGES) stage = 0;
+    if (S == 1 || g + 1 < PER) {
+#pragma unroll
+      for (int i = 0; i < 8; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          const float2 p = *reinterpret_cast<const float2*>(&acc[i][j]);
+          tot[i][j] += p.x + p.y;
+          acc[i][j] = 0ull;
+        }
+    }
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
-  // partial sums into the ring, then every CTA of the cluster finishes its share of the rows
+  // the sums into the ring, then every CTA of the cluster finishes its share of the rows
   float* const red = ring;
 #pragma unroll
   for (int i = 0; i < 8; i++)
 #pragma unroll
     for (int j = 0; j < 4; j++) {
       const float2 p = *reinterpret_cast<const float2*>(&acc[i][j]);
-      red[(r0 + 4 * i) * FRED + c0 + 8 * j] = p.x + p.y;
+      float* const at = red + (r0 + 4 * i) * FRED + c0 + 8 * j;
+      if (PER > 1) at[0] = tot[i][j];
+      if (S > 1) at[(SUMS - 1) * FM * FRED] = p.x + p.y;
     }
   cg::cluster_group cluster = cg::this_cluster();
   if (S > 1) cluster.sync(); else __syncthreads();
@@ -148,8 +177,11 @@ __global__ void __launch_bounds__(FTHREADS, 3) k_conv_f32(const float* __restric
     float h[4] = {0.f, 0.f, 0.f, 0.f};
     for (int q = 0; q < S; q++) {
       const float* from = S > 1 ? cluster.map_shared_rank(red, q) : red;
-      const float4 p = *(const float4*)(from + r * FRED + c);
-      h[0] += p.x; h[1] += p.y; h[2] += p.z; h[3] += p.w;
+#pragma unroll
+      for (int k = 0; k < SUMS; k++) {
+        const float4 p = *(const float4*)(from + (k * FM + r) * FRED + c);
+        h[0] += p.x; h[1] += p.y; h[2] += p.z; h[3] += p.w;
+      }
     }
     const int orow = order[tile.start + sub * FM + r];
     int sp = 0, ss = 0;
@@ -168,7 +200,7 @@ __global__ void __launch_bounds__(FTHREADS, 3) k_conv_f32(const float* __restric
     else
       for (int q = 0; q < n; q++) yp[q] = h[q];
   }
-  if (S > 1) cluster.sync();               // nobody leaves while a peer reads its partial sums
+  if (S > 1) cluster.sync();               // nobody leaves while a peer reads its sums
 }
 
 }  // namespace
@@ -179,23 +211,24 @@ int conv_f32_launch(t2sc_ctx* ctx, const t2sc_plan* plan, const float* x, const 
   if (rc != T2SC_OK) return rc;
   const TilePart tp = tile_part(plan, part);
   T2_CUDA(ctx, cudaSetDevice(ctx->device));
-  static bool attr_set[64] = {};
-  if (ctx->device >= 64 || !attr_set[ctx->device]) {
-    T2_CUDA(ctx, cudaFuncSetAttribute(k_conv_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, F_SMEM));
-    if (ctx->device < 64) attr_set[ctx->device] = true;
-  }
   const i64 parts = plan->max_tiles * (plan->tile_rows / FM);
   const int ny = cdiv_i(Co, FN);
-  int S = 1;
-  while (S < 8 && cdiv_i(plan->n_out, FM) * (i64)ny * S < 3 * ctx->num_sms) S *= 2;
+  const i64 whole = cdiv_i(plan->n_out, FM) * (i64)ny, places = 3ll * ctx->num_sms;
+  const int S = whole >= places ? 1 : 4 * whole >= places ? 4 : 8;
+  const auto kernel = S == 1 ? k_conv_f32<1> : S == 4 ? k_conv_f32<4> : k_conv_f32<8>;
+  static bool attr_set[64][9] = {};
+  if (ctx->device >= 64 || !attr_set[ctx->device][S]) {
+    T2_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, F_SMEM));
+    if (ctx->device < 64) attr_set[ctx->device][S] = true;
+  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(parts * S), (unsigned)ny); cfg.blockDim = dim3(FTHREADS); cfg.dynamicSmemBytes = F_SMEM; cfg.stream = ctx->stream;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = S; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
   cfg.attrs = at; cfg.numAttrs = S > 1 ? 1 : 0;
-  T2_CUDA(ctx, cudaLaunchKernelEx(&cfg, k_conv_f32, x, w, (const uint32_t*)plan->tnbr, (const int*)plan->order, (const PlanTile*)plan->tiles,
-                                  (const int*)(plan->balanced ? plan->perm : nullptr), tp.lo, tp.hi, ep, y, Ci, Co, plan->tile_rows, S));
+  T2_CUDA(ctx, cudaLaunchKernelEx(&cfg, kernel, x, w, (const uint32_t*)plan->tnbr, (const int*)plan->order, (const PlanTile*)plan->tiles,
+                                  (const int*)(plan->balanced ? plan->perm : nullptr), tp.lo, tp.hi, ep, y, Ci, Co, plan->tile_rows));
   ctx->launches++;
   return T2SC_OK;
 }
