@@ -105,3 +105,23 @@ def test_two_sm_variant_of_the_subdivision_conv(sp):
         y = sp.subdiv_conv(x, w, b, level, variant="umma_pair", **kw)
         sp.context().device_status()
         assert torch.equal(y, sp.subdiv_conv(x, w, b, level, variant="umma", **kw))
+
+
+@pytest.mark.parametrize("derived", [True, False])
+def test_a_level_belongs_to_the_stream_it_is_made_on(sp, derived):
+    """Convs over the children run on the stream that was current when the level was made, whether their map was read off the parents' or
+    hashed, and the parent's stream has filled it by then."""
+    c = torch.from_numpy(cube(3000, 16, 7)).cuda()
+    sub = torch.ones((3000, 8), dtype=torch.uint8, device="cuda")
+    parent = sp.build_neighbors(c)
+    if not derived:
+        parent = sp.cache_from_map(c, parent.nbr, parent.gray)
+    want = sp.build_neighbors(sp.subdivide(parent, sub).coords, want_sorted=False)
+    torch.cuda.synchronize()
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        level = sp.subdivide(parent, sub)
+        assert level.nb.ctx is sp.context() and level.nb.ctx is not parent.ctx
+        same = torch.equal(level.nb.nbr, want.nbr) and torch.equal(level.nb.gray, want.gray)
+    torch.cuda.synchronize()
+    assert same and (level._info is not None) == derived

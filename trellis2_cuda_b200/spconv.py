@@ -32,6 +32,7 @@ class Context:
     def __init__(self, device: int, stream_handle: int):
         self.lib = _lib.load()
         self.device = device
+        self.stream = torch.cuda.ExternalStream(stream_handle, device) if stream_handle else torch.cuda.default_stream(device)
         h = ctypes.c_void_p()
         rc = self.lib.t2sc_ctx_create(device, ctypes.c_void_p(stream_handle or 1), ctypes.byref(h))
         if rc:
@@ -441,7 +442,18 @@ def subdivide(parent: SpConvCache, sub: torch.Tensor, want_sorted: bool = False)
     n = parent.N
     if sub.shape != (n, 8) or sub.dtype not in (torch.float16, torch.bfloat16, torch.uint8):
         raise T2scError(-1, f"sub must be [{n},8] fp16/bf16/uint8, got {tuple(sub.shape)} {sub.dtype}")
-    ctx = parent.ctx
+    # The maps are made on the parent's stream.  The level belongs to the current one, as any cache does: where the two differ each waits
+    # for the other, and the parent's stream is named to the allocator for every tensor that it writes.
+    ctx, here = parent.ctx, context(sub.device)
+    if here is not ctx:
+        ctx.stream.wait_stream(here.stream)
+
+    def handed_over(*tensors):
+        if here is not ctx:
+            here.stream.wait_stream(ctx.stream)
+            for t in tensors:
+                if t is not None:
+                    t.record_stream(ctx.stream)
     off = torch.empty(n + 1, dtype=torch.int32, device=sub.device)
     m = ctypes.c_int64(0)
     extent = parent._map_extent()
@@ -458,12 +470,14 @@ def subdivide(parent: SpConvCache, sub: torch.Tensor, want_sorted: bool = False)
         ctx.check(ctx.lib.t2sc_subdivide_emit_info(ctx.h, _ptr(sub), _DT[sub.dtype], _ptr(parent.coords), _ptr(off), n, _ptr(coords), _ptr(src), _ptr(info)))
     known = (info, src, _version(src)) if info is not None and m.value and _version(src) is not None else None
     if not (whole.value and m.value) or want_sorted:
+        handed_over(sub, off, info, coords, src)
         return Level(coords, src, build_neighbors(coords, 4096, 4096, 4096, want_sorted=want_sorted), parent, None, known)
     # every parent is in the grid and alone at its place: the children's map follows from the parents'
     nbr = torch.empty((m.value, 27), dtype=torch.int32, device=sub.device)
     gray = torch.empty(m.value, dtype=torch.int32, device=sub.device)
     ctx.check(ctx.lib.t2sc_subdivide_neighbors(ctx.h, _ptr(parent.nbr), _ptr(info), n, _ptr(nbr), _ptr(gray)))
-    return Level(coords, src, SpConvCache(ctx, coords, nbr, gray, None)._built((4096, 4096, 4096)), parent, None, known)
+    handed_over(sub, off, info, coords, src, nbr, gray)
+    return Level(coords, src, SpConvCache(here, coords, nbr, gray, None)._built((4096, 4096, 4096)), parent, None, known)
 
 
 def subdiv_conv(x: torch.Tensor, w: torch.Tensor, b: Optional[torch.Tensor], level: Level, *, ln=None, act=None,
