@@ -168,3 +168,18 @@ def test_fp32_sums_do_not_depend_on_the_rows_beside_them(sp, Co):
     for m in (1, 700, 2500, 6000, 9000, 15000, 28000):
         part = sp.cache_from_map(whole.coords[:m], whole.nbr[:m].contiguous(), whole.gray[:m].contiguous())
         assert torch.equal(sp.subm_conv_local(x, w, b, part), want[:m]), m
+
+
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs a second GPU")
+def test_fp32_conv_on_a_device_that_is_not_current(sp):
+    """Every launch of the call, the check of the plan's table included, goes to the context's device."""
+    c, x, w, b = (torch.from_numpy(t) for t in scene(700, 64, 64, "f32"))
+    want = sp.subm_conv(x.cuda(0), w.cuda(0), b.cuda(0), sp.build_neighbors(c.cuda(0)))
+    xd, wd, bd, cd = (t.cuda(1) for t in (x, w, b, c))
+    torch.cuda.synchronize(1)
+    with torch.cuda.device(1):
+        cache = sp.build_neighbors(cd)
+    assert torch.cuda.current_device() == 0
+    y = sp.subm_conv(xd, wd, bd, cache)
+    torch.cuda.synchronize(1)
+    assert torch.equal(y.cpu(), want.cpu())

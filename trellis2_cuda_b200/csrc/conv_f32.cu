@@ -207,10 +207,10 @@ __global__ void __launch_bounds__(FTHREADS, 3) k_conv_f32(const float* __restric
 
 int conv_f32_launch(t2sc_ctx* ctx, const t2sc_plan* plan, const float* x, const float* w, const EpiDev& ep, float* y, i64 n_in, int Ci, int Co, int part) {
   T2_REQ(ctx, Ci % FK == 0, "Ci=%d", Ci);
+  T2_CUDA(ctx, cudaSetDevice(ctx->device));
   const int rc = plan_table_prepare(ctx, const_cast<t2sc_plan*>(plan), n_in);
   if (rc != T2SC_OK) return rc;
   const TilePart tp = tile_part(plan, part);
-  T2_CUDA(ctx, cudaSetDevice(ctx->device));
   const i64 parts = plan->max_tiles * (plan->tile_rows / FM);
   const int ny = cdiv_i(Co, FN);
   const i64 whole = cdiv_i(plan->n_out, FM) * (i64)ny, places = 3ll * ctx->num_sms;
