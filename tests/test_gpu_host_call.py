@@ -8,6 +8,23 @@ from trellis2_cuda_b200 import scenes
 pytestmark = pytest.mark.gpu
 
 
+def test_results_over_the_features():
+    """The first results lie where the last features do: nothing of them may arrive before those have been read."""
+    import trellis2_cuda_b200 as sp
+    n, C = 200000, 64
+    g = torch.Generator().manual_seed(0)
+    cells = torch.arange(n)
+    c = torch.stack([0 * cells, cells // 3600, cells // 60 % 60, cells % 60], 1).to(torch.int32).pin_memory()
+    buf = torch.empty((2 * n, C), dtype=torch.bfloat16).pin_memory()
+    x, y = buf[:n], buf[n * 7 // 8:n * 15 // 8]
+    features = torch.randn((n, C), generator=g).to(torch.bfloat16)
+    w = torch.from_numpy(scenes.kaiming_uniform_weight(C, C, 1)).to(torch.bfloat16).pin_memory()
+    want = sp.subm_conv(features.cuda(), w.cuda(), None, sp.build_neighbors(c.cuda(), want_sorted=False))
+    for _ in range(5):
+        x.copy_(features)
+        assert torch.equal(sp.subm_conv_host(c, x, w, None, out=y).cuda(), want)
+
+
 @pytest.mark.parametrize("dt,C,n,order", [(torch.bfloat16, 256, 20001, "morton"), (torch.float32, 128, 65536, "morton"), (torch.float16, 64, 140001, "morton"),
                                           (torch.bfloat16, 256, 30000, "random"), (torch.bfloat16, 64, 5000, "morton"), (torch.float16, 256, 20001, "pageable")])
 def test_host_call_overlaps_and_gives_the_same_bits(dt, C, n, order):

@@ -315,6 +315,7 @@ cudaError_t side_streams(t2sc_ctx* ctx) {
 // stream.  The rows of it that still wait for a later chunk (a few per cent of a scene in Morton order) are written to the
 // host buffer by k_rows_out at the end.  Where they are more than an eighth of all rows (a scene in random order), everything
 // goes out at the end in one copy.  A chunk is at least 4 MB, 70 us of link time: less than that is not worth its launches.
+// Results that overlap the features in memory must wait until all of those are in, so they take the plain order as well.
 extern "C" int t2sc_subm_conv_host(t2sc_ctx* ctx, const int32_t* coords_host, int64_t n, int W, int H, int D,
                                    const void* x_host, const void* w_host, const void* bias_host, void* y_host,
                                    int dtype, int Ci, int Co) {
@@ -330,7 +331,9 @@ extern "C" int t2sc_subm_conv_host(t2sc_ctx* ctx, const int32_t* coords_host, in
   const size_t lesser = (size_t)n * (xrow < yrow ? xrow : yrow);
   int chunks = (int)(lesser / CHUNK < 8 ? lesser / CHUNK : 8);
   void* y_mapped = nullptr;
-  if (chunks < 2 || yrow % 16 || !pinned_address(x_host) || !(y_mapped = pinned_address(y_host)) || (uintptr_t)y_mapped % 16) chunks = 1;
+  const uintptr_t xa = (uintptr_t)x_host, ya = (uintptr_t)y_host;
+  const bool overlap = xa < ya + (size_t)n * yrow && ya < xa + (size_t)n * xrow;
+  if (chunks < 2 || overlap || yrow % 16 || !pinned_address(x_host) || !(y_mapped = pinned_address(y_host)) || (uintptr_t)y_mapped % 16) chunks = 1;
   const i64 chunk_rows = (n + chunks - 1) / chunks;
   chunks = (int)((n + chunk_rows - 1) / chunk_rows);
   HostCall c(ctx);
