@@ -125,3 +125,21 @@ def test_a_level_belongs_to_the_stream_it_is_made_on(sp, derived):
         same = torch.equal(level.nb.nbr, want.nbr) and torch.equal(level.nb.gray, want.gray)
     torch.cuda.synchronize()
     assert same and (level._info is not None) == derived
+
+
+def test_subdivision_conv_follows_a_map_changed_after_the_parents_plan(sp):
+    """The parents' plan is made by a conv on them; a map written to after that is not what it holds, and the subdivision conv has to
+    go by the map, as it does with a plan of its own."""
+    n = 900
+    g = torch.Generator(device="cuda").manual_seed(9)
+    parent = sp.build_neighbors(torch.from_numpy(cube(n, 9, 11)).cuda())
+    x = torch.randn((n, 64), generator=g, device="cuda").half()
+    w = (torch.randn((8 * 64, 27, 64), generator=g, device="cuda") * 0.03).half()
+    sp.subm_conv(x, w[:64].contiguous(), None, parent)
+    level = sp.subdivide(parent, torch.ones((n, 8), dtype=torch.uint8, device="cuda"))
+    assert level._from_parents(x, 64)
+    parent.nbr[:, 0] = -1
+    assert not level._from_parents(x, 64)
+    alone = sp.cache_from_map(parent.coords, parent.nbr, parent.gray)
+    want = sp.subdiv_conv(x, w, None, sp.Level(level.coords, level.src, level.nb, alone))
+    assert torch.equal(sp.subdiv_conv(x, w, None, level), want)

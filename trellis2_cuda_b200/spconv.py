@@ -157,20 +157,20 @@ class SpConvCache:
         self.vk: dict = {}
         self._plan = None
         self._block_rows, self._tile_rows = block_rows, tile_rows
-        self._extent = None       # set by build_neighbors: the grid, and what its map and coordinates were then
+        self._extent = None       # set by build_neighbors: the grid, and what its coordinates, map and masks were then
 
     def _built(self, extent) -> "SpConvCache":
-        cv, nv = _version(self.coords), _version(self.nbr)
-        if cv is not None and nv is not None:
-            self._extent = (extent, self.coords, cv, self.nbr, nv)
+        made = [(t, _version(t)) for t in (self.coords, self.nbr, self.gray)]
+        if all(v is not None for _, v in made):
+            self._extent = (extent, made)
         return self
 
     def _map_extent(self):
-        """The grid this cache's map was built in, or None if the map or the coordinates may have changed since."""
+        """The grid this cache's map was built in, or None if the map, its masks or the coordinates may have changed since."""
         if self._extent is None:
             return None
-        extent, coords, cv, nbr, nv = self._extent
-        same = self.coords is coords and self.nbr is nbr and _version(coords) == cv and _version(nbr) == nv
+        extent, made = self._extent
+        same = all(now is t and _version(t) == v for now, (t, v) in zip((self.coords, self.nbr, self.gray), made))
         return extent if same else None
 
     def valid(self, B1: int):
@@ -414,7 +414,8 @@ class Level:
         computes a quarter of what the 256-column tile of four slots computes; the children's tiles also need a schedule of
         their own.  Whole up block at 3.7 children per parent, children's tiles against parents': 60,000 parents, 128 -> 64: 539 ->
         449 us; 880,000: 4411 -> 4031, of which the conv and its schedule are about 2150 against 1770: even at 3 children."""
-        return (self._info is not None and self.src is self._info[1] and _version(self.src) == self._info[2] and Cc == 64
+        # The parents' plan may be older than this level: it is the one for their map only while the map is as it was built.
+        return (self._info is not None and self.parent._map_extent() is not None and self.src is self._info[1] and _version(self.src) == self._info[2] and Cc == 64
                 and x.dtype in (torch.float16, torch.bfloat16) and x.shape[1] % 64 == 0
                 and self.parent._tile_rows_for(256, x.shape[1]) == 128 and self.src.shape[0] > 3 * self.parent.N)
 
