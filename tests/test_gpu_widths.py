@@ -183,3 +183,13 @@ def test_fp32_conv_on_a_device_that_is_not_current(sp):
     y = sp.subm_conv(xd, wd, bd, cache)
     torch.cuda.synchronize(1)
     assert torch.equal(y.cpu(), want.cpu())
+
+
+@pytest.mark.parametrize("dt,n,Ci,Co", [("bf16", 700, 32, 64), ("f16", 3000, 96, 160), ("bf16", 129, 224, 256), ("f16", 257, 96, 128)])
+def test_half_chunks_give_the_same_bits_on_either_schedule(sp, dt, n, Ci, Co):
+    """128- and 256-row tiles add up a row's products in one order."""
+    c, x, w, b = scene(n, Ci, Co, dt)
+    xd, wd, bd = (torch.from_numpy(t).cuda().to(TD[dt]) for t in (x, w, b))
+    y = [sp.subm_conv(xd, wd, bd, sp.build_neighbors(torch.from_numpy(c).cuda(), tile_rows=r)) for r in (128, 256)]
+    sp.context().device_status()
+    assert torch.equal(*y)

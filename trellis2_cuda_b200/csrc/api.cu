@@ -129,7 +129,7 @@ int conv_dispatch(t2sc_ctx* ctx, t2sc_plan* plan, const void* x, const void* w, 
   if (e.skip_x) T2_REQ(ctx, e.skip_src && e.skip_cin % 8 == 0 && e.skip_rep > 0 && Co == (e.skip_cin / 8) * e.skip_rep,
                        "skip: Co=%d Cin=%d rep=%d", Co, e.skip_cin, e.skip_rep);
   i64 w_rows = plan->src ? 8ll * Co : Co;
-  bool umma_ok = conv_umma_supported(dtype, Ci, Co, plan->tile_rows);
+  bool umma_ok = conv_umma_supported(dtype, Ci, Co);
   // asked for by name the tcgen05 form keeps the contract of the header (whole 64-channel chunks)
   if (variant == T2SC_VARIANT_UMMA && !(umma_ok && Ci % 64 == 0))
     return t2sc_fail(ctx, T2SC_ERR_UNSUPPORTED, "tcgen05 variant needs fp16/bf16, Ci %% 64 == 0, Co %% 32 == 0 (Ci=%d Co=%d dtype=%d)", Ci, Co, dtype);
@@ -189,7 +189,7 @@ extern "C" int t2sc_subm_conv_peers_part(t2sc_ctx* ctx, t2sc_plan* plan, const u
   T2_REQ(ctx, w && y, "null tensor");
   for (int r = 0; r < n_peers; r++) T2_REQ(ctx, x_peers[r] && (uintptr_t)x_peers[r] % 16 == 0, "peer array %d is null or not 16-byte aligned", r);
   EpiDev e = epi_dev(ep);
-  if (!conv_umma_supported(dtype, Ci, Co, 256) || (e.ln && !conv_umma_fuses_ln(Co)) || plan->src)
+  if (!conv_umma_supported(dtype, Ci, Co) || Ci % 64 || (e.ln && !conv_umma_fuses_ln(Co)) || plan->src)
     return t2sc_fail(ctx, T2SC_ERR_UNSUPPORTED, "peer conv needs a submanifold plan, fp16/bf16, Ci %% 64 == 0, Co %% 32 == 0, LayerNorm only for Co in {32,64,128,256} (Ci=%d Co=%d dtype=%d)", Ci, Co, dtype);
   return conv_umma_launch(ctx, plan, x_peers[self_rank], w, Co, e, y, dtype, rows_peers[self_rank], Ci, Co, part, x_peers, rows_peers, n_peers,
                           self_rank, peer_nbr);
@@ -206,7 +206,7 @@ extern "C" int t2sc_linear(t2sc_ctx* ctx, const void* x, const void* w, const t2
   T2_REQ(ctx, ((uintptr_t)x % 16 == 0) && ((uintptr_t)w % 16 == 0) && ((uintptr_t)y % 16 == 0), "x, w, y must be 16-byte aligned");
   T2_REQ(ctx, !ep || (((uintptr_t)ep->bias % 16 == 0) && ((uintptr_t)ep->residual % 16 == 0)), "epilogue bias and residual must be 16-byte aligned");
   EpiDev e = epi_dev(ep);
-  if (!conv_umma_supported(dtype, Ci, Co, 256) || e.skip_x)
+  if (!conv_umma_supported(dtype, Ci, Co) || Ci % 64 || e.skip_x)
     return t2sc_fail(ctx, T2SC_ERR_UNSUPPORTED, "t2sc_linear runs on the tcgen05 path only: fp16/bf16, Ci %% 64 == 0, Co %% 32 == 0, no skip (Ci=%d Co=%d dtype=%d)", Ci, Co, dtype);
   if (!e.ln || conv_umma_fuses_ln(Co)) return linear_umma_launch(ctx, x, w, e, y, dtype, n, Ci, Co);
   EpiDev first = e, rest = e;       // LayerNorm over a row wider than one accumulator: GEMM + bias now, the rest in the row pass

@@ -171,7 +171,7 @@ int conv_simt_launch(t2sc_ctx* ctx, const t2sc_plan* plan, const void* x, const 
                      int dtype, i64 n_in, int Ci, int Co, int part = T2SC_PART_ALL);
 int conv_f32_launch(t2sc_ctx* ctx, const t2sc_plan* plan, const float* x, const float* w, const EpiDev& ep, float* y, i64 n_in, int Ci, int Co,
                     int part);
-bool conv_umma_supported(int dtype, int Ci, int Co, int tile_rows);
+bool conv_umma_supported(int dtype, int Ci, int Co);      // Linear layers and peers' rows need whole 64-channel chunks besides
 bool conv_umma_fuses_ln(int Co);      // is LayerNorm over Co part of the tcgen05 kernel's epilogue?
 int conv_umma_launch(t2sc_ctx* ctx, const t2sc_plan* plan, const void* x, const void* w, i64 w_rows, const EpiDev& ep, void* y,
                      int dtype, i64 n_in, int Ci, int Co, int part = T2SC_PART_ALL, const void* const* x_peers = nullptr,

@@ -57,7 +57,7 @@ using namespace umma;
 // treats each as a row of its own, of the child that sits there, and skips slots that are not kept.
 template <int BN, int MH, int G, bool PEERS, bool TAIL, int CHILD, int OCC, bool SKIP, class T>
 __global__ void __launch_bounds__(num_threads(MH, G), OCC) k_conv_umma(const __grid_constant__ CUtensorMap tmw, const ConvArgs a) {
-  static_assert(!TAIL || (MH == 1 && !PEERS), "half chunks run on 128-row tiles of local rows");
+  static_assert(!TAIL || !PEERS, "half chunks run on local rows");
   static_assert(G == 1 || (G == 2 && MH == 1), "a second gather group only fits beside 128-row tiles");
   constexpr int STAGE = stage_bytes(BN, MH);          // one unit: MH gathered A halves + one weight slab
   constexpr int S = num_stages(BN, MH, PEERS, OCC);
@@ -404,7 +404,13 @@ __global__ void __launch_bounds__(num_threads(MH, G), OCC) k_conv_umma(const __g
             bool half = false;
             if constexpr (TAIL) {
               half = ++c == nchunk;
-              if (half) { c = 0; tc_mma_k32(d_tmem, ds, ds + ((MH * A_BYTES) >> 4), idesc, acc); }
+              if (half) {
+                c = 0;
+#pragma unroll
+                for (int h = 0; h < MH; h++) {
+                  if (h < halves) tc_mma_k32(d_tmem + h * BN, ds + ((h * A_BYTES) >> 4), ds + ((MH * A_BYTES) >> 4), idesc, acc);
+                }
+              }
             }
             if (!half) {
 #pragma unroll
@@ -540,6 +546,7 @@ int launch_bn(t2sc_ctx* ctx, const CUtensorMap& tm, const ConvArgs& args, i64 ma
     }
     return launch_p<BN, MH, 1, false, T, false, 0, OCC, false>(ctx, tm, args, max_items);
   } else {
+    if (args.Ci % KCH != 0) return launch_p<BN, MH, 1, false, T, true>(ctx, tm, args, max_items);
     return launch_p<BN, MH, 1, false, T>(ctx, tm, args, max_items);
   }
 }
@@ -573,8 +580,8 @@ int pick_bn(int Co, bool pow2 = false) {
 
 }  // namespace
 
-bool conv_umma_supported(int dtype, int Ci, int Co, int tile_rows) {
-  return (dtype == T2SC_F16 || dtype == T2SC_BF16) && Ci % (tile_rows == TILE_M ? KCH / 2 : KCH) == 0 && Co % 32 == 0;
+bool conv_umma_supported(int dtype, int Ci, int Co) {
+  return (dtype == T2SC_F16 || dtype == T2SC_BF16) && Ci % (KCH / 2) == 0 && Co % 32 == 0;
 }
 
 bool conv_umma_fuses_ln(int Co) { return pick_bn(Co, true) == Co; }
