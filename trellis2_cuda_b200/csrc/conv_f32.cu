@@ -12,10 +12,13 @@
 //
 // A small map has too few tiles for the 148 SMs (14,534 rows: 228 tiles of 64), so the taps of a tile are split over a
 // cluster of S = 4 or 8 CTAs, whose sums meet in distributed shared memory.  S grows until there are three CTAs per SM, as many as
-// fit: below that the chip idles, above it the reduction costs more than it gives.
+// fit: below that the chip idles, above it the reduction costs more than it gives.  One wave of whole tiles takes about 155 us at
+// 64 -> 64 channels however full it is, a wave of quarters 41: from nine tenths of a wave of tiles on S stays 1.
 // Every S adds in one order, so a row's bits depend neither on timing nor on the plan nor on how many rows come with it (a scene
 // and its parts give the same): tap v belongs to group v % 8, a group is summed by itself, and the eight sums are added in order.
 // With S = 1 a CTA adds them up as it goes, with S = 4 it hands on two, with S = 8 one; S = 2 would have to keep four apart.
+// Measured, conv alone, 64 -> 64 (without the one order, splits of 1, 2, 4 and 8): 700 rows 25 us (25), 5,000 57 (59), 14,534
+// 103 (98), 20,000 129 (121), 60,000 252 (246).
 #include "common.cuh"
 #include <cooperative_groups.h>
 
@@ -214,7 +217,7 @@ int conv_f32_launch(t2sc_ctx* ctx, const t2sc_plan* plan, const float* x, const 
   const i64 parts = plan->max_tiles * (plan->tile_rows / FM);
   const int ny = cdiv_i(Co, FN);
   const i64 whole = cdiv_i(plan->n_out, FM) * (i64)ny, places = 3ll * ctx->num_sms;
-  const int S = whole >= places ? 1 : 4 * whole >= places ? 4 : 8;
+  const int S = 10 * whole >= 9 * places ? 1 : 4 * whole >= places ? 4 : 8;
   const auto kernel = S == 1 ? k_conv_f32<1> : S == 4 ? k_conv_f32<4> : k_conv_f32<8>;
   static bool attr_set[64][9] = {};
   if (ctx->device >= 64 || !attr_set[ctx->device][S]) {
