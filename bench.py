@@ -410,7 +410,7 @@ def run_single_conv(args, rank, world, local_rank, dev):
     else:
         gbs = ab / (conv_avg_own * 1e-3) / 1e9
         roof = {"bound": "hbm", "achieved": gbs, "peak": pk["hbm_gbs"], "unit": "GB/s", "frac": gbs / pk["hbm_gbs"], "traffic": traffic,
-                "peak_source": f"{pk_src} copy", "kernel": "k_conv_simt", "kernel_ms": conv_avg_own}
+                "peak_source": f"{pk_src} copy", "kernel": "k_conv_f32", "kernel_ms": conv_avg_own}
     h2d = n * 16 + n * Ci * es + Co * 27 * Ci * es
     d2h = n * Co * es
     line = {"metric": METRIC, "value": value, "unit": "TFLOP/s", "n_gpus": world, "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms,
@@ -446,6 +446,18 @@ def run_single_conv(args, rank, world, local_rank, dev):
 
 
 # ------------------------------------------------------------------------------------------ our arm: cfg3, both halves
+def up_schedule(lv, x, Cc):
+    """What the subdivision conv of these features runs: tiles, work items, taps of the children and row-taps multiplied for them (the
+    parents' form multiplies every row of a tile with all 8 slots, four of them to a 256-column item)."""
+    plan = lv.conv_plan_for(x, Cc)
+    st, parents = plan.stats(), plan.src is None
+    masks = lv.parent.gray[(lv.src >> 3).long()]
+    active = sum(int(((masks >> v) & 1).sum()) for v in range(27))
+    bn = 256 if parents else max(b for b in (256, 128, 64, 32) if Cc % b == 0)
+    return {"tiles": st["tiles"], "items": st["tiles"] * ((8 * Cc if parents else Cc) // bn), "ctas_per_sm": 2 if bn < 256 else 1,
+            "active_taps": active, "computed_taps": st["computed_taps"] * (8 if parents else 1)}
+
+
 def run_cfg3(args, rank, world, local_rank, dev):
     import trellis2_cuda_b200 as sp
     from trellis2_cuda_b200 import scenes
@@ -472,7 +484,7 @@ def run_cfg3(args, rank, world, local_rank, dev):
         mark(1)
         lv = sp.subdivide(parent, flags)
         mark(2)
-        lv.up_plan_for(Cc).check(n); lv.nb.plan_for(Cc, Cc).check(lv.coords.shape[0])
+        lv.conv_plan_for(x, Cc).check(n); lv.nb.plan_for(Cc, Cc).check(lv.coords.shape[0])
         mark(3)
         up = sp.subdiv_conv(x, w1, None, lv)
         mark(4)
@@ -482,7 +494,7 @@ def run_cfg3(args, rank, world, local_rank, dev):
 
     lv, y = step()
     m = lv.coords.shape[0]
-    st1, st2 = lv.up_plan_for(Cc).stats(), lv.nb.plan_for(Cc, Cc).stats()
+    st1, st2 = up_schedule(lv, x, Cc), lv.nb.plan_for(Cc, Cc).stats()
     flops = [0, 0, 0, 2.0 * st1["active_taps"] * Ci * Cc, 2.0 * st2["active_taps"] * Cc * Cc]
     byts = [n * 16 + n * 27 * 4 + n * 4, n * 8 + m * 16 + m * 4 + m * 16 + m * 27 * 4 + m * 4, 0,
             alg_bytes(n, m, Ci, Cc, 8 * Cc, es), alg_bytes(m, m, Cc, Cc, Cc, es)]
@@ -582,12 +594,13 @@ def run_cfg4(args, rank, world, local_rank, dev):
             lv = sp.subdivide(cache, flags[l])
             if evs:
                 evs[l][2].record()
+            if info is not None:
+                st = up_schedule(lv, x, C // 2)
+                info[-1].update(up_tiles=st["tiles"], up_items=st["items"], up_places=st["ctas_per_sm"] * nsm, up_active_taps=st["active_taps"],
+                                up_computed_taps=st["computed_taps"])
             x = sp.subdiv_conv(x, up, None, lv)
             if evs:
                 evs[l][3].record()
-            if info is not None:
-                st = lv.up_plan_for(C // 2).stats()
-                info[-1].update(up_tiles=st["tiles"], up_active_taps=st["active_taps"], up_computed_taps=st["computed_taps"])
             cache = lv.nb
         return x
 
@@ -625,11 +638,11 @@ def run_cfg4(args, rank, world, local_rank, dev):
     for l, C in enumerate(chans):
         i = info[l]
         bn = max(b for b in (256, 128, 64, 32) if C % b == 0)
-        items = i["tiles"] * (C // bn)
+        items, places = i["tiles"] * (C // bn), nsm * (2 if bn < 256 else 1)          # CTAs of the persistent kernel
         f_blocks = 4 * 2.0 * i["active_taps"] * C * C
         t_blocks = acc[l][0] / args.steps
         row = {"level": l, "grid": 64 << l, "voxels": i["voxels"], "C": C, "tiles": i["tiles"], "work_items_per_conv": items,
-               "sm_fill": items / (-(-items // nsm) * nsm), "blocks_ms": t_blocks, "blocks_tflops": f_blocks / (t_blocks * 1e-3) / 1e12,
+               "sm_fill": items / (-(-items // places) * places), "blocks_ms": t_blocks, "blocks_tflops": f_blocks / (t_blocks * 1e-3) / 1e12,
                "blocks_frac_of_sustained": f_blocks / (t_blocks * 1e-3) / 1e12 / pk["bf16_tflops_sustained"],
                "active_over_computed_taps": i["active_taps"] / max(i["computed_taps"], 1)}
         flops_total += f_blocks
@@ -637,10 +650,9 @@ def run_cfg4(args, rank, world, local_rank, dev):
             Cc = C // 2
             f_up = 2.0 * i["up_active_taps"] * C * Cc
             t_map, t_up = acc[l][1] / args.steps, acc[l][2] / args.steps
-            bnu = max(b for b in (256, 128, 64, 32) if Cc % b == 0)
-            items_up = i["up_tiles"] * (Cc // bnu)
             row.update(subdivide_and_child_map_ms=t_map, up_conv_ms=t_up, up_conv_tflops=f_up / (t_up * 1e-3) / 1e12, up_tiles=i["up_tiles"],
-                       up_sm_fill=items_up / (-(-items_up // nsm) * nsm))
+                       up_active_over_computed_taps=i["up_active_taps"] / max(i["up_computed_taps"], 1),
+                       up_sm_fill=i["up_items"] / (-(-i["up_items"] // i["up_places"]) * i["up_places"]))
             flops_total += f_up
         table.append(row)
     line = {"metric": METRIC, "value": flops_total / (ms * 1e-3) / 1e12, "unit": "TFLOP/s", "n_gpus": 1, "steps": args.steps, "warmup": args.warmup,

@@ -34,7 +34,9 @@ def test_child_map_from_the_parents(sp, name, coords, extent, derived):
     sub[n // 2] = -1
     sub[0] = 1
     d = torch.from_numpy(coords).cuda()
-    lv = sp.subdivide(sp.build_neighbors(d, extent, extent, extent), torch.from_numpy(sub).cuda())
+    parent, flags, launches = sp.build_neighbors(d, extent, extent, extent), torch.from_numpy(sub).cuda(), sp.context().launch_count()
+    lv = sp.subdivide(parent, flags)
+    assert sp.context().launch_count() - launches == (3 if derived else 4), name          # count, emit, and one kernel for the map or two for the hash
     cc, src = oracle.subdivide(coords, sub.astype(np.float32) > 0)
     assert np.array_equal(lv.coords.cpu().numpy(), cc) and np.array_equal(lv.src.cpu().numpy(), src), name
     want = sp.build_neighbors(lv.coords, want_sorted=False)

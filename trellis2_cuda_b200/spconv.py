@@ -95,7 +95,7 @@ class SpConvCfg:
 def spconv_cfg(N: int, Ci: int, Co: int) -> SpConvCfg:
     """The reference replays FlexGEMM's autotuned (B1, BK, SPLITK) per shape (src/spconv.cu:186-221); on a
     B200 its table has no entry and it runs 128/64/1.  This build has one schedule: 128-row tiles, 64-channel
-    K steps, no split-K (the persistent tcgen05 kernel keeps all SMs busy without it)."""
+    K steps, no split-K on the tensor cores (the fp32 conv of a small map splits a tile's taps over a cluster)."""
     return SpConvCfg(128, 64, 1)
 
 
@@ -191,10 +191,9 @@ class SpConvCache:
         return self.plan_for(256)
 
     def _tile_rows_for(self, Co: int, Ci: int) -> int:
-        """128-row tiles unless forced: every layer narrower than 256 output channels runs the form of the kernel that packs
-        several (tap, chunk) units into one pipeline stage, which exists for 128-row tiles; 256-channel slabs share nothing
-        between two 128-row halves that the L2 does not already give them (measured on 218 k rows: 256-row tiles are 10 %
-        slower there because one union mask then covers 256 rows)."""
+        """128-row tiles unless forced, at every width: one tap mask covers fewer rows (256-row tiles are 10 % slower at 256 channels
+        on 218 k rows), and the form of the kernel that runs two CTAs per SM, below 256 output channels, exists for them only.
+        What two halves of a 256-row tile share of a weight slab the L2 gives them anyway."""
         return self._tile_rows or 128
 
     def plan_for(self, Co: int, Ci: int = 0) -> _Plan:
@@ -430,6 +429,10 @@ class Level:
             self._up_plans[tile_rows] = _Plan(self.parent.ctx, self.parent.nbr, self.parent.gray, self.src, 0, tile_rows)
         return self._up_plans[tile_rows]
 
+    def conv_plan_for(self, x: torch.Tensor, Cc: int) -> _Plan:
+        """The schedule :func:`subdiv_conv` takes for the features x: the parents' or the level's own."""
+        return self.parent.plan_for(256, x.shape[1]) if self._from_parents(x, Cc) else self.up_plan_for(Cc)
+
     @property
     def up_plan(self) -> _Plan:
         """The subdivision schedule made last (for inspection)."""
@@ -438,7 +441,9 @@ class Level:
 
 def subdivide(parent: SpConvCache, sub: torch.Tensor, want_sorted: bool = False) -> Level:
     """SDecoder::c2s (src/sdec.cu:45-57): ``sub`` [n,8] fp16/bf16 logits (kept iff > 0) or uint8 flags ->
-    child coords in (parent, slot) order, ``src``, and the children's neighbour cache."""
+    child coords in (parent, slot) order, ``src``, and the children's neighbour cache.  The children's map is read off the parents'
+    where that is as :func:`build_neighbors` made it, else hashed; under ``torch.inference_mode``, whose tensors do not count
+    how often they were written, it is hashed too."""
     _chk(sub, "sub", None, 2)
     n = parent.N
     if sub.shape != (n, 8) or sub.dtype not in (torch.float16, torch.bfloat16, torch.uint8):
